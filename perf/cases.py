@@ -226,6 +226,7 @@ def run(state):
         return {"parent": parent if host else _device_result(g, 0, v, "<i4")}
     if do == "pagerank":
         ranks, deltas, _ = g.pagerank(ITERATIONS, to_host=host, f32=case["f32"])
+        deltas = torch.as_tensor(deltas, dtype=torch.float32 if case["f32"] else torch.float64)  # as exact as the ranks
         return {"ranks": ranks if host else _device_result(g, 0, v, "<f4" if case["f32"] else "<f8"), "deltas": deltas}
     if do == "cc":
         label, _ = g.cc(to_host=host)
