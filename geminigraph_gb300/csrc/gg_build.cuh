@@ -12,11 +12,20 @@ namespace gg {
 // Bits of the largest vertex id (at least 1): keys pack (major << b) | minor.
 int bits_for(uint32_t V);
 
-// Stable LSD radix sort of n keys (and optional 32-bit values) on the low
-// key_bits bits, ping-ponging between (k0, v0) and (k1, v1); *kres / *vres
-// name the buffers holding the result.
-int radix_sort(gg_graph *g, uint64_t *k0, uint32_t *v0, uint64_t *k1, uint32_t *v1, size_t n, int key_bits,
-               uint64_t **kres, uint32_t **vres);
+// The 32-bit values of a sort: read from `in` (null: keys only), moved
+// between b0 and b1 (b0 may be `in`; `in` is only read when it is neither),
+// the last pass writing to `last` when it is set.
+struct SortValues {
+  uint32_t *in = nullptr, *b0 = nullptr, *b1 = nullptr, *last = nullptr;
+};
+
+// Stable LSD radix sort of n < 2^32 keys (and values) on the key bits
+// [lo_bit, hi_bit), ping-ponging the keys between k0 (the input) and k1;
+// *kres / *vres name the buffers holding the result.  scratch: device memory
+// of radix_scratch_bytes(n), 16-byte aligned.  Waits for the stream.
+size_t radix_scratch_bytes(size_t n);
+int radix_sort(gg_graph *g, void *scratch, uint64_t *k0, uint64_t *k1, const SortValues &v, size_t n, int lo_bit,
+               int hi_bit, uint64_t **kres, uint32_t **vres);
 
 // Neighbour / weight storage in device memory, or in mapped pinned host memory.
 int adj_alloc(gg_graph *g, bool host, void **p, size_t bytes);
@@ -47,6 +56,20 @@ struct DevScratch {
   DevScratch &operator=(const DevScratch &) = delete;
   ~DevScratch() {
     for (void *q : p) cudaFree(q);
+  }
+  // The sort buffers of n entries in one allocation (a cudaMalloc and its
+  // cudaFree cost about 0.15 ms together at these sizes).
+  int sort_buffers(size_t n, bool values, uint64_t **k0, uint64_t **k1, uint32_t **v0, uint32_t **v1, void **scratch) {
+    const size_t keys = (sizeof(uint64_t) * n + 255) / 256 * 256;
+    const size_t vals = values ? (sizeof(uint32_t) * n + 255) / 256 * 256 : 0;
+    char *q = nullptr;
+    GG_TRY(get(&q, 2 * keys + 2 * vals + radix_scratch_bytes(n)));
+    *k0 = (uint64_t *)q;
+    *k1 = (uint64_t *)(q + keys);
+    *v0 = values ? (uint32_t *)(q + 2 * keys) : nullptr;
+    *v1 = values ? (uint32_t *)(q + 2 * keys + vals) : nullptr;
+    *scratch = q + 2 * keys + 2 * vals;
+    return GG_OK;
   }
   template <typename T>
   int get(T **out, size_t count) {

@@ -78,6 +78,9 @@ struct Dir {
   uint32_t *big_chunk = nullptr;    // nbig+1: prefix of per-vertex chunk counts (aligned blocks, see big_range)
   uint32_t *big_owner = nullptr;    // nbigchunks: index into big of each chunk
   uint32_t nbigchunks = 0;
+  uint32_t *bins_mem = nullptr;     // the allocations of the bins: big, big_chunk;
+  uint32_t *owner_mem = nullptr;    // the owners, med, heavy and heavy_chunk
+  size_t owner_words = 0;
   // bounds of the ids and entries, and the graph's error word (GG_CHECK builds)
   uint32_t nv = 0;
   uint64_t ne = 0;

@@ -109,11 +109,6 @@ __global__ void __launch_bounds__(OC_THREADS) oc_degree_both(const uint32_t *__r
   }
 }
 
-struct U32AsU64 {
-  const uint32_t *p;
-  __device__ __forceinline__ uint64_t operator()(size_t i) const { return p[i]; }
-};
-
 // One thread: greedy ranges [bounds[k], bounds[k+1]) of at most cap entries
 // (a single longer list is a range of its own).  *nparts = 0 when more than
 // max_parts ranges would be needed.
@@ -272,7 +267,7 @@ __global__ void oc_emit(const uint64_t *__restrict__ ks, const uint32_t *__restr
 }
 
 // Sort-buffer bytes per entry of a range: two key buffers, two value
-// buffers when weighted, the radix sort's per-tile digit counts.
+// buffers when weighted, the radix sort's look-back words.
 static uint64_t oc_entry_bytes(int weighted) { return 16 + (weighted ? 8 : 0) + 1; }
 
 // One direction by ranges of at most cap entries (force_parts > 0: ranges of
@@ -386,6 +381,8 @@ static int build_dir_partitioned(gg_graph *g, const uint32_t *rec, uint64_t E, i
     *groups_out = (uint32_t)gstart.size() - 1;
     uint64_t *k0 = nullptr, *k1 = nullptr;
     uint32_t *v0 = nullptr, *v1 = nullptr;
+    char *sort_scratch = nullptr;
+    GG_TRY(tmp.get(&sort_scratch, radix_scratch_bytes(maxnp)));
     GG_TRY(tmp.get(&k0, gmax));
     GG_TRY(tmp.get(&k1, maxnp));
     if (g->weighted) {
@@ -405,8 +402,9 @@ static int build_dir_partitioned(gg_graph *g, const uint32_t *rec, uint64_t E, i
         const uint64_t at = hbase[p] - hbase[p0];
         uint64_t *ks;
         uint32_t *vs;
-        GG_TRY(radix_sort(g, k0 + at, v0 ? v0 + at : nullptr, k1, v1, np, bits + bits_for(hb[p + 1] - hb[p]), &ks,
-                          &vs));
+        SortValues sv;
+        if (v0) sv = SortValues{v0 + at, v0 + at, v1, nullptr};
+        GG_TRY(radix_sort(g, sort_scratch, k0 + at, k1, sv, np, 0, bits + bits_for(hb[p + 1] - hb[p]), &ks, &vs));
         oc_emit<<<grid_for(np, 256, g->num_sms, 16), 256, 0, g->stream>>>(
             ks, vs, np, bits, d->nbr + hbase[p], d->w ? (uint32_t *)d->w + hbase[p] : nullptr);
         GG_CUDA(cudaGetLastError());

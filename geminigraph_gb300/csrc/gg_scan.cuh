@@ -17,6 +17,12 @@ struct ArrayIn {
   __device__ __forceinline__ T operator()(size_t i) const { return p[i]; }
 };
 
+// 32-bit values scanned in 64 bits.
+struct U32AsU64 {
+  const uint32_t *p;
+  __device__ __forceinline__ uint64_t operator()(size_t i) const { return p[i]; }
+};
+
 // Degree of queue entry i: deg[q[i]].
 struct QueueDegreeIn {
   const uint32_t *q;

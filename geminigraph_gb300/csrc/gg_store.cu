@@ -3,9 +3,10 @@
 // Replaces Graph::load_directed (core/graph.hpp:771-1339) and
 // Graph::load_undirected_from_directed (core/graph.hpp:349-757).  The
 // reference makes five passes over the file with MPI self-shuffles and racing
-// fetch_add fills; here every direction is one stable LSD radix sort of
-// packed 64-bit (major << b | minor) keys on the device (b = bits of V-1),
-// followed by a boundary pass that writes the offsets.  Lists come out sorted
+// fetch_add fills; here the CSR is one stable LSD radix sort of packed 64-bit
+// (src << b | dst) keys on the device (b = bits of V-1), the CSC a stable sort
+// of the CSR's order on dst alone, each followed by a boundary pass that
+// writes the offsets.  Lists come out sorted
 // by neighbour id with duplicate edges in record order, so the build is
 // deterministic.  Degrees are offset differences; symmetric graphs sort the
 // records plus their reverses once and alias CSC = CSR (core/graph.hpp:733-738);
@@ -195,130 +196,8 @@ int timed_end(gg_graph *g, gg_run_stats *st, int launches) {
   return GG_OK;
 }
 
-// ------------------------------------------------------------------ radix sort
-constexpr int RS_THREADS = 256;
-constexpr int RS_ITEMS = 16;
-constexpr int RS_TILE = RS_THREADS * RS_ITEMS;   // 4096 keys per tile
-constexpr int RS_WARP_KEYS = 32 * RS_ITEMS;      // 512 consecutive keys per warp
-
-__global__ void __launch_bounds__(RS_THREADS) rs_upsweep(const uint64_t *__restrict__ keys, size_t n, int shift,
-                                                         uint32_t *__restrict__ counts, uint32_t ntiles) {
-  __shared__ uint32_t hist[256];
-  hist[threadIdx.x] = 0;
-  __syncthreads();
-  size_t base = (size_t)blockIdx.x * RS_TILE;
-#pragma unroll 4
-  for (int k = 0; k < RS_ITEMS; k++) {
-    size_t idx = base + (size_t)k * RS_THREADS + threadIdx.x;
-    if (idx < n) atomicAdd(&hist[(keys[idx] >> shift) & 255u], 1u);
-  }
-  __syncthreads();
-  counts[(size_t)threadIdx.x * ntiles + blockIdx.x] = hist[threadIdx.x];
-}
-
-// Stable scatter of one tile.  Warp w ranks keys [w*512, w*512+512) of the
-// tile in order (round r, lane) with __match_any_sync peer groups and a
-// warp-private digit histogram; warps are then offset by the per-digit prefix
-// over lower warps, and tiles by the digit-major scan of the upsweep counts.
-__global__ void __launch_bounds__(RS_THREADS) rs_scatter(const uint64_t *__restrict__ kin,
-                                                         const uint32_t *__restrict__ vin,
-                                                         uint64_t *__restrict__ kout, uint32_t *__restrict__ vout,
-                                                         size_t n, int shift, const uint32_t *__restrict__ scanned,
-                                                         uint32_t ntiles) {
-  __shared__ uint32_t whist[RS_THREADS / 32][256];
-  __shared__ uint32_t gbase[256];
-  for (int i = threadIdx.x; i < (RS_THREADS / 32) * 256; i += RS_THREADS) (&whist[0][0])[i] = 0;
-  gbase[threadIdx.x] = scanned[(size_t)threadIdx.x * ntiles + blockIdx.x];
-  __syncthreads();
-  const unsigned w = threadIdx.x >> 5, lane = lane_id();
-  const size_t base = (size_t)blockIdx.x * RS_TILE + (size_t)w * RS_WARP_KEYS;
-  uint64_t key[RS_ITEMS];
-  uint32_t val[RS_ITEMS];
-  uint32_t rank[RS_ITEMS];
-#pragma unroll
-  for (int r = 0; r < RS_ITEMS; r++) {
-    size_t idx = base + (size_t)r * 32 + lane;
-    bool valid = idx < n;
-    key[r] = valid ? kin[idx] : 0ull;
-    val[r] = (vin && valid) ? vin[idx] : 0u;
-    uint32_t d = valid ? (uint32_t)((key[r] >> shift) & 255u) : 256u + lane;
-    unsigned peers = __match_any_sync(GG_FULL, d);
-    unsigned leader = __ffs(peers) - 1;
-    uint32_t cnt = valid ? whist[w][d] : 0u;
-    __syncwarp();
-    if (valid && lane == leader) whist[w][d] = cnt + __popc(peers);
-    __syncwarp();
-    rank[r] = cnt + __popc(peers & lanemask_lt());
-  }
-  __syncthreads();
-  {
-    uint32_t run = 0;
-#pragma unroll
-    for (int ww = 0; ww < RS_THREADS / 32; ww++) {
-      uint32_t t = whist[ww][threadIdx.x];
-      whist[ww][threadIdx.x] = run;
-      run += t;
-    }
-  }
-  __syncthreads();
-#pragma unroll
-  for (int r = 0; r < RS_ITEMS; r++) {
-    size_t idx = base + (size_t)r * 32 + lane;
-    if (idx < n) {
-      uint32_t d = (uint32_t)((key[r] >> shift) & 255u);
-      uint32_t pos = gbase[d] + whist[w][d] + rank[r];
-      kout[pos] = key[r];
-      if (vout) vout[pos] = val[r];
-    }
-  }
-}
-
-// Sorts n keys (and optional values) on the low `key_bits` bits.  Returns the
-// buffers holding the result through *kres / *vres (either the inputs or the
-// alternates).
-int radix_sort(gg_graph *g, uint64_t *k0, uint32_t *v0, uint64_t *k1, uint32_t *v1, size_t n, int key_bits,
-                      uint64_t **kres, uint32_t **vres) {
-  *kres = k0;
-  *vres = v0;
-  if (n <= 1) return GG_OK;
-  size_t ntiles = (n + RS_TILE - 1) / RS_TILE;
-  size_t ncounts = 256 * ntiles;
-  uint32_t *counts = nullptr, *scanned = nullptr, *scratch = nullptr;
-  GG_CUDA(cudaMalloc(&counts, sizeof(uint32_t) * ncounts));
-  GG_CUDA(cudaMalloc(&scanned, sizeof(uint32_t) * (ncounts + 1)));
-  GG_CUDA(cudaMalloc(&scratch, sizeof(uint32_t) * scan_scratch_elems(ncounts)));
-  uint64_t *ka = k0, *kb = k1;
-  uint32_t *va = v0, *vb = v1;
-  int status = GG_OK;
-  for (int shift = 0; shift < key_bits; shift += 8) {
-    rs_upsweep<<<(unsigned)ntiles, RS_THREADS, 0, g->stream>>>(ka, n, shift, counts, (uint32_t)ntiles);
-    cudaError_t e = cudaGetLastError();
-    if (e == cudaSuccess)
-      e = exclusive_scan<uint32_t, ArrayIn<uint32_t>>(ArrayIn<uint32_t>{counts}, ncounts, scanned, scratch,
-                                                      g->stream, nullptr);
-    if (e == cudaSuccess) {
-      rs_scatter<<<(unsigned)ntiles, RS_THREADS, 0, g->stream>>>(ka, va, kb, vb, n, shift, scanned,
-                                                                 (uint32_t)ntiles);
-      e = cudaGetLastError();
-    }
-    if (e != cudaSuccess) {
-      status = cuda_status(e, "radix sort");
-      break;
-    }
-    uint64_t *tk = ka; ka = kb; kb = tk;
-    uint32_t *tv = va; va = vb; vb = tv;
-  }
-  cudaStreamSynchronize(g->stream);
-  cudaFree(counts);
-  cudaFree(scanned);
-  cudaFree(scratch);
-  *kres = ka;
-  *vres = va;
-  return status;
-}
-
 // ------------------------------------------------------------------ build kernels
-// mode 0: key (src,dst); 1: key (dst,src); 2: both, records then reverses.
+// mode 0: key (src,dst); 2: both (src,dst) and (dst,src), records then reverses.
 __global__ void make_keys(const uint32_t *__restrict__ rec, size_t E, int words, int mode, int bits, uint32_t V,
                           uint64_t *__restrict__ keys, uint32_t *__restrict__ vals, unsigned *err) {
   for (size_t i = (size_t)blockIdx.x * blockDim.x + threadIdx.x; i < E; i += (size_t)gridDim.x * blockDim.x) {
@@ -330,14 +209,8 @@ __global__ void make_keys(const uint32_t *__restrict__ rec, size_t E, int words,
       d = 0;
     }
     uint64_t fwd = ((uint64_t)s << bits) | d, rev = ((uint64_t)d << bits) | s;
-    if (mode == 0) {
-      keys[i] = fwd;
-    } else if (mode == 1) {
-      keys[i] = rev;
-    } else {
-      keys[i] = fwd;
-      keys[E + i] = rev;
-    }
+    keys[i] = fwd;
+    if (mode == 2) keys[E + i] = rev;
     if (vals) {
       vals[i] = wb;
       if (mode == 2) vals[E + i] = wb;
@@ -345,15 +218,19 @@ __global__ void make_keys(const uint32_t *__restrict__ rec, size_t E, int words,
   }
 }
 
-// off[v] = first position whose major id is >= v, for v in [0, V].
-__global__ void offsets_from_keys(const uint64_t *__restrict__ keys, size_t n, int bits, uint32_t V,
+// off[v] = first position whose major id is >= v, for v in [0, V], and nbr =
+// the minor ids, from n sorted keys.  The major id is a key's upper part
+// (low_major: its low `bits` bits).
+__global__ void offsets_from_keys(const uint64_t *__restrict__ keys, size_t n, int bits, bool low_major, uint32_t V,
                                   uint64_t *__restrict__ off, uint32_t *__restrict__ nbr) {
-  const uint64_t mask = (bits >= 64) ? ~0ull : ((1ull << bits) - 1);
+  const uint64_t mask = (1ull << bits) - 1;
   for (size_t i = (size_t)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += (size_t)gridDim.x * blockDim.x) {
-    uint64_t k = keys[i];
-    uint64_t maj = k >> bits;
-    nbr[i] = (uint32_t)(k & mask);
-    long long prev = i ? (long long)(keys[i - 1] >> bits) : -1ll;
+    const uint64_t k = keys[i];
+    const uint64_t low = k & mask, high = k >> bits;
+    const uint64_t maj = low_major ? low : high;
+    nbr[i] = (uint32_t)(low_major ? high : low);
+    long long prev = -1ll;
+    if (i) prev = (long long)(low_major ? keys[i - 1] & mask : keys[i - 1] >> bits);
     for (long long v = prev + 1; v <= (long long)maj; v++) off[v] = i;
     if (i == n - 1)
       for (uint64_t v = maj + 1; v <= V; v++) off[v] = n;
@@ -376,29 +253,28 @@ __global__ void degrees_from_offsets(const uint64_t *__restrict__ off, uint32_t 
     deg[v] = (uint32_t)(off[v + 1] - off[v]);
 }
 
-// 1 if LIGHT/HEAVY bin bounds lo < deg[i] <= hi.
-struct DegInRange {
+// 1 where lo < deg[i].
+struct DegAbove {
   const uint32_t *deg;
-  uint32_t lo, hi;
-  __device__ __forceinline__ uint32_t operator()(size_t i) const {
-    uint32_t d = deg[i];
-    return (d > lo && d <= hi) ? 1u : 0u;
-  }
+  uint32_t lo;
+  __device__ __forceinline__ uint32_t operator()(size_t i) const { return deg[i] > lo ? 1u : 0u; }
 };
 
-__global__ void compact_by_pos(const uint32_t *__restrict__ deg, uint32_t V, uint32_t lo, uint32_t hi,
+__global__ void compact_by_pos(const uint32_t *__restrict__ deg, uint32_t V, uint32_t lo,
                                const uint32_t *__restrict__ pos, uint32_t *__restrict__ out) {
-  for (size_t v = (size_t)blockIdx.x * blockDim.x + threadIdx.x; v < V; v += (size_t)gridDim.x * blockDim.x) {
-    uint32_t d = deg[v];
-    if (d > lo && d <= hi) out[pos[v]] = (uint32_t)v;
-  }
+  for (size_t v = (size_t)blockIdx.x * blockDim.x + threadIdx.x; v < V; v += (size_t)gridDim.x * blockDim.x)
+    if (deg[v] > lo) out[pos[v]] = (uint32_t)v;
 }
 
-struct ChunkCount {
+// Heavy vertices among a vertex list (1 each), and their HEAVY_CHUNK chunks.
+struct HeavyCount {
   const uint32_t *list;
   const uint32_t *deg;
-  uint32_t chunk;
-  __device__ __forceinline__ uint32_t operator()(size_t i) const { return (deg[list[i]] + chunk - 1) / chunk; }
+  uint32_t chunk;  // 0: count the vertices
+  __device__ __forceinline__ uint32_t operator()(size_t i) const {
+    const uint32_t d = deg[list[i]];
+    return d <= HEAVY_DEG ? 0u : chunk ? (d + chunk - 1) / chunk : 1u;
+  }
 };
 
 // Long lists are cut at absolute multiples of the chunk size in the adjacency
@@ -414,6 +290,24 @@ struct AlignedChunkCount {
     return e > b ? (uint32_t)((e - 1) / chunk - b / chunk + 1) : 0u;
   }
 };
+
+// The long-list vertices split into medium and heavy ones; pos, first: the
+// scans of HeavyCount over the list (vertices, chunks).
+__global__ void split_heavy(const uint32_t *__restrict__ big, uint32_t nbig, const uint32_t *__restrict__ deg,
+                            const uint32_t *__restrict__ pos, const uint32_t *__restrict__ first,
+                            uint32_t *__restrict__ med, uint32_t *__restrict__ heavy,
+                            uint32_t *__restrict__ heavy_chunk) {
+  for (size_t i = (size_t)blockIdx.x * blockDim.x + threadIdx.x; i < nbig; i += (size_t)gridDim.x * blockDim.x) {
+    const uint32_t v = big[i], h = pos[i];
+    if (deg[v] > HEAVY_DEG) {
+      heavy[h] = v;
+      heavy_chunk[h] = first[i];
+    } else {
+      med[i - h] = v;
+    }
+    if (i == nbig - 1) heavy_chunk[pos[nbig]] = first[nbig];
+  }
+}
 
 __global__ void fill_chunk_owner(const uint32_t *__restrict__ heavy_chunk, uint32_t nheavy,
                                  uint32_t *__restrict__ owner) {
@@ -449,73 +343,72 @@ int bits_for(uint32_t V) {
   return b;
 }
 
-// Ordered list of the vertices with lo < deg <= hi (scan + scatter).
-static int bin_list(gg_graph *g, const Dir *d, uint32_t lo, uint32_t hi, uint32_t **list, uint32_t *count) {
-  uint32_t V = g->V;
-  uint32_t *pos = nullptr, *scratch = nullptr;
-  GG_CUDA(cudaMalloc(&pos, sizeof(uint32_t) * ((size_t)V + 1)));
-  GG_CUDA(cudaMalloc(&scratch, sizeof(uint32_t) * scan_scratch_elems(V)));
-  GG_CUDA((exclusive_scan<uint32_t, DegInRange>(DegInRange{d->deg, lo, hi}, V, pos, scratch, g->stream, nullptr)));
-  uint32_t n = 0;
-  GG_CUDA(cudaMemcpyAsync(&n, pos + V, sizeof(uint32_t), cudaMemcpyDeviceToHost, g->stream));
-  GG_CUDA(cudaStreamSynchronize(g->stream));
-  GG_CUDA(cudaMalloc(list, sizeof(uint32_t) * (n ? n : 1)));
-  if (n) {
-    compact_by_pos<<<grid_for(V, 256, g->num_sms, 16), 256, 0, g->stream>>>(d->deg, V, lo, hi, pos, *list);
-    GG_CUDA(cudaGetLastError());
-  }
-  GG_CUDA(cudaStreamSynchronize(g->stream));
-  cudaFree(pos);
-  cudaFree(scratch);
-  *count = n;
-  g->graph_bytes += sizeof(uint32_t) * n;
-  return GG_OK;
-}
-
-// Chunk table of a vertex list: *prefix (n+1) of ceil(deg/chunk), *owner[c] =
-// list index of chunk c.
-static int chunk_table(gg_graph *g, const Dir *d, const uint32_t *list, uint32_t n, uint32_t chunk,
-                       uint32_t **prefix, uint32_t **owner, uint32_t *nchunks, bool aligned = false) {
-  GG_CUDA(cudaMalloc(prefix, sizeof(uint32_t) * ((size_t)n + 1)));
-  uint32_t *scratch = nullptr;
-  GG_CUDA(cudaMalloc(&scratch, sizeof(uint32_t) * scan_scratch_elems((size_t)n + 1)));
-  if (aligned)
-    GG_CUDA((exclusive_scan<uint32_t, AlignedChunkCount>(AlignedChunkCount{list, d->off, chunk}, n, *prefix, scratch,
-                                                         g->stream, nullptr)));
-  else
-    GG_CUDA((exclusive_scan<uint32_t, ChunkCount>(ChunkCount{list, d->deg, chunk}, n, *prefix, scratch, g->stream,
-                                                  nullptr)));
-  uint32_t nc = 0;
-  GG_CUDA(cudaMemcpyAsync(&nc, *prefix + n, sizeof(uint32_t), cudaMemcpyDeviceToHost, g->stream));
-  GG_CUDA(cudaStreamSynchronize(g->stream));
-  cudaFree(scratch);
-  *nchunks = nc;
-  GG_CUDA(cudaMalloc(owner, sizeof(uint32_t) * (nc ? nc : 1)));
-  if (n) {
-    fill_chunk_owner<<<grid_for(n, 128, g->num_sms, 8), 128, 0, g->stream>>>(*prefix, n, *owner);
-    GG_CUDA(cudaGetLastError());
-  }
-  GG_CUDA(cudaStreamSynchronize(g->stream));
-  g->graph_bytes += sizeof(uint32_t) * ((size_t)n + 1 + nc);
-  return GG_OK;
-}
-
-// Degree bins of one direction (see Dir).
+// Degree bins of one direction (see Dir): the long lists (deg > light) with
+// their aligned chunks, split into medium and heavy ones for the BFS pulls.
+// Two allocations hold all of them (bins_mem once the number of long lists
+// is known, owner_mem once the chunk counts are).
 static int build_bins(gg_graph *g, Dir *d) {
-  GG_TRY(bin_list(g, d, d->light, HEAVY_DEG, &d->med, &d->nmed));
-  GG_TRY(bin_list(g, d, HEAVY_DEG, 0xffffffffu, &d->heavy, &d->nheavy));
-  GG_TRY(chunk_table(g, d, d->heavy, d->nheavy, HEAVY_CHUNK, &d->heavy_chunk, &d->chunk_owner, &d->nchunks));
-  GG_TRY(bin_list(g, d, d->light, 0xffffffffu, &d->big, &d->nbig));
-  GG_TRY(chunk_table(g, d, d->big, d->nbig, d->chunk, &d->big_chunk, &d->big_owner, &d->nbigchunks, true));
+  const uint32_t V = g->V;
+  cudaStream_t s = g->stream;
+  DevScratch tmp;
+  uint32_t *pos = nullptr, *scratch = nullptr;
+  GG_TRY(tmp.get(&pos, (size_t)V + 1 + scan_scratch_elems(V)));
+  scratch = pos + V + 1;
+  GG_CUDA((exclusive_scan<uint32_t, DegAbove>(DegAbove{d->deg, d->light}, V, pos, scratch, s, nullptr)));
+  uint32_t n = 0;
+  GG_CUDA(cudaMemcpyAsync(&n, pos + V, sizeof(uint32_t), cudaMemcpyDeviceToHost, s));
+  GG_CUDA(cudaStreamSynchronize(s));
+  if (n == 0) return GG_OK;
+  GG_CUDA(cudaMalloc(&d->bins_mem, sizeof(uint32_t) * (2 * (size_t)n + 1)));
+  d->nbig = n;
+  d->big = d->bins_mem;
+  d->big_chunk = d->big + n;
+  g->graph_bytes += sizeof(uint32_t) * (2 * (size_t)n + 1);
+  compact_by_pos<<<grid_for(V, 256, g->num_sms, 16), 256, 0, s>>>(d->deg, V, d->light, pos, d->big);
+  GG_CUDA(cudaGetLastError());
+  uint32_t *hpos = nullptr, *hfirst = nullptr, *sc = nullptr;
+  GG_TRY(tmp.get(&hpos, 2 * ((size_t)n + 1) + scan_scratch_elems(n)));
+  hfirst = hpos + n + 1;
+  sc = hfirst + n + 1;
+  GG_CUDA((exclusive_scan<uint32_t, AlignedChunkCount>(AlignedChunkCount{d->big, d->off, d->chunk}, n, d->big_chunk,
+                                                       sc, s, nullptr)));
+  GG_CUDA((exclusive_scan<uint32_t, HeavyCount>(HeavyCount{d->big, d->deg, 0}, n, hpos, sc, s, nullptr)));
+  GG_CUDA((exclusive_scan<uint32_t, HeavyCount>(HeavyCount{d->big, d->deg, HEAVY_CHUNK}, n, hfirst, sc, s, nullptr)));
+  uint32_t tot[3] = {0, 0, 0};
+  GG_CUDA(cudaMemcpyAsync(&tot[0], d->big_chunk + n, sizeof(uint32_t), cudaMemcpyDeviceToHost, s));
+  GG_CUDA(cudaMemcpyAsync(&tot[1], hpos + n, sizeof(uint32_t), cudaMemcpyDeviceToHost, s));
+  GG_CUDA(cudaMemcpyAsync(&tot[2], hfirst + n, sizeof(uint32_t), cudaMemcpyDeviceToHost, s));
+  GG_CUDA(cudaStreamSynchronize(s));
+  const size_t nmed = n - tot[1], words = (size_t)tot[0] + tot[2] + nmed + 2 * (size_t)tot[1] + 1;
+  GG_CUDA(cudaMalloc(&d->owner_mem, sizeof(uint32_t) * words));
+  g->graph_bytes += sizeof(uint32_t) * words;
+  d->owner_words = words;
+  d->nbigchunks = tot[0];
+  d->nheavy = tot[1];
+  d->nchunks = tot[2];
+  d->nmed = (uint32_t)nmed;
+  d->big_owner = d->owner_mem;
+  d->chunk_owner = d->big_owner + tot[0];
+  d->med = d->chunk_owner + tot[2];
+  d->heavy = d->med + nmed;
+  d->heavy_chunk = d->heavy + tot[1];
+  fill_chunk_owner<<<grid_for(n, 128, g->num_sms, 8), 128, 0, s>>>(d->big_chunk, n, d->big_owner);
+  split_heavy<<<grid_for(n, 256, g->num_sms, 8), 256, 0, s>>>(d->big, n, d->deg, hpos, hfirst, d->med, d->heavy,
+                                                             d->heavy_chunk);
+  if (tot[1]) fill_chunk_owner<<<grid_for(tot[1], 128, g->num_sms, 8), 128, 0, s>>>(d->heavy_chunk, tot[1],
+                                                                                  d->chunk_owner);
+  GG_CUDA(cudaGetLastError());
+  GG_CUDA(cudaStreamSynchronize(s));
   return GG_OK;
 }
 
 static void free_bins(gg_graph *g, Dir *d) {
-  g->graph_bytes -= sizeof(uint32_t) * ((size_t)d->nmed + d->nheavy + d->nheavy + 1 + d->nchunks + d->nbig +
-                                        d->nbig + 1 + d->nbigchunks);
-  uint32_t *lists[] = {d->med, d->heavy, d->heavy_chunk, d->chunk_owner, d->big, d->big_chunk, d->big_owner};
-  for (uint32_t *p : lists)
-    if (p) cudaFree(p);
+  if (d->bins_mem) g->graph_bytes -= sizeof(uint32_t) * (2 * (size_t)d->nbig + 1);
+  g->graph_bytes -= sizeof(uint32_t) * d->owner_words;
+  if (d->bins_mem) cudaFree(d->bins_mem);
+  if (d->owner_mem) cudaFree(d->owner_mem);
+  d->bins_mem = d->owner_mem = nullptr;
+  d->owner_words = 0;
   d->med = d->heavy = d->heavy_chunk = d->chunk_owner = d->big = d->big_chunk = d->big_owner = nullptr;
   d->nmed = d->nheavy = d->nchunks = d->nbig = d->nbigchunks = 0;
 }
@@ -610,12 +503,9 @@ int finish_dir(gg_graph *g, Dir *d) {
   return build_bins(g, d);
 }
 
-// Builds one direction from keys already written by make_keys.
-static int build_dir(gg_graph *g, uint64_t *keys, uint32_t *vals, uint64_t *k_alt, uint32_t *v_alt, size_t n,
-                     int bits, Dir *d, bool weights = true, bool host = false) {
-  uint64_t *ks;
-  uint32_t *vs;
-  GG_TRY(radix_sort(g, keys, vals, k_alt, v_alt, n, 2 * bits, &ks, &vs));
+// One direction from its n sorted keys (see offsets_from_keys): offsets,
+// neighbours, degrees and bins.  The weights, if any, are in place.
+static int emit_dir(gg_graph *g, const uint64_t *keys, size_t n, int bits, bool low_major, Dir *d, bool host) {
   uint32_t V = g->V;
   GG_CUDA(cudaMalloc(&d->off, sizeof(uint64_t) * ((size_t)V + 1)));
   // padded to a multiple of 64 entries: chunked pulls load whole aligned
@@ -628,14 +518,23 @@ static int build_dir(gg_graph *g, uint64_t *keys, uint32_t *vals, uint64_t *k_al
   if (n == 0) {
     GG_CUDA(cudaMemsetAsync(d->off, 0, sizeof(uint64_t) * ((size_t)V + 1), g->stream));
   } else {
-    offsets_from_keys<<<grid_for(n, 256, g->num_sms, 16), 256, 0, g->stream>>>(ks, n, bits, V, d->off, d->nbr);
+    offsets_from_keys<<<grid_for(n, 256, g->num_sms, 16), 256, 0, g->stream>>>(keys, n, bits, low_major, V, d->off,
+                                                                               d->nbr);
     GG_CUDA(cudaGetLastError());
   }
-  if (g->weighted && weights) {
-    GG_TRY(adj_alloc(g, host, (void **)&d->w, sizeof(float) * (n ? n : 1)));
-    if (n) GG_CUDA(cudaMemcpyAsync(d->w, vs, sizeof(float) * n, cudaMemcpyDefault, g->stream));
-  }
   return finish_dir(g, d);
+}
+
+// Sorts keys (and weights, values vin moved between b0 and b1) on the key
+// bits [0, hi_bit) and emits the direction.  The last pass writes the
+// weights where they stay, in device memory; host adjacency takes a copy.
+static int sort_dir(gg_graph *g, void *scratch, uint64_t *ka, uint64_t *kb, uint32_t *vin, uint32_t *b0, uint32_t *b1,
+                    size_t n, int bits, bool low_major, Dir *d, bool host, uint64_t **ks, uint32_t **vs) {
+  if (vin) GG_TRY(adj_alloc(g, host, (void **)&d->w, sizeof(float) * (n ? n : 1)));
+  SortValues v{vin, b0, b1, host ? nullptr : (uint32_t *)d->w};
+  GG_TRY(radix_sort(g, scratch, ka, kb, v, n, 0, low_major ? bits : 2 * bits, ks, vs));
+  if (vin && host && n) GG_CUDA(cudaMemcpyAsync(d->w, *vs, sizeof(float) * n, cudaMemcpyDefault, g->stream));
+  return emit_dir(g, *ks, n, bits, low_major, d, host);
 }
 
 static void free_dir(Dir *d, bool adj_host) {
@@ -644,13 +543,8 @@ static void free_dir(Dir *d, bool adj_host) {
   adj_release(adj_host, d->w);
   if (d->deg) cudaFree(d->deg);
   if (d->nz) cudaFree(d->nz);
-  if (d->med) cudaFree(d->med);
-  if (d->heavy) cudaFree(d->heavy);
-  if (d->heavy_chunk) cudaFree(d->heavy_chunk);
-  if (d->chunk_owner) cudaFree(d->chunk_owner);
-  if (d->big) cudaFree(d->big);
-  if (d->big_chunk) cudaFree(d->big_chunk);
-  if (d->big_owner) cudaFree(d->big_owner);
+  if (d->bins_mem) cudaFree(d->bins_mem);
+  if (d->owner_mem) cudaFree(d->owner_mem);
   *d = Dir();
 }
 
@@ -683,27 +577,65 @@ __global__ void rank_tables(const uint64_t *__restrict__ keys, uint32_t V, int b
   }
 }
 
-// keys[k] = (rank(v) << bits) | rank(nbr[k]) for every entry k of v's in-list:
-// lane per vertex for lists up to d.light, warp per long-list chunk.
-__global__ void rank_edge_keys_light(Dir d, uint32_t V, int bits, const uint32_t *__restrict__ rank_of,
-                                     uint64_t *__restrict__ keys) {
-  for (size_t v = (size_t)blockIdx.x * blockDim.x + threadIdx.x; v < V; v += (size_t)gridDim.x * blockDim.x) {
-    const uint64_t b = d.off[v], e = d.off[v + 1];
-    if (e - b > d.light) continue;
-    const uint64_t hi = (uint64_t)rank_of[v] << bits;
-    for (uint64_t k = b; k < e; k++) keys[k] = hi | rank_of[nbr_at(d, k, GG_SITE)];
-  }
-}
-
-__global__ void rank_edge_keys_big(Dir d, int bits, const uint32_t *__restrict__ rank_of,
-                                   uint64_t *__restrict__ keys) {
-  const size_t nwarps = (size_t)gridDim.x * (blockDim.x / 32);
-  for (size_t c = ((size_t)blockIdx.x * blockDim.x + threadIdx.x) / 32; c < d.nbigchunks; c += nwarps) {
-    uint32_t v;
-    unsigned long long lo, b, e;
-    big_range(d, (uint32_t)c, d.chunk, &v, &lo, &b, &e);
-    const uint64_t hi = (uint64_t)rank_of[v] << bits;
-    for (unsigned long long k = b + lane_id(); k < e; k += 32) keys[k] = hi | rank_of[nbr_at(d, k, GG_SITE)];
+// Entry p of the lists taken in the order list_of[0], list_of[1], ... (null:
+// 0, 1, ...), list r at first[r]: keys[p] = (r << bits) | rank_of[its
+// neighbour] (rank_of null: the neighbour), vals[p] = its weight.  Tiles of
+// consecutive p, each thread finding its list by binary search in the tile's
+// slice of `first` in shared memory, so reads of long lists and all writes
+// are coalesced.  Lists from nlist on are empty.
+constexpr int EX_THREADS = 256;
+constexpr int EX_TILE = 2048;
+__global__ void __launch_bounds__(EX_THREADS)
+    expand_keys(Dir d, const uint64_t *__restrict__ first, uint32_t nlist, const uint32_t *__restrict__ list_of,
+                const uint32_t *__restrict__ rank_of, size_t n, int bits, uint64_t *__restrict__ keys,
+                uint32_t *__restrict__ vals) {
+  __shared__ uint64_t s_first[EX_TILE + 1];
+  __shared__ uint64_t s_off[EX_TILE + 1];
+  __shared__ uint32_t s_lo, s_hi;
+  const size_t ntiles = (n + EX_TILE - 1) / EX_TILE;
+  for (size_t tile = blockIdx.x; tile < ntiles; tile += gridDim.x) {
+    const uint64_t p0 = tile * EX_TILE, p1 = p0 + EX_TILE < n ? p0 + EX_TILE : n;
+    if (threadIdx.x < 2) {
+      // the list holding entry x: the last r with first[r] <= x
+      const uint64_t x = threadIdx.x ? p1 - 1 : p0;
+      uint32_t lo = 0, hi = nlist - 1;
+      while (lo < hi) {
+        const uint32_t mid = lo + (hi - lo + 1) / 2;
+        if (first[mid] <= x)
+          lo = mid;
+        else
+          hi = mid - 1;
+      }
+      if (threadIdx.x)
+        s_hi = lo;
+      else
+        s_lo = lo;
+    }
+    __syncthreads();
+    const uint32_t lo = s_lo, cnt = s_hi - s_lo + 1;
+    const bool staged = cnt <= EX_TILE;
+    if (staged)
+      for (uint32_t i = threadIdx.x; i < cnt; i += EX_THREADS) {
+        s_first[i] = first[lo + i];
+        s_off[i] = d.off[list_of ? list_of[lo + i] : lo + i];
+      }
+    __syncthreads();
+    for (uint64_t p = p0 + threadIdx.x; p < p1; p += EX_THREADS) {
+      uint32_t a = 0, b = cnt - 1;
+      while (a < b) {
+        const uint32_t mid = a + (b - a + 1) / 2;
+        if ((staged ? s_first[mid] : first[lo + mid]) <= p)
+          a = mid;
+        else
+          b = mid - 1;
+      }
+      const uint64_t k = staged ? s_off[a] + (p - s_first[a])
+                                : d.off[list_of ? list_of[lo + a] : lo + a] + (p - first[lo + a]);
+      const uint32_t u = nbr_at(d, k, GG_SITE);
+      keys[p] = ((uint64_t)(lo + a) << bits) | (rank_of ? rank_of[u] : u);
+      if (vals) vals[p] = __float_as_uint(d.w[k]);
+    }
+    __syncthreads();
   }
 }
 
@@ -731,48 +663,44 @@ void pr_layout_free(gg_graph *g) {
   if (g->pr_out_ready) free_hot_dir(g, &g->pr_out);
   g->pr_out_ready = false;
   cudaFree(g->pr_rank_of);
-  cudaFree(g->pr_id_of_rank);
-  cudaFree(g->pr_od);
   g->pr_rank_of = g->pr_id_of_rank = g->pr_od = nullptr;
   g->pr_ready = false;
 }
 
-// src renumbered: list of rank r = the list of vertex id_of_rank[r], its
-// entries' neighbour ranks sorted ascending (weights carried along), built by
-// the load's radix sort.
-static int hot_dir(gg_graph *g, const Dir &src, Dir *dst, bool weights) {
-  const uint32_t V = g->V;
+// The transpose of src's lists taken in the order of list_of, as a direction:
+// its list r' holds the numbers r of the lists that hold r', ascending.  The
+// expansion walks the lists in ascending number, so one stable sort on the
+// other end's number alone orders both (half the passes of a sort on the
+// pair).  Weights are carried along; duplicate edges keep src's order.
+// first: V + 1 positions of the lists in that order.
+static int transpose_dir(gg_graph *g, const Dir &src, const uint64_t *first, const uint32_t *list_of,
+                         const uint32_t *rank_of, Dir *dst) {
   const size_t n = g->nadj;
-  const int bits = bits_for(V);
+  const int bits = bits_for(g->V);
   DevScratch tmp;
-  uint64_t *k0 = nullptr, *k1 = nullptr;
-  uint32_t *v0 = nullptr, *v1 = nullptr;
-  GG_TRY(tmp.get(&k0, n));
-  GG_TRY(tmp.get(&k1, n));
-  if (weights) {
-    GG_TRY(tmp.get(&v0, n));
-    GG_TRY(tmp.get(&v1, n));
-    if (n) GG_CUDA(cudaMemcpyAsync(v0, src.w, sizeof(float) * n, cudaMemcpyDefault, g->stream));
+  uint64_t *k0 = nullptr, *k1 = nullptr, *ks = nullptr;
+  uint32_t *v0 = nullptr, *v1 = nullptr, *vs = nullptr;
+  void *scratch = nullptr;
+  GG_TRY(tmp.sort_buffers(n, g->weighted != 0, &k0, &k1, &v0, &v1, &scratch));
+  if (n) {
+    expand_keys<<<grid_for((n + EX_TILE - 1) / EX_TILE * EX_THREADS, EX_THREADS, g->num_sms, 6), EX_THREADS, 0,
+                  g->stream>>>(src, first, g->V, list_of, rank_of, n, bits, k0, v0);
+    GG_CUDA(cudaGetLastError());
   }
-  rank_edge_keys_light<<<grid_for(V, 256, g->num_sms, 16), 256, 0, g->stream>>>(src, V, bits, g->pr_rank_of, k0);
-  if (src.nbigchunks)
-    rank_edge_keys_big<<<grid_for((size_t)src.nbigchunks * 32, 256, g->num_sms, 16), 256, 0, g->stream>>>(
-        src, bits, g->pr_rank_of, k0);
-  GG_CUDA(cudaGetLastError());
   *dst = Dir();
   dst->light = src.light;
   dst->chunk = src.chunk;
   dst->vec = src.vec;
-  GG_TRY(build_dir(g, k0, v0, k1, v1, n, bits, dst, weights, false));
-  GG_CUDA(cudaStreamSynchronize(g->stream));
-  return GG_OK;
+  return sort_dir(g, scratch, k0, k1, v0, v0, v1, n, bits, true, dst, false, &ks, &vs);
 }
 
+// The outgoing adjacency in the hot-source numbering: the transpose of the
+// renumbered incoming one.
 int hot_out_build(gg_graph *g) {
   if (g->pr_out_ready) return GG_OK;
   GG_TRY(pr_layout_build(g));
   GG_CUDA(cudaSetDevice(g->device));
-  const int s = hot_dir(g, g->out, &g->pr_out, g->weighted != 0);
+  const int s = transpose_dir(g, g->pr, g->pr.off, nullptr, nullptr, &g->pr_out);
   if (s != GG_OK) {
     free_hot_dir(g, &g->pr_out);
     return s;
@@ -781,50 +709,54 @@ int hot_out_build(gg_graph *g) {
   return GG_OK;
 }
 
+// The vertices ranked by descending out-degree (equal degrees by id): the
+// three tables and the positions of the out-lists taken in that order.
+static int rank_vertices(gg_graph *g, uint64_t *first) {
+  const uint32_t V = g->V;
+  const int bits = bits_for(V);
+  int dbits = 1;
+  while (dbits < 32 && (1ull << dbits) <= g->nadj) dbits++;
+  const uint32_t dmax = dbits >= 32 ? 0xFFFFFFFFu : (uint32_t)((1ull << dbits) - 1);
+  DevScratch tmp;
+  uint64_t *k0 = nullptr, *k1 = nullptr, *ks = nullptr;
+  uint32_t *v0 = nullptr, *v1 = nullptr, *vs = nullptr;
+  void *scratch = nullptr;
+  uint64_t *scan = nullptr;
+  GG_TRY(tmp.sort_buffers(V, false, &k0, &k1, &v0, &v1, &scratch));
+  GG_TRY(tmp.get(&scan, scan_scratch_elems(V)));
+  degree_rank_keys<<<grid_for(V, 256, g->num_sms, 16), 256, 0, g->stream>>>(g->out.deg, V, bits, dmax, k0);
+  GG_CUDA(cudaGetLastError());
+  // the keys start in id order and the sort is stable: the degree bits suffice
+  GG_TRY(radix_sort(g, scratch, k0, k1, SortValues(), V, bits, bits + dbits, &ks, &vs));
+  rank_tables<<<grid_for(V, 256, g->num_sms, 16), 256, 0, g->stream>>>(ks, V, bits, g->out.deg, g->pr_id_of_rank,
+                                                                      g->pr_rank_of, g->pr_od);
+  GG_CUDA(cudaGetLastError());
+  GG_CUDA((exclusive_scan<uint64_t, U32AsU64>(U32AsU64{g->pr_od}, V, first, scan, g->stream, nullptr)));
+  GG_CUDA(cudaStreamSynchronize(g->stream));
+  return GG_OK;
+}
+
 int pr_layout_build(gg_graph *g) {
   if (g->pr_ready) return GG_OK;
   GG_CUDA(cudaSetDevice(g->device));
   const uint32_t V = g->V;
-  const size_t n = g->nadj;
-  const int bits = bits_for(V);
-  int dbits = 1;
-  while (dbits < 32 && (1ull << dbits) <= n) dbits++;
-  const uint32_t dmax = dbits >= 32 ? 0xFFFFFFFFu : (uint32_t)((1ull << dbits) - 1);
-  const size_t nk = V;  // degree keys of the ranking sort
-  uint64_t *k0 = nullptr, *k1 = nullptr;
-  GG_CUDA(cudaMalloc(&g->pr_rank_of, sizeof(uint32_t) * V));
-  GG_CUDA(cudaMalloc(&g->pr_id_of_rank, sizeof(uint32_t) * V));
-  GG_CUDA(cudaMalloc(&g->pr_od, sizeof(uint32_t) * V));
+  GG_CUDA(cudaMalloc(&g->pr_rank_of, sizeof(uint32_t) * 3 * (size_t)V));
+  g->pr_id_of_rank = g->pr_rank_of + V;
+  g->pr_od = g->pr_id_of_rank + V;
   g->graph_bytes += sizeof(uint32_t) * 3 * (size_t)V;
-  int status = GG_OK;
-  cudaError_t e = cudaMalloc(&k0, sizeof(uint64_t) * (nk ? nk : 1));
-  if (e == cudaSuccess) e = cudaMalloc(&k1, sizeof(uint64_t) * (nk ? nk : 1));
-  if (e != cudaSuccess) status = cuda_status(e, "PageRank layout keys");
-  uint64_t *ks = nullptr;
-  uint32_t *vs = nullptr;
+  DevScratch tmp;
+  uint64_t *first = nullptr;
+  int status = tmp.get(&first, (size_t)V + 1);
+  if (status == GG_OK) status = rank_vertices(g, first);
+  // the incoming adjacency renumbered (the transpose of the out-lists in
+  // rank order), with its weights when the graph has them (SSSP's pulls
+  // gather them)
   if (status == GG_OK) {
-    degree_rank_keys<<<grid_for(V, 256, g->num_sms, 16), 256, 0, g->stream>>>(g->out.deg, V, bits, dmax, k0);
-    status = radix_sort(g, k0, nullptr, k1, nullptr, V, bits + dbits, &ks, &vs);
-  }
-  if (status == GG_OK) {
-    rank_tables<<<grid_for(V, 256, g->num_sms, 16), 256, 0, g->stream>>>(ks, V, bits, g->out.deg,
-                                                                        g->pr_id_of_rank, g->pr_rank_of, g->pr_od);
-    e = cudaGetLastError();
-    if (e != cudaSuccess) status = cuda_status(e, "PageRank layout");
-  }
-  cudaStreamSynchronize(g->stream);
-  if (k0) cudaFree(k0);
-  if (k1) cudaFree(k1);
-  // the incoming adjacency renumbered, with its weights when the graph has
-  // them (SSSP's pulls gather them)
-  if (status == GG_OK) {
-    status = hot_dir(g, g->in, &g->pr, g->weighted != 0);
+    status = transpose_dir(g, g->out, first, g->pr_id_of_rank, g->pr_rank_of, &g->pr);
     if (status != GG_OK) free_hot_dir(g, &g->pr);
   }
   if (status != GG_OK) {
     cudaFree(g->pr_rank_of);
-    cudaFree(g->pr_id_of_rank);
-    cudaFree(g->pr_od);
     g->graph_bytes -= sizeof(uint32_t) * 3 * (size_t)V;
     g->pr_rank_of = g->pr_id_of_rank = g->pr_od = nullptr;
     return status;
@@ -909,51 +841,39 @@ int build_from_device_records(gg_graph *g, const uint32_t *rec, uint64_t E) {
               (unsigned long long)n);
     return GG_ERR_TOO_LARGE;
   }
-  int bits = bits_for(g->V);
-  uint64_t *k0 = nullptr, *k1 = nullptr;
-  uint32_t *v0 = nullptr, *v1 = nullptr;
+  const int bits = bits_for(g->V);
+  const bool host = g->adj_host != 0;
+  DevScratch tmp;
+  uint64_t *k0 = nullptr, *k1 = nullptr, *ks = nullptr;
+  uint32_t *v0 = nullptr, *v1 = nullptr, *vs = nullptr;
+  void *scratch = nullptr;
   unsigned *err = nullptr;
-  int status = GG_OK;
-  cudaError_t e = cudaMalloc(&k0, sizeof(uint64_t) * (n ? n : 1));
-  if (e == cudaSuccess) e = cudaMalloc(&k1, sizeof(uint64_t) * (n ? n : 1));
-  if (e == cudaSuccess && g->weighted) e = cudaMalloc(&v0, sizeof(uint32_t) * (n ? n : 1));
-  if (e == cudaSuccess && g->weighted) e = cudaMalloc(&v1, sizeof(uint32_t) * (n ? n : 1));
-  if (e == cudaSuccess) e = cudaMalloc(&err, sizeof(unsigned));
-  if (e == cudaSuccess) e = cudaMemsetAsync(err, 0, sizeof(unsigned), g->stream);
-  if (e != cudaSuccess) status = cuda_status(e, "build buffers");
-  unsigned blocks = grid_for(E, 256, g->num_sms, 16);
-  for (int pass = 0; status == GG_OK && pass < (g->symmetric ? 1 : 2); pass++) {
-    int mode = g->symmetric ? 2 : pass;
-    if (E) {
-      make_keys<<<blocks, 256, 0, g->stream>>>(rec, E, words, mode, bits, g->V, k0, v0, err);
-      e = cudaGetLastError();
-      if (e != cudaSuccess) {
-        status = cuda_status(e, "make_keys");
-        break;
-      }
-      unsigned herr = 0;
-      e = cudaMemcpyAsync(&herr, err, sizeof(unsigned), cudaMemcpyDeviceToHost, g->stream);
-      if (e == cudaSuccess) e = cudaStreamSynchronize(g->stream);
-      if (e != cudaSuccess) {
-        status = cuda_status(e, "make_keys");
-        break;
-      }
-      if (herr) {
-        set_error("an edge names a vertex id >= vertices (%u)", g->V);
-        status = GG_ERR_RANGE;
-        break;
-      }
+  GG_TRY(tmp.sort_buffers(n, g->weighted != 0, &k0, &k1, &v0, &v1, &scratch));
+  GG_TRY(tmp.get(&err, 1));
+  GG_CUDA(cudaMemsetAsync(err, 0, sizeof(unsigned), g->stream));
+  if (E) {
+    make_keys<<<grid_for(E, 256, g->num_sms, 16), 256, 0, g->stream>>>(rec, E, words, g->symmetric ? 2 : 0, bits,
+                                                                       g->V, k0, v0, err);
+    GG_CUDA(cudaGetLastError());
+    unsigned herr = 0;
+    GG_CUDA(cudaMemcpyAsync(&herr, err, sizeof(unsigned), cudaMemcpyDeviceToHost, g->stream));
+    GG_CUDA(cudaStreamSynchronize(g->stream));
+    if (herr) {
+      set_error("an edge names a vertex id >= vertices (%u)", g->V);
+      return GG_ERR_RANGE;
     }
-    status = build_dir(g, k0, v0, k1, v1, n, bits, pass == 0 ? &g->out : &g->in, true, g->adj_host != 0);
   }
-  cudaStreamSynchronize(g->stream);
-  cudaFree(k0);
-  cudaFree(k1);
-  if (v0) cudaFree(v0);
-  if (v1) cudaFree(v1);
-  if (err) cudaFree(err);
-  if (status == GG_OK && g->symmetric) g->in = g->out;
-  return status;
+  GG_TRY(sort_dir(g, scratch, k0, k1, v0, v0, v1, n, bits, false, &g->out, host, &ks, &vs));
+  if (g->symmetric) {
+    g->in = g->out;
+  } else {
+    // the CSC from the CSR's order (source, destination, record): a stable
+    // sort on the destination bits alone gives (destination, source, record)
+    uint32_t *b0 = vs == v1 ? v1 : v0, *b1 = vs == v1 ? v0 : v1;
+    GG_TRY(sort_dir(g, scratch, ks, ks == k0 ? k1 : k0, vs, b0, b1, n, bits, true, &g->in, host, &ks, &vs));
+  }
+  GG_CUDA(cudaStreamSynchronize(g->stream));
+  return GG_OK;
 }
 
 static uint64_t unit_of(int weighted) { return weighted ? 12 : 8; }
