@@ -384,11 +384,7 @@ __global__ void __launch_bounds__(PUSH_THREADS)
   for (unsigned long long tile = blockIdx.x; tile < ntiles; tile += gridDim.x) {
     const unsigned long long e0 = tile * PUSH_TILE;
     const unsigned long long e1 = e0 + PUSH_TILE < total ? e0 + PUSH_TILE : total;
-    if (threadIdx.x == 0) {
-      uint32_t lo = upper_bound_idx<unsigned long long>(P, 0, n + 1, e0) - 1;
-      s_lo = lo;
-      s_hi = upper_bound_idx<unsigned long long>(P, lo, n + 1, e1 - 1);
-    }
+    tile_bounds(P, n, e0, e1, &s_lo, &s_hi);
     __syncthreads();
     const uint32_t lo = s_lo, hi = s_hi;
     __syncthreads();
@@ -814,11 +810,7 @@ __global__ void __launch_bounds__(PUSH_THREADS)
   for (unsigned long long tile = blockIdx.x; tile < ntiles; tile += gridDim.x) {
     const unsigned long long e0 = tile * PUSH_TILE;
     const unsigned long long e1 = e0 + PUSH_TILE < total ? e0 + PUSH_TILE : total;
-    if (threadIdx.x == 0) {
-      uint32_t lo = upper_bound_idx<unsigned long long>(P, 0, n + 1, e0) - 1;
-      s_lo = lo;
-      s_hi = upper_bound_idx<unsigned long long>(P, lo, n + 1, e1 - 1);
-    }
+    tile_bounds(P, n, e0, e1, &s_lo, &s_hi);
     __syncthreads();
     const uint32_t lo = s_lo, hi = s_hi, cnt = hi - lo;
     const bool staged = cnt <= (uint32_t)PUSH_STAGE;
@@ -899,11 +891,7 @@ __global__ void __launch_bounds__(PUSH_THREADS, 8)
   for (unsigned long long tile = blockIdx.x; tile < ntiles; tile += gridDim.x) {
     const unsigned long long e0 = tile * PUSH_TILE;
     const unsigned long long e1 = e0 + PUSH_TILE < total ? e0 + PUSH_TILE : total;
-    if (threadIdx.x == 0) {
-      uint32_t lo = upper_bound_idx<unsigned long long>(P, 0, n + 1, e0) - 1;
-      s_lo = lo;
-      s_hi = upper_bound_idx<unsigned long long>(P, lo, n + 1, e1 - 1);
-    }
+    tile_bounds(P, n, e0, e1, &s_lo, &s_hi);
     __syncthreads();
     const uint32_t lo = s_lo, hi = s_hi, cnt = hi - lo;
     const bool staged = cnt <= (uint32_t)PUSH_STAGE;

@@ -144,11 +144,21 @@ struct PrPull {
   const uint32_t *out_deg;
   int last;
   uint32_t hot = 0xffffffffu;  // sources below this number are gathered through L1
+  int zeros_done = 0;          // both buffers hold the vertices without in-edges
+  static constexpr bool kDelta = true;
+  static constexpr bool kDense = true;  // curr[V] is 0
+  static constexpr bool kCompensated = sizeof(T) == 4;
   __device__ __forceinline__ bool want(uint32_t) const { return true; }
+  __host__ __device__ __forceinline__ bool zero_kept() const { return zeros_done; }
   __device__ __forceinline__ T identity(uint32_t) const { return T(0); }
   __device__ __forceinline__ T identity_coop() const { return T(0); }
   __device__ __forceinline__ T gather(const Dir &, unsigned long long, uint32_t u) const {
     return ld_gather(curr, u, hot);
+  }
+  __host__ __forceinline__ bool gathers_all(uint32_t V) const { return hot >= V; }
+  template <bool ALL>
+  __device__ __forceinline__ T value(uint32_t u, float) const {
+    return ALL ? curr[u] : ld_gather(curr, u, hot);
   }
   __device__ __forceinline__ T combine(T a, T b) const { return a + b; }
   __device__ __forceinline__ T warp_combine(T x) const { return warp_sum(x); }
@@ -180,17 +190,20 @@ __device__ __forceinline__ bool PrPull<float>::finish(uint32_t v, float sum, uin
     uint32_t od = out_deg[v];
     if (od > 0) {
       nv = __fdiv_rn(nv, (float)od);
-      t.delta += (double)fabsf(__fadd_rn(nv, -curr[v])) * (double)od;
+      t.add_delta(fabsf(__fadd_rn(nv, -curr[v])), od);
     } else {
-      t.delta += (double)fabsf(__fadd_rn(nv, -curr[v]));
+      t.add_delta(fabsf(__fadd_rn(nv, -curr[v])), 1);
     }
   }
   next[v] = nv;
   return false;
 }
 
+// curr = 1 / out-degree (1 where it is 0); both buffers are 0 at V, where the
+// rows' empty places point.
 template <typename T>
-__global__ void pr_init(T *curr, const uint32_t *out_deg, uint32_t V) {
+__global__ void pr_init(T *curr, T *other, const uint32_t *out_deg, uint32_t V) {
+  if (blockIdx.x == 0 && threadIdx.x == 0) curr[V] = other[V] = T(0);
   for (size_t v = (size_t)blockIdx.x * blockDim.x + threadIdx.x; v < V; v += (size_t)gridDim.x * blockDim.x) {
     uint32_t od = out_deg[v];
     curr[v] = od > 0 ? T(1) / (T)od : T(1);
@@ -224,8 +237,8 @@ static int pr_run(gg_graph *g, int iterations, T *ranks_host, double *deltas_hos
   T *buf[2], *out = nullptr;
   Counters *per_iter;
   if (ranked) GG_TRY(ws(g, WS_S0, (size_t)V, &out));
-  GG_TRY(ws(g, WS_S2, (size_t)V, &buf[0]));
-  GG_TRY(ws(g, WS_S3, (size_t)V, &buf[1]));
+  GG_TRY(ws(g, WS_S2, (size_t)V + 1, &buf[0]));
+  GG_TRY(ws(g, WS_S3, (size_t)V + 1, &buf[1]));
   GG_TRY(ws(g, WS_HUBSUM, (size_t)(iterations > 0 ? iterations : 1), &per_iter));
   Launch L(g);
   Trace tr(st, g, "gg_pagerank");
@@ -261,7 +274,7 @@ static int pr_run(gg_graph *g, int iterations, T *ranks_host, double *deltas_hos
   auto enqueue = [&](bool launch) -> int {
     if (launch) {
       GG_CUDA(cudaMemsetAsync(per_iter, 0, sizeof(Counters) * (iterations > 0 ? iterations : 1), s));
-      pr_init<T><<<grid_for(V, 256, g->num_sms), 256, 0, s>>>(buf[0], od, V);
+      pr_init<T><<<grid_for(V, 256, g->num_sms), 256, 0, s>>>(buf[0], buf[1], od, V);
     }
     L.launches += 1;
     cur = 0;
@@ -269,7 +282,10 @@ static int pr_run(gg_graph *g, int iterations, T *ranks_host, double *deltas_hos
     unsigned long long ae = g->nadj;
     for (int i = 0; i < iterations; i++) {
       tr.add(ae < g->E / 20 ? 0 : 1, ae, V);
-      PrPull<T> op{buf[cur], buf[cur ^ 1], od, i == iterations - 1, hot};
+      // a vertex without in-edges has one value from iteration 0 on (its
+      // delta is 0 then), written to either buffer by iterations 0 and 1;
+      // the last iteration writes it undivided
+      PrPull<T> op{buf[cur], buf[cur ^ 1], od, i == iterations - 1, hot, i >= 2 && i < iterations - 1};
       GG_TRY(tr.kbegin());
       if (launch)
         GG_TRY(L.pull(din, op, ActOut(), per_iter + i));

@@ -31,10 +31,17 @@ struct CcPull {
   const uint32_t *ids = nullptr;  // hot-source layout: vertex id of each rank (the message starts at dst's id)
   uint32_t hot = 0xffffffffu;     // sources below this number are gathered through L1
   __device__ __forceinline__ bool want(uint32_t) const { return true; }
+  // no call changes a vertex without in-edges: both buffers hold its label
+  __host__ __device__ __forceinline__ bool zero_kept() const { return true; }
   __device__ __forceinline__ uint32_t identity(uint32_t v) const { return ids ? ids[v] : v; }
   __device__ __forceinline__ uint32_t identity_coop() const { return 0xffffffffu; }
   __device__ __forceinline__ uint32_t gather(const Dir &, unsigned long long, uint32_t u) const {
     return ld_gather(cur, u, hot);
+  }
+  __host__ __forceinline__ bool gathers_all(uint32_t V) const { return hot >= V; }
+  template <bool ALL>
+  __device__ __forceinline__ uint32_t value(uint32_t u, float) const {
+    return ALL ? cur[u] : ld_gather(cur, u, hot);
   }
   __device__ __forceinline__ uint32_t combine(uint32_t a, uint32_t b) const { return b < a ? b : a; }
   __device__ __forceinline__ uint32_t warp_combine(uint32_t x) const { return warp_min(x); }
@@ -81,6 +88,8 @@ struct SsspPull {
   float *nxt;
   uint32_t hot = 0xffffffffu;  // sources below this number are gathered through L1
   __device__ __forceinline__ bool want(uint32_t) const { return true; }
+  // no call changes a vertex without in-edges: both buffers hold its distance
+  __host__ __device__ __forceinline__ bool zero_kept() const { return true; }
   __device__ __forceinline__ float identity(uint32_t) const { return 1e9f; }
   __device__ __forceinline__ float identity_coop() const { return 1e9f; }
   __device__ __forceinline__ float gather(const Dir &d, unsigned long long k, uint32_t u) const {
@@ -88,6 +97,11 @@ struct SsspPull {
   }
   // the same candidate with the weight read by the kernel
   __device__ __forceinline__ float gather_w(uint32_t u, float w) const { return __fadd_rn(ld_gather(cur, u, hot), w); }
+  __host__ __forceinline__ bool gathers_all(uint32_t V) const { return hot >= V; }
+  template <bool ALL>
+  __device__ __forceinline__ float value(uint32_t u, float w) const {
+    return __fadd_rn(ALL ? cur[u] : ld_gather(cur, u, hot), w);
+  }
   __device__ __forceinline__ float combine(float a, float b) const { return b < a ? b : a; }
   __device__ __forceinline__ float warp_combine(float x) const { return warp_min(x); }
   __device__ __forceinline__ bool finish(uint32_t v, float m, uint32_t, Tally &) const {
@@ -184,6 +198,16 @@ static int relax_loop(gg_graph *g, const Dir &dout, const Dir &din, const PullOp
   return GG_OK;
 }
 
+// a[v] = b[v] = src[v]
+template <typename T>
+__global__ void copy_twice(const T *__restrict__ src, size_t n, T *__restrict__ a, T *__restrict__ b) {
+  for (size_t v = (size_t)blockIdx.x * blockDim.x + threadIdx.x; v < n; v += (size_t)gridDim.x * blockDim.x) {
+    const T x = src[v];
+    a[v] = x;
+    b[v] = x;
+  }
+}
+
 // out[v] = by_rank[rank_of[v]]
 template <typename T>
 __global__ void unrank(const T *__restrict__ by_rank, const uint32_t *__restrict__ rank_of, uint32_t V,
@@ -219,11 +243,11 @@ static int cc_run(gg_graph *g, uint32_t *label_host, gg_run_stats *st) {
   GG_TRY(timed_begin(g));
   // label[v] = v over active_in = all (cc.cpp:31-37)
   if (ranked)
-    GG_CUDA(cudaMemcpyAsync(lab[0], g->pr_id_of_rank, sizeof(uint32_t) * V, cudaMemcpyDeviceToDevice, s));
+    copy_twice<uint32_t><<<grid_for(V, 256, g->num_sms), 256, 0, s>>>(g->pr_id_of_rank, V, lab[0], lab[1]);
   else
     iota_u32<<<grid_for(V, 256, g->num_sms), 256, 0, s>>>(lab[0], V);
   bitmap_fill<<<grid_for(words, 256, g->num_sms), 256, 0, s>>>(bm[0], words, V);
-  L.launches += ranked ? 1 : 2;
+  L.launches += 2;
   GG_CUDA(cudaGetLastError());
   uint32_t *res = nullptr;
   CcPull pull{};
@@ -245,9 +269,10 @@ static int cc_run(gg_graph *g, uint32_t *label_host, gg_run_stats *st) {
   return GG_OK;
 }
 
-__global__ void sssp_root(float *dist, uint32_t root, uint32_t *active, uint32_t *q, const uint32_t *out_deg,
-                          Counters *ctr) {
+__global__ void sssp_root(float *dist, float *other, uint32_t root, uint32_t *active, uint32_t *q,
+                          const uint32_t *out_deg, Counters *ctr) {
   dist[root] = 0.0f;
+  other[root] = 0.0f;
   active[root >> 5] |= 1u << (root & 31);
   q[0] = root;
   ctr->edges = out_deg[root];
@@ -299,8 +324,9 @@ static int sssp_run(gg_graph *g, uint32_t root, float *dist_host, gg_run_stats *
   GG_CUDA(cudaMemsetAsync(bm[0], 0, words * 4, s));
   GG_TRY(counters_reset(g));
   fill_kernel<float><<<grid_for(V, 256, g->num_sms), 256, 0, s>>>(dist[0], V, 1e9f);
-  sssp_root<<<1, 1, 0, s>>>(dist[0], start, bm[0], q[0], dout.deg, g->ws.ctr);
-  L.launches += 2;
+  fill_kernel<float><<<grid_for(V, 256, g->num_sms), 256, 0, s>>>(dist[1], V, 1e9f);
+  sssp_root<<<1, 1, 0, s>>>(dist[0], dist[1], start, bm[0], q[0], dout.deg, g->ws.ctr);
+  L.launches += 3;
   GG_CUDA(cudaGetLastError());
   Counters c;
   GG_TRY(counters_read(g, &c));
@@ -343,9 +369,15 @@ struct BcFwdPull {
   const uint32_t *active_in;
   const uint32_t *visited;
   __device__ __forceinline__ bool want(uint32_t v) const { return !bm_test(visited, v); }
+  __host__ __device__ __forceinline__ bool zero_kept() const { return true; }
   __device__ __forceinline__ double identity(uint32_t) const { return 0.0; }
   __device__ __forceinline__ double identity_coop() const { return 0.0; }
   __device__ __forceinline__ double gather(const Dir &, unsigned long long, uint32_t s) const {
+    return bm_test_ldg(active_in, s) ? np[s] : 0.0;
+  }
+  __host__ __forceinline__ bool gathers_all(uint32_t) const { return true; }
+  template <bool ALL>
+  __device__ __forceinline__ double value(uint32_t s, float) const {
     return bm_test_ldg(active_in, s) ? np[s] : 0.0;
   }
   __device__ __forceinline__ double combine(double a, double b) const { return a + b; }
@@ -377,9 +409,15 @@ struct BcBwdPull {
   const uint32_t *level;
   const uint32_t *visited;
   __device__ __forceinline__ bool want(uint32_t v) const { return !bm_test(visited, v); }
+  __host__ __device__ __forceinline__ bool zero_kept() const { return true; }
   __device__ __forceinline__ double identity(uint32_t) const { return 0.0; }
   __device__ __forceinline__ double identity_coop() const { return 0.0; }
   __device__ __forceinline__ double gather(const Dir &, unsigned long long, uint32_t s) const {
+    return bm_test_ldg(level, s) ? dep[s] : 0.0;
+  }
+  __host__ __forceinline__ bool gathers_all(uint32_t) const { return true; }
+  template <bool ALL>
+  __device__ __forceinline__ double value(uint32_t s, float) const {
     return bm_test_ldg(level, s) ? dep[s] : 0.0;
   }
   __device__ __forceinline__ double combine(double a, double b) const { return a + b; }
@@ -444,7 +482,7 @@ static int bc_run(gg_graph *g, uint32_t root, double *dep_host, double *inv_host
   // are exact and dependencies change only in summation order.
   if (g->pr_layout) {
     GG_TRY(pr_layout_build(g));
-    if (!g->symmetric) GG_TRY(hot_out_build(g));
+    if (!g->symmetric) GG_TRY(hot_out_rows(g));
   }
   const bool ranked = g->pr_layout && g->pr_ready && (g->symmetric || g->pr_out_ready);
   const Dir &dout = ranked ? (g->symmetric ? g->pr : g->pr_out) : g->out;

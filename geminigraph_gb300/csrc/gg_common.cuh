@@ -81,6 +81,14 @@ struct Dir {
   uint32_t *bins_mem = nullptr;     // the allocations of the bins: big, big_chunk;
   uint32_t *owner_mem = nullptr;    // the owners, med, heavy and heavy_chunk
   size_t owner_words = 0;
+  // Rows of a hot-source direction (see pull_rows): 32 consecutive vertices
+  // make a slice whose light lists are stored column-major, four entries per
+  // lane and step; desc lists the slices with entries first.
+  uint4 *sell_desc = nullptr;       // {slice, first step, steps, 0}; null: a plain direction
+  uint4 *sell_col = nullptr;        // step t, lane l: entries 4t .. 4t + 3 of the lane's list at [(first + t) * 32 + l]
+  float4 *sell_w = nullptr;         // their weights
+  uint32_t nslices = 0, nfull = 0;  // slices; slices with a vertex of degree > 0
+  uint64_t sell_steps = 0;
   // bounds of the ids and entries, and the graph's error word (GG_CHECK builds)
   uint32_t nv = 0;
   uint64_t ne = 0;
@@ -132,6 +140,7 @@ class LanePool;
 void pools_destroy(gg_graph *g);
 int pr_layout_build(gg_graph *g);
 int hot_out_build(gg_graph *g);
+int hot_out_rows(gg_graph *g);
 void pr_layout_free(gg_graph *g);
 
 }  // namespace gg
@@ -186,6 +195,9 @@ struct gg_graph {
   gg::Dir pr_out;
   bool pr_out_ready = false;
   int pr_layout = 1;                  // 0: PageRank pulls the plain incoming adjacency
+  // gg_graph_set_bins was called: the hot-source directions take its light
+  // bound and chunk size instead of their own (hot_bins)
+  int bins_set = 0;
   // batched SSSP bucket width (0: plain Bellman-Ford rounds) and the least
   // edge weight (bucketing needs none negative), found on first use
   float sssp_delta = 0.0f;
@@ -363,14 +375,16 @@ __device__ __forceinline__ unsigned lane_id() { return threadIdx.x & 31u; }
 
 // Chunk c of the long-list table: owner vertex v, aligned block start lo
 // (a multiple of chunk in the adjacency array) and the list's part [b, e)
-// inside [lo, lo + chunk).
+// inside [lo, lo + chunk).  chunk is a power of two (a 64-bit division by
+// another number costs more than the chunk's loads).
 __device__ __forceinline__ void big_range(const Dir &d, uint32_t c, uint32_t chunk, uint32_t *v,
                                           unsigned long long *lo, unsigned long long *b,
                                           unsigned long long *e) {
   const uint32_t o = d.big_owner[c];
   *v = d.big[o];
   const unsigned long long b0 = d.off[*v], e0 = d.off[*v + 1];
-  *lo = (b0 / chunk + (c - d.big_chunk[o])) * (unsigned long long)chunk;
+  const int shift = 31 - __clz(chunk);
+  *lo = ((b0 >> shift) + (c - d.big_chunk[o])) << shift;
   *b = b0 > *lo ? b0 : *lo;
   *e = e0 < *lo + chunk ? e0 : *lo + chunk;
 }
@@ -497,6 +511,24 @@ __device__ __forceinline__ T warp_min(T x) {
   return x;
 }
 
+// First index in [lo, hi) with P[i] > x (hi if none), by a whole warp: 32
+// probes a step, so 2^25 entries take 5 dependent loads instead of 25.  All
+// lanes call with the same arguments.
+template <typename T>
+__device__ __forceinline__ uint32_t warp_upper_bound(const T *P, uint32_t lo, uint32_t hi, T x) {
+  while (lo < hi) {
+    const uint32_t step = (hi - lo + 31) / 32;
+    const uint64_t at = (uint64_t)lo + (uint64_t)(lane_id() + 1) * step - 1;
+    const uint32_t p = at < hi ? (uint32_t)at : hi - 1;
+    const unsigned above = __ballot_sync(GG_FULL, P[p] > x);
+    if (!above) return hi;
+    const unsigned f = __ffs(above) - 1;
+    hi = __shfl_sync(GG_FULL, p, f);
+    lo += f * step;
+  }
+  return hi;
+}
+
 // Warp-aggregated append: every lane of the warp must call it.
 __device__ __forceinline__ void queue_push(bool pred, uint32_t v, uint32_t *q, unsigned *qlen) {
   unsigned m = __ballot_sync(GG_FULL, pred);
@@ -515,22 +547,52 @@ struct Tally {
   unsigned int activated = 0;
   unsigned int maxdeg = 0;
   double delta = 0.0;
+  // delta += x * d exactly up to 2^-46 of the sum: the product and the sum as
+  // unevaluated pairs of floats (Dekker, Knuth).  A double product and sum
+  // per vertex keeps GB300's FP64 pipe (16 cycles per warp instruction) busy
+  // for longer than the gathers take.
+  float dhi = 0.0f, dlo = 0.0f;
+  __device__ __forceinline__ void add_delta(float x, uint32_t d) {
+    if (d >> 24) {  // not a float
+      delta += (double)x * (double)d;
+      return;
+    }
+    const float df = (float)d;
+    const float p = __fmul_rn(x, df), pe = __fmaf_rn(x, df, -p);
+    const float s = __fadd_rn(dhi, p), b = __fsub_rn(s, dhi);
+    const float se = __fadd_rn(__fsub_rn(dhi, __fsub_rn(s, b)), __fsub_rn(p, b));
+    dhi = s;
+    dlo = __fadd_rn(dlo, __fadd_rn(se, pe));
+  }
+  // The block's delta into ctr (all threads call): one warp adds a value
+  // of every other warp per lane before its tree, a fraction of the FP64
+  // instructions of a tree per warp.
+  template <int THREADS>
+  __device__ __forceinline__ void flush_delta(Counters *ctr) {
+    __shared__ double s_t[THREADS];
+    s_t[threadIdx.x] = delta + ((double)dhi + (double)dlo);
+    __syncthreads();
+    if (threadIdx.x < 32) {
+      double x = s_t[threadIdx.x];
+#pragma unroll
+      for (int i = 1; i < THREADS / 32; i++) x += s_t[threadIdx.x + 32 * i];
+      x = warp_sum(x);
+      if (threadIdx.x == 0 && x != 0.0) atomicAdd(&ctr->delta, x);
+    }
+  }
   // all threads of the block must call flush
   __device__ __forceinline__ void flush(Counters *ctr) {
     __shared__ unsigned long long s_e[32], s_i[32];
     __shared__ unsigned int s_a[32], s_m[32];
-    __shared__ double s_d[32];
     unsigned long long e = warp_sum(edges), ie = warp_sum(in_edges);
     unsigned int a = warp_sum(activated);
     unsigned int m = __reduce_max_sync(GG_FULL, maxdeg);
-    double dl = warp_sum(delta);
     unsigned w = threadIdx.x >> 5, lane = lane_id();
     if (lane == 0) {
       s_e[w] = e;
       s_i[w] = ie;
       s_a[w] = a;
       s_m[w] = m;
-      s_d[w] = dl;
     }
     __syncthreads();
     if (w == 0) {
@@ -539,18 +601,15 @@ struct Tally {
       ie = lane < nw ? s_i[lane] : 0ull;
       a = lane < nw ? s_a[lane] : 0u;
       m = lane < nw ? s_m[lane] : 0u;
-      dl = lane < nw ? s_d[lane] : 0.0;
       e = warp_sum(e);
       ie = warp_sum(ie);
       a = warp_sum(a);
       m = __reduce_max_sync(GG_FULL, m);
-      dl = warp_sum(dl);
       if (lane == 0) {
         if (m) atomicMax(&ctr->maxdeg, m);
         if (e) atomicAdd(&ctr->edges, e);
         if (ie) atomicAdd(&ctr->in_edges, ie);
         if (a) atomicAdd(&ctr->activated, a);
-        if (dl != 0.0) atomicAdd(&ctr->delta, dl);
       }
     }
   }

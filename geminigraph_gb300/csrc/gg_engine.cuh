@@ -40,6 +40,17 @@ struct has_gather_w : std::false_type {};
 template <class Op>
 struct has_gather_w<Op, std::void_t<decltype(&Op::gather_w)>> : std::true_type {};
 constexpr int PUSH_THREADS = 256;
+// Ops whose finish adds to the tally's delta (PageRank).
+template <class Op, class = void>
+struct has_delta : std::false_type {};
+template <class Op>
+struct has_delta<Op, std::void_t<decltype(Op::kDelta)>> : std::true_type {};
+// The end of a pull kernel: what the op and the call tally, once per block.
+template <class Op, int THREADS>
+__device__ __forceinline__ void pull_flush(Tally &t, bool activates, Counters *ctr) {
+  if constexpr (has_delta<Op>::value) t.template flush_delta<THREADS>(ctr);
+  if (activates) t.flush(ctr);
+}
 constexpr int PUSH_TILE = 1024;              // edges per block iteration of push_lb
 constexpr int PUSH_STAGE = PUSH_TILE + 1;    // queue entries a tile spans when each has >= 1 edge
 constexpr int PULL_THREADS = 256;
@@ -106,6 +117,21 @@ __device__ __forceinline__ uint32_t upper_bound_idx(const T *P, uint32_t lo, uin
   return lo;
 }
 
+// The queue entry holding edge e0 of the prefix P and one past the entry
+// holding edge e1 - 1, by the block's first two warps (one thread's two
+// binary searches are 40 dependent loads for a queue of a million).
+__device__ __forceinline__ void tile_bounds(const unsigned long long *P, uint32_t n, unsigned long long e0,
+                                            unsigned long long e1, uint32_t *s_lo, uint32_t *s_hi) {
+  if (threadIdx.x >= 64) return;
+  const uint32_t b = warp_upper_bound<unsigned long long>(P, 0, n + 1, threadIdx.x < 32 ? e0 : e1 - 1);
+  if (lane_id() == 0) {
+    if (threadIdx.x < 32)
+      *s_lo = b - 1;
+    else
+      *s_hi = b;
+  }
+}
+
 // ---------------------------------------------------------------- push
 // Sparse mode (core/graph.hpp:1510-1663): for every queued vertex q[i] and
 // every out-edge, op.push(src, i, dst, w) applies the slot and returns
@@ -130,11 +156,7 @@ __global__ void __launch_bounds__(PUSH_THREADS)
   for (unsigned long long tile = blockIdx.x; tile < ntiles; tile += gridDim.x) {
     unsigned long long e0 = tile * PUSH_TILE;
     unsigned long long e1 = e0 + PUSH_TILE < total ? e0 + PUSH_TILE : total;
-    if (threadIdx.x == 0) {
-      uint32_t lo = upper_bound_idx<unsigned long long>(P, 0, n + 1, e0) - 1;
-      s_lo = lo;
-      s_hi = upper_bound_idx<unsigned long long>(P, lo, n + 1, e1 - 1);  // one past the entry holding e1-1
-    }
+    tile_bounds(P, n, e0, e1, &s_lo, &s_hi);
     __syncthreads();
     const uint32_t lo = s_lo, hi = s_hi, cnt = hi - lo;
     const bool staged = cnt <= (uint32_t)PUSH_STAGE;
@@ -246,7 +268,7 @@ __global__ void __launch_bounds__(PULL_THREADS) pull_light(Dir d, uint32_t V, Op
     }
     if (act.active_out) pull_activate(a, v, g, act, t);
   }
-  t.flush(ctr);
+  pull_flush<Op, PULL_THREADS>(t, act.active_out != nullptr, ctr);
 }
 
 // Lists longer than d.light: one warp per d.chunk-edge aligned block of the
@@ -348,20 +370,62 @@ __global__ void __launch_bounds__(PULL_THREADS)
     part = op.warp_combine(part);
     if (lane == 0) op.finish(v, op.combine(op.identity(v), part), d.deg[v], t);
   }
-  t.flush(ctr);
+  pull_flush<Op, PULL_THREADS>(t, false, ctr);
 }
 
-// One lane per long-list vertex combines its chunk partials in order (a warp
-// does it for vertices with more than 32 chunks), then applies the slot.
+// g[0] .. g[N - 1] (N a power of two) combined in pairs: as many operations as
+// one after another, a third of the rounding error on long lists.
+template <int N, class Op>
+__device__ __forceinline__ typename Op::Acc combine_tree(const Op &op, typename Op::Acc *g) {
+#pragma unroll
+  for (int s = 1; s < N; s *= 2)
+#pragma unroll
+    for (int j = 0; j < N; j += 2 * s) g[j] = op.combine(g[j], g[j + s]);
+  return g[0];
+}
+// The running result of a list walked a few entries at a time.  Float sums
+// (Op::kCompensated) keep the rounding errors of the additions beside the sum
+// (Knuth's two-sum): a lane now adds up to 1024 entries itself, where chunks
+// of 256 went through trees, and this leaves the ranks' error no larger (20
+// iterations, 2-norm against 64 bits, mean of R-MAT graphs of 2^20, 2^22,
+// 200003, 20001 and 1001 vertices: 6.15e-8 with the trees, 6.44e-8 without
+// the errors kept, 5.95e-8 with; no difference in time).
+template <class Op, class = void>
+struct Running {
+  typename Op::Acc a;
+  __device__ __forceinline__ explicit Running(typename Op::Acc x) : a(x) {}
+  __device__ __forceinline__ void add(const Op &op, typename Op::Acc x) { a = op.combine(a, x); }
+  __device__ __forceinline__ typename Op::Acc value() const { return a; }
+};
 template <class Op>
+struct Running<Op, std::enable_if_t<Op::kCompensated>> {
+  float a, lost = 0.0f;
+  __device__ __forceinline__ explicit Running(float x) : a(x) {}
+  __device__ __forceinline__ void add(const Op &, float x) {
+    const float s = __fadd_rn(a, x), b = __fsub_rn(s, a);
+    lost = __fadd_rn(lost, __fadd_rn(__fsub_rn(a, __fsub_rn(s, b)), __fsub_rn(x, b)));
+    a = s;
+  }
+  __device__ __forceinline__ float value() const { return __fadd_rn(a, lost); }
+};
+
+// One lane per long-list vertex combines its chunk partials in order (a warp
+// does it for vertices with more than SERIAL chunks), then applies the slot.
+// SPREAD: a warp takes vertices nwarps apart: on a hot-source direction the
+// longest lists lead, and 32 of them in one warp are combined one after
+// another (R-MAT 20: 32 us of a 75-us iteration).
+template <class Op, uint32_t SERIAL, bool SPREAD>
 __global__ void __launch_bounds__(PULL_THREADS)
     pull_big_finish(Dir d, Op op, const typename Op::Acc *__restrict__ partials, ActOut act, Counters *ctr) {
   using Acc = typename Op::Acc;
   Tally t;
   const size_t stride = (size_t)gridDim.x * PULL_THREADS;
-  const size_t n = ((size_t)d.nbig + 31) / 32 * 32;
+  const size_t n = SPREAD ? ((size_t)d.nbig + stride - 1) / stride * stride : ((size_t)d.nbig + 31) / 32 * 32;
   const unsigned lane = lane_id();
-  for (size_t i = (size_t)blockIdx.x * PULL_THREADS + threadIdx.x; i < n; i += stride) {
+  const size_t tid = (size_t)blockIdx.x * PULL_THREADS + threadIdx.x;
+  const size_t first = SPREAD ? (size_t)lane * (stride / 32) + tid / 32 : tid;
+  for (size_t base = 0; base + (SPREAD ? 0 : tid) < n; base += stride) {
+    const size_t i = base + first;
     const bool valid = i < d.nbig;
     const uint32_t v = valid ? d.big[i] : 0u;
     const bool todo = valid && op.want(v);
@@ -371,22 +435,187 @@ __global__ void __launch_bounds__(PULL_THREADS)
       c1 = d.big_chunk[i + 1];
     }
     Acc acc = op.identity(v);
-    if (todo && c1 - c0 <= 32)
-      for (uint32_t c = c0; c < c1; c++) acc = op.combine(acc, partials[c]);
-    unsigned coop = __ballot_sync(GG_FULL, todo && c1 - c0 > 32);
+    if (todo && c1 - c0 <= SERIAL) {
+      Running<Op> run(acc);
+      for (uint32_t c = c0; c < c1; c++) run.add(op, partials[c]);
+      acc = run.value();
+    }
+    unsigned coop = __ballot_sync(GG_FULL, todo && c1 - c0 > SERIAL);
     while (coop) {
       const unsigned leader = __ffs(coop) - 1;
       coop &= coop - 1;
       const uint32_t lc0 = __shfl_sync(GG_FULL, c0, leader), lc1 = __shfl_sync(GG_FULL, c1, leader);
-      Acc part = op.identity_coop();
-      for (uint32_t c = lc0 + lane; c < lc1; c += 32) part = op.combine(part, partials[c]);
-      part = op.warp_combine(part);
+      Running<Op> run(op.identity_coop());
+      for (uint32_t c = lc0 + lane; c < lc1; c += 128) {
+        Acc g[4];
+#pragma unroll
+        for (int j = 0; j < 4; j++) g[j] = c + 32 * j < lc1 ? partials[c + 32 * j] : op.identity_coop();
+        run.add(op, combine_tree<4>(op, g));
+      }
+      const Acc part = op.warp_combine(run.value());
       if (lane == leader) acc = op.combine(acc, part);
     }
     const bool a = todo && op.finish(v, acc, d.deg[v], t);
     if (act.active_out) push_activate(a, v, act, t);
   }
-  t.flush(ctr);
+  pull_flush<Op, PULL_THREADS>(t, act.active_out != nullptr, ctr);
+}
+
+// The reduction pull on a hot-source direction (Dir.sell_desc), one launch
+// for every list and a finish for the long ones.
+// Rows: the numbering sorts vertices of about equal out-degree by in-degree,
+// so 32 consecutive vertices (a slice) have lists of nearly equal length and
+// a lane walks its own list without waiting for longer ones.  The light
+// lists of a slice are stored column-major, so a warp reads the next four
+// entries of its 32 lists with one coalesced 16-byte load per lane, each
+// lane adds up its own list (no tree, no partial result: on GB300 an FP64
+// add costs a warp 16 cycles whatever the number of lanes that need it), and
+// 32 results are finished at once.  The places past a list's end name vertex
+// V: a dense op in double (has_dense; its state holds a neutral value there)
+// reads them like any other, which takes the length tests from around its
+// adds (double PageRank, 117 M edges: 9.9 -> 9.4 ms); the others stop at the
+// list's length (in float the extra requests cost more: R-MAT 26 70 against
+// 66 ms).
+// Long lists: a warp per aligned chunk, lane-strided entries, 8 in flight.
+// Slices whose 32 vertices have no list are left out where op.zero_kept()
+// says that their values are in place.
+// ALL: every gather through L1; else op.load's choice by source number.
+// Four blocks of 256 threads per SM: what bounds the kernel is the L1s'
+// rate of requests to L2 (at R-MAT 24 74% busy, one request per missing
+// gather), and more resident warps lose L1 hits (R-MAT 26: 83 ms for 20
+// iterations with six blocks of fewer registers, 67 with four).  The hottest
+// 32 K sources' values in shared memory served the gathers that L1 serves
+// here: no gain.
+// PageRank, 20 iterations, against a lane-serial light kernel with warps
+// over chunks beside it and a finish: float R-MAT 20 1.56 -> 1.03 ms, R-MAT
+// 26 100 -> 66 ms; double, 7.3 M vertices and 117 M edges, 27.4 -> 8.7 ms.
+template <class Op, class = void>
+struct has_dense : std::false_type {};
+template <class Op>
+struct has_dense<Op, std::void_t<decltype(Op::kDense)>> : std::true_type {};
+constexpr int ROWS_THREADS = 256;
+constexpr int ROWS_BLOCKS = 4;  // per SM
+constexpr int ROWS_Q = 2;       // columns of four entries in flight per lane
+template <class Op, bool ALL>
+__global__ void __launch_bounds__(ROWS_THREADS, ROWS_BLOCKS)
+    pull_rows(Dir d, uint32_t V, Op op, ActOut act, Counters *ctr, typename Op::Acc *__restrict__ partials) {
+  using Acc = typename Op::Acc;
+  constexpr bool WT = has_gather_w<Op>::value;
+  constexpr bool DENSE = has_dense<Op>::value && sizeof(Acc) == 8;
+  constexpr int CH = 8;
+  Tally t;
+  const uint32_t nwarps = gridDim.x * (ROWS_THREADS / 32);
+  // consecutive slices and chunks on different SMs
+  const uint32_t warp = (threadIdx.x >> 5) * gridDim.x + blockIdx.x;
+  const unsigned lane = lane_id();
+  for (uint32_t c = warp; c < d.nbigchunks; c += nwarps) {
+    uint32_t v;
+    unsigned long long lo, b, e;
+    big_range(d, c, d.chunk, &v, &lo, &b, &e);
+    Running<Op> run(op.identity_coop());
+    if (op.want(v)) {
+      const uint32_t n = (uint32_t)(e - b);
+      for (uint32_t k0 = lane; k0 - lane < n; k0 += 32 * CH) {
+        uint32_t u[CH];
+        float wt[WT ? CH : 1];
+#pragma unroll
+        for (int j = 0; j < CH; j++) {
+          const uint32_t k = k0 + 32 * j;
+          u[j] = k < n ? nbr_once(d, b + k, GG_SITE) : 0u;
+          if constexpr (WT) wt[j] = k < n ? ld_once(d.w + b + k) : 0.0f;
+        }
+        Acc g[CH];
+#pragma unroll
+        for (int j = 0; j < CH; j++) {
+          const uint32_t k = k0 + 32 * j;
+          g[j] = k < n ? op.template value<ALL>(u[j], WT ? wt[WT ? j : 0] : 0.0f) : op.identity_coop();
+        }
+        run.add(op, combine_tree<CH>(op, g));
+      }
+    }
+    const Acc part = op.warp_combine(run.value());
+    if (lane == 0) partials[c] = part;
+  }
+  const uint32_t nsl = op.zero_kept() ? d.nfull : d.nslices;
+  uint4 ds = warp < nsl ? d.sell_desc[warp] : make_uint4(0, 0, 0, 0);
+  for (uint32_t i = warp; i < nsl; i += nwarps) {
+    const uint4 dn = i + nwarps < nsl ? d.sell_desc[i + nwarps] : make_uint4(0, 0, 0, 0);
+    const uint32_t v = ds.x * 32 + lane;
+    const uint32_t *col = reinterpret_cast<const uint32_t *>(d.sell_col + (size_t)ds.y * 32 + lane);
+    const uint32_t *wcol = WT ? reinterpret_cast<const uint32_t *>(d.sell_w + (size_t)ds.y * 32 + lane) : nullptr;
+    uint4 c[ROWS_Q], w[WT ? ROWS_Q : 1];
+    w[0] = make_uint4(0, 0, 0, 0);
+    // the first columns do not wait for the degrees
+#pragma unroll
+    for (int q = 0; q < ROWS_Q; q++) {
+      c[q] = make_uint4(0, 0, 0, 0);
+      if (ds.z > q) c[q] = ld_once_v4(col + 128 * q);
+      if constexpr (WT) {
+        w[q] = make_uint4(0, 0, 0, 0);
+        if (ds.z > q) w[q] = ld_once_v4(wcol + 128 * q);
+      }
+    }
+    const uint32_t deg = v < V ? d.deg[v] : 0u;
+    const bool todo = v < V && deg <= d.light && op.want(v);
+    const uint32_t n = todo ? deg : 0u;
+    Running<Op> run(op.identity(v < V ? v : 0u));
+    if constexpr (DENSE) {
+      uint32_t t4 = 0;
+      for (; t4 + ROWS_Q <= ds.z; t4 += ROWS_Q) {
+        col += 128 * ROWS_Q;
+        Acc g[4 * ROWS_Q];
+#pragma unroll
+        for (int q = 0; q < ROWS_Q; q++) {
+          const uint32_t u[4] = {c[q].x, c[q].y, c[q].z, c[q].w};
+#pragma unroll
+          for (int j = 0; j < 4; j++) g[4 * q + j] = op.template value<ALL>(u[j], 0.0f);
+        }
+        // the next columns beside this step's gathers
+#pragma unroll
+        for (int q = 0; q < ROWS_Q; q++)
+          if (t4 + ROWS_Q + q < ds.z) c[q] = ld_once_v4(col + 128 * q);
+        run.add(op, combine_tree<4 * ROWS_Q>(op, g));
+      }
+#pragma unroll
+      for (int q = 0; q < ROWS_Q - 1; q++)
+        if (t4 + q < ds.z) {
+          const uint32_t u[4] = {c[q].x, c[q].y, c[q].z, c[q].w};
+          Acc g[4];
+#pragma unroll
+          for (int j = 0; j < 4; j++) g[j] = op.template value<ALL>(u[j], 0.0f);
+          run.add(op, combine_tree<4>(op, g));
+        }
+    } else {
+      for (uint32_t k = 0; k < n; k += 4 * ROWS_Q) {
+        col += 128 * ROWS_Q;
+        wcol += 128 * ROWS_Q;
+        Acc g[4 * ROWS_Q];
+#pragma unroll
+        for (int q = 0; q < ROWS_Q; q++) {
+          const uint32_t u[4] = {c[q].x, c[q].y, c[q].z, c[q].w};
+          const uint4 wq = w[WT ? q : 0];
+          const uint32_t wb[4] = {wq.x, wq.y, wq.z, wq.w};
+#pragma unroll
+          for (int j = 0; j < 4; j++)
+            g[4 * q + j] = k + 4 * q + j < n ? op.template value<ALL>(vertex_ok(d, u[j], GG_SITE),
+                                                                      __uint_as_float(wb[j]))
+                                             : op.identity_coop();
+        }
+        // the next columns beside this step's gathers
+#pragma unroll
+        for (int q = 0; q < ROWS_Q; q++)
+          if (k + 4 * ROWS_Q + 4 * q < n) {
+            c[q] = ld_once_v4(col + 128 * q);
+            if constexpr (WT) w[q] = ld_once_v4(wcol + 128 * q);
+          }
+        run.add(op, combine_tree<4 * ROWS_Q>(op, g));
+      }
+    }
+    const bool a = todo && op.finish(v, run.value(), deg, t);
+    if (act.active_out) pull_activate(a, v, ds.x, act, t);
+    ds = dn;
+  }
+  pull_flush<Op, ROWS_THREADS>(t, act.active_out != nullptr, ctr);
 }
 
 // ---------------------------------------------------------------- BFS pull
@@ -929,10 +1158,33 @@ struct Launch {
     return grid_for((size_t)d.nchunks * 32, PULL_THREADS, g->num_sms, 8);
   }
   // Kernels one reduction pull launches.
-  static int pull_launches(const Dir &d) { return d.nbig ? 3 : 1; }
+  static int pull_launches(const Dir &d) { return d.sell_desc ? (d.nbig ? 2 : 1) : d.nbig ? 3 : 1; }
+  // The pull of a hot-source direction (pull_rows): no second stream, the
+  // long lists' chunks lead in the same launch.
+  template <class Op>
+  int pull_hot(const Dir &d, const Op &op, const ActOut &act, Counters *ctr) {
+    cudaStream_t s = g->stream;
+    typename Op::Acc *part = nullptr;
+    if (d.nbig) GG_TRY(ws(g, WS_PARTIAL, d.nbigchunks, &part));
+    const size_t warps = (size_t)(op.zero_kept() ? d.nfull : d.nslices) + d.nbigchunks;
+    const unsigned grid = grid_for(warps * 32, ROWS_THREADS, g->num_sms, ROWS_BLOCKS);
+    if (op.gathers_all(g->V))
+      pull_rows<Op, true><<<grid, ROWS_THREADS, 0, s>>>(d, g->V, op, act, ctr, part);
+    else
+      pull_rows<Op, false><<<grid, ROWS_THREADS, 0, s>>>(d, g->V, op, act, ctr, part);
+    launches += 1;
+    if (d.nbig) {
+      pull_big_finish<Op, 8, true><<<grid_for(d.nbig, PULL_THREADS, g->num_sms, 8), PULL_THREADS, 0, s>>>(d, op, part, act,
+                                                                                                   ctr);
+      launches += 1;
+    }
+    GG_CUDA(cudaGetLastError());
+    return GG_OK;
+  }
   // All bins of one dense call, in order: light, medium, heavy chunks, heavy finish.
   template <class Op>
   int pull(const Dir &d, const Op &op, const ActOut &act, Counters *ctr) {
+    if (d.sell_desc) return pull_hot(d, op, act, ctr);
     cudaStream_t s = g->stream;
     // light lists on the side stream, beside the chunk kernel (disjoint
     // vertices); the finish, which sets bitmap bits atomically in words the
@@ -975,7 +1227,7 @@ struct Launch {
       }
       if (fork) GG_CUDA(cudaStreamWaitEvent(s, g->join, 0));
       if (act.active_out)
-        pull_big_finish<Op><<<grid_for(d.nbig, PULL_THREADS, g->num_sms, 8), PULL_THREADS, 0, s>>>(d, op, part, act,
+        pull_big_finish<Op, 32, false><<<grid_for(d.nbig, PULL_THREADS, g->num_sms, 8), PULL_THREADS, 0, s>>>(d, op, part, act,
                                                                                                     ctr);
       else
         pull_big_finish_warps<Op><<<grid_for((size_t)d.nbig * 32, PULL_THREADS, g->num_sms, 8), PULL_THREADS, 0, s>>>(

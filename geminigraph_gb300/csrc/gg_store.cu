@@ -220,20 +220,50 @@ __global__ void make_keys(const uint32_t *__restrict__ rec, size_t E, int words,
 
 // off[v] = first position whose major id is >= v, for v in [0, V], and nbr =
 // the minor ids, from n sorted keys.  The major id is a key's upper part
-// (low_major: its low `bits` bits).
+// (low_major: its low `bits` bits).  The vertices between two keys' majors
+// (and after the last) share one offset: up to GAP_INLINE of them are written
+// by the key's own thread, longer runs go to the gap list in pieces for
+// fill_gaps (a hot-source numbering ends with all vertices without a list: 30
+// M of them took one thread 150 ms at R-MAT 26).  A full list falls back to
+// the thread.
+constexpr uint32_t GAP_INLINE = 64, GAP_PIECE = 1u << 16, GAP_CAP = 1u << 16;
+struct Gap {
+  uint64_t value, from, to;  // off[from .. to) = value
+};
+__device__ __forceinline__ void write_gap(uint64_t *off, uint64_t from, uint64_t to, uint64_t value, Gap *gaps,
+                                          unsigned *ngaps) {
+  if (to - from > GAP_INLINE) {
+    const uint32_t pieces = (uint32_t)((to - from + GAP_PIECE - 1) / GAP_PIECE);
+    const uint32_t at = atomicAdd(ngaps, pieces);
+    if (at < GAP_CAP && GAP_CAP - at >= pieces) {
+      for (uint32_t i = 0; i < pieces; i++, from += GAP_PIECE)
+        gaps[at + i] = Gap{value, from, from + GAP_PIECE < to ? from + GAP_PIECE : to};
+      return;
+    }
+    for (uint32_t i = at; i < GAP_CAP && i - at < pieces; i++) gaps[i] = Gap{0, 0, 0};
+  }
+  for (; from < to; from++) off[from] = value;
+}
 __global__ void offsets_from_keys(const uint64_t *__restrict__ keys, size_t n, int bits, bool low_major, uint32_t V,
-                                  uint64_t *__restrict__ off, uint32_t *__restrict__ nbr) {
+                                  uint64_t *__restrict__ off, uint32_t *__restrict__ nbr, Gap *gaps,
+                                  unsigned *ngaps) {
   const uint64_t mask = (1ull << bits) - 1;
   for (size_t i = (size_t)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += (size_t)gridDim.x * blockDim.x) {
     const uint64_t k = keys[i];
     const uint64_t low = k & mask, high = k >> bits;
     const uint64_t maj = low_major ? low : high;
     nbr[i] = (uint32_t)(low_major ? high : low);
-    long long prev = -1ll;
-    if (i) prev = (long long)(low_major ? keys[i - 1] & mask : keys[i - 1] >> bits);
-    for (long long v = prev + 1; v <= (long long)maj; v++) off[v] = i;
-    if (i == n - 1)
-      for (uint64_t v = maj + 1; v <= V; v++) off[v] = n;
+    uint64_t next = 0;  // first vertex without an offset yet
+    if (i) next = (low_major ? keys[i - 1] & mask : keys[i - 1] >> bits) + 1;
+    if (next <= maj) write_gap(off, next, maj + 1, i, gaps, ngaps);
+    if (i == n - 1) write_gap(off, maj + 1, (uint64_t)V + 1, n, gaps, ngaps);
+  }
+}
+__global__ void fill_gaps(uint64_t *__restrict__ off, const Gap *__restrict__ gaps, const unsigned *ngaps) {
+  const uint32_t n = *ngaps < GAP_CAP ? *ngaps : GAP_CAP;
+  for (uint32_t g = blockIdx.x; g < n; g += gridDim.x) {
+    const Gap p = gaps[g];
+    for (uint64_t v = p.from + threadIdx.x; v < p.to; v += blockDim.x) off[v] = p.value;
   }
 }
 
@@ -343,6 +373,10 @@ int bits_for(uint32_t V) {
   return b;
 }
 
+static void free_sell(gg_graph *g, Dir *d);
+static int sell_or_plain(gg_graph *g, Dir *d);
+static void hot_bins(const gg_graph *g, Dir *d);
+
 // Degree bins of one direction (see Dir): the long lists (deg > light) with
 // their aligned chunks, split into medium and heavy ones for the BFS pulls.
 // Two allocations hold all of them (bins_mem once the number of long lists
@@ -437,17 +471,16 @@ int rebuild_bins(gg_graph *g, uint32_t light, uint32_t chunk, uint32_t vec) {
     g->in.chunk = chunk;
     GG_TRY(build_bins(g, &g->in));
   }
-  if (g->pr_ready) {
-    free_bins(g, &g->pr);
-    g->pr.light = light;
-    g->pr.chunk = chunk;
-    GG_TRY(build_bins(g, &g->pr));
-  }
-  if (g->pr_out_ready) {
-    free_bins(g, &g->pr_out);
-    g->pr_out.light = light;
-    g->pr_out.chunk = chunk;
-    GG_TRY(build_bins(g, &g->pr_out));
+  g->bins_set = 1;
+  Dir *hot[2] = {g->pr_ready ? &g->pr : nullptr, g->pr_out_ready ? &g->pr_out : nullptr};
+  for (Dir *d : hot) {
+    if (!d) continue;
+    const bool rows = d->sell_desc != nullptr;
+    free_sell(g, d);
+    free_bins(g, d);
+    hot_bins(g, d);
+    GG_TRY(build_bins(g, d));
+    if (rows) GG_TRY(sell_or_plain(g, d));
   }
   return GG_OK;
 }
@@ -518,8 +551,15 @@ static int emit_dir(gg_graph *g, const uint64_t *keys, size_t n, int bits, bool 
   if (n == 0) {
     GG_CUDA(cudaMemsetAsync(d->off, 0, sizeof(uint64_t) * ((size_t)V + 1), g->stream));
   } else {
+    DevScratch tmp;
+    char *blob = nullptr;
+    GG_TRY(tmp.get(&blob, 16 + sizeof(Gap) * GAP_CAP));
+    unsigned *ngaps = (unsigned *)blob;
+    Gap *gaps = (Gap *)(blob + 16);
+    GG_CUDA(cudaMemsetAsync(ngaps, 0, sizeof(unsigned), g->stream));
     offsets_from_keys<<<grid_for(n, 256, g->num_sms, 16), 256, 0, g->stream>>>(keys, n, bits, low_major, V, d->off,
-                                                                               d->nbr);
+                                                                               d->nbr, gaps, ngaps);
+    fill_gaps<<<(unsigned)g->num_sms * 4, 256, 0, g->stream>>>(d->off, gaps, ngaps);
     GG_CUDA(cudaGetLastError());
   }
   return finish_dir(g, d);
@@ -556,11 +596,27 @@ static void free_dir(Dir *d, bool adj_host) {
 // in-list by the new numbers puts a hub's hottest in-neighbours side by side
 // in one warp's loads.  The renumbered incoming adjacency is built once by
 // the same radix sort as the load; ranks map back to vertex order on output.
-__global__ void degree_rank_keys(const uint32_t *__restrict__ deg, uint32_t V, int bits, uint32_t dmax,
-                                 uint64_t *__restrict__ keys) {
+// Sort key of a vertex: its out-degree to an eighth of its power of two
+// (exact below 16; descending), then its in-degree (exact below 2048;
+// descending), then its id.  How often a source is gathered decides where it
+// lies to within 12%, and runs of vertices that are alike in that lie by list
+// length, which is what pull_rows needs of 32 consecutive rows.
+constexpr int RANK_BITS = 20;
+__device__ __forceinline__ uint32_t out_class(uint32_t d) {
+  if (d < 16) return d;
+  const uint32_t e = 31 - __clz(d);
+  return 16 + (e - 4) * 8 + ((d >> (e - 3)) & 7u);  // at most 239
+}
+__device__ __forceinline__ uint32_t in_class(uint32_t d) {
+  if (d < 2048) return d;
+  const uint32_t e = 31 - __clz(d);
+  return 2048 + (e - 11) * 64 + ((d >> (e - 6)) & 63u);  // at most 3391
+}
+__global__ void degree_rank_keys(const uint32_t *__restrict__ out_deg, const uint32_t *__restrict__ in_deg, uint32_t V,
+                                 int bits, uint64_t *__restrict__ keys) {
   for (size_t v = (size_t)blockIdx.x * blockDim.x + threadIdx.x; v < V; v += (size_t)gridDim.x * blockDim.x) {
-    const uint32_t dv = deg[v] < dmax ? deg[v] : dmax;
-    keys[v] = ((uint64_t)(dmax - dv) << bits) | v;
+    const uint32_t k = ((255u - out_class(out_deg[v])) << 12) | (4095u - in_class(in_deg[v]));
+    keys[v] = ((uint64_t)k << bits) | v;
   }
 }
 
@@ -595,21 +651,11 @@ __global__ void __launch_bounds__(EX_THREADS)
   const size_t ntiles = (n + EX_TILE - 1) / EX_TILE;
   for (size_t tile = blockIdx.x; tile < ntiles; tile += gridDim.x) {
     const uint64_t p0 = tile * EX_TILE, p1 = p0 + EX_TILE < n ? p0 + EX_TILE : n;
-    if (threadIdx.x < 2) {
-      // the list holding entry x: the last r with first[r] <= x
-      const uint64_t x = threadIdx.x ? p1 - 1 : p0;
-      uint32_t lo = 0, hi = nlist - 1;
-      while (lo < hi) {
-        const uint32_t mid = lo + (hi - lo + 1) / 2;
-        if (first[mid] <= x)
-          lo = mid;
-        else
-          hi = mid - 1;
-      }
-      if (threadIdx.x)
-        s_hi = lo;
-      else
-        s_lo = lo;
+    if (threadIdx.x < 64) {
+      // the lists holding the tile's first and last entry: the last r with first[r] <= x
+      const uint64_t x = threadIdx.x < 32 ? p0 : p1 - 1;
+      const uint32_t r = warp_upper_bound(first, 0u, nlist, x) - 1;
+      if (lane_id() == 0) (threadIdx.x < 32 ? s_lo : s_hi) = r;
     }
     __syncthreads();
     const uint32_t lo = s_lo, cnt = s_hi - s_lo + 1;
@@ -620,6 +666,7 @@ __global__ void __launch_bounds__(EX_THREADS)
         s_off[i] = d.off[list_of ? list_of[lo + i] : lo + i];
       }
     __syncthreads();
+#pragma unroll 4
     for (uint64_t p = p0 + threadIdx.x; p < p1; p += EX_THREADS) {
       uint32_t a = 0, b = cnt - 1;
       while (a < b) {
@@ -639,9 +686,138 @@ __global__ void __launch_bounds__(EX_THREADS)
   }
 }
 
+// Steps of every slice (the longest light list over four), and whether any
+// of its vertices has a list.
+__global__ void sell_widths(const uint32_t *__restrict__ deg, uint32_t V, uint32_t light, uint32_t nslices,
+                            uint32_t *__restrict__ steps, uint32_t *__restrict__ full) {
+  const uint32_t nwarps = gridDim.x * (blockDim.x / 32);
+  const unsigned lane = lane_id();
+  for (uint32_t s = (blockIdx.x * blockDim.x + threadIdx.x) / 32; s < nslices; s += nwarps) {
+    const size_t v = (size_t)s * 32 + lane;
+    const uint32_t d = v < V ? deg[v] : 0u;
+    const uint32_t m = __reduce_max_sync(GG_FULL, d <= light ? d : 0u);
+    const bool any = __any_sync(GG_FULL, d > 0);
+    if (lane == 0) {
+      steps[s] = (m + 3) / 4;
+      full[s] = any;
+    }
+  }
+}
+
+// Descriptors (slices with lists first, both in slice order) and the
+// column-major entries.  first, place: the scans of steps and full.
+__global__ void sell_fill(Dir d, uint32_t V, uint32_t nslices, uint32_t nfull, const uint32_t *__restrict__ first,
+                          const uint32_t *__restrict__ place, uint4 *__restrict__ desc, uint4 *__restrict__ col,
+                          float4 *__restrict__ wcol) {
+  const uint32_t nwarps = gridDim.x * (blockDim.x / 32);
+  const unsigned lane = lane_id();
+  for (uint32_t s = (blockIdx.x * blockDim.x + threadIdx.x) / 32; s < nslices; s += nwarps) {
+    const uint32_t t0 = first[s], steps = first[s + 1] - t0, p = place[s];
+    if (lane == 0) desc[place[s + 1] > p ? p : nfull + (s - p)] = make_uint4(s, t0, steps, 0);
+    const size_t v = (size_t)s * 32 + lane;
+    uint64_t b = 0;
+    uint32_t n = 0;
+    if (v < V) {
+      b = d.off[v];
+      n = d.deg[v] <= d.light ? d.deg[v] : 0u;
+    }
+    for (uint32_t t = 0; t < steps; t++) {
+      uint32_t u[4];
+      float w[4];
+#pragma unroll
+      for (int j = 0; j < 4; j++) {
+        const bool in = 4 * t + j < n;
+        u[j] = in ? nbr_at(d, b + 4 * t + j, GG_SITE) : V;
+        w[j] = in && wcol ? d.w[b + 4 * t + j] : 0.0f;
+      }
+      const size_t at = (size_t)(t0 + t) * 32 + lane;
+      col[at] = make_uint4(u[0], u[1], u[2], u[3]);
+      if (wcol) wcol[at] = make_float4(w[0], w[1], w[2], w[3]);
+    }
+  }
+}
+
+static void free_sell(gg_graph *g, Dir *d) {
+  if (d->sell_desc) g->graph_bytes -= sizeof(uint4) * d->nslices;
+  if (d->sell_col) g->graph_bytes -= sizeof(uint4) * 32 * d->sell_steps * (d->sell_w ? 2 : 1);
+  if (d->sell_desc) cudaFree(d->sell_desc);
+  if (d->sell_col) cudaFree(d->sell_col);
+  d->sell_desc = d->sell_col = nullptr;
+  d->sell_w = nullptr;
+  d->nslices = d->nfull = 0;
+  d->sell_steps = 0;
+}
+
+// The rows of a hot-source direction (see pull_rows) from its lists and bins.
+static int build_sell(gg_graph *g, Dir *d) {
+  cudaStream_t s = g->stream;
+  const uint32_t V = g->V, ns = (uint32_t)(((size_t)V + 31) / 32);
+  DevScratch tmp;
+  uint32_t *steps = nullptr;
+  GG_TRY(tmp.get(&steps, 4 * ((size_t)ns + 1) + scan_scratch_elems(ns)));
+  uint32_t *full = steps + ns + 1, *first = full + ns + 1, *place = first + ns + 1, *scratch = place + ns + 1;
+  const unsigned grid = grid_for((size_t)ns * 32, 256, g->num_sms, 8);
+  sell_widths<<<grid, 256, 0, s>>>(d->deg, V, d->light, ns, steps, full);
+  GG_CUDA(cudaGetLastError());
+  GG_CUDA((exclusive_scan<uint32_t, ArrayIn<uint32_t>>(ArrayIn<uint32_t>{steps}, ns, first, scratch, s, nullptr)));
+  GG_CUDA((exclusive_scan<uint32_t, ArrayIn<uint32_t>>(ArrayIn<uint32_t>{full}, ns, place, scratch, s, nullptr)));
+  uint32_t tot[2] = {0, 0};
+  GG_CUDA(cudaMemcpyAsync(&tot[0], first + ns, sizeof(uint32_t), cudaMemcpyDeviceToHost, s));
+  GG_CUDA(cudaMemcpyAsync(&tot[1], place + ns, sizeof(uint32_t), cudaMemcpyDeviceToHost, s));
+  GG_CUDA(cudaStreamSynchronize(s));
+  const size_t entries = 32 * (size_t)tot[0];
+  uint4 *col = nullptr;
+  GG_CUDA(cudaMalloc(&col, sizeof(uint4) * (entries ? entries : 1) * (d->w ? 2 : 1)));
+  d->sell_col = col;
+  d->sell_w = d->w ? reinterpret_cast<float4 *>(col + entries) : nullptr;
+  d->sell_steps = tot[0];
+  d->nslices = ns;
+  d->nfull = tot[1];
+  g->graph_bytes += sizeof(uint4) * entries * (d->w ? 2 : 1);
+  uint4 *desc = nullptr;
+  GG_CUDA(cudaMalloc(&desc, sizeof(uint4) * ns));
+  g->graph_bytes += sizeof(uint4) * ns;
+  d->sell_desc = desc;
+  sell_fill<<<grid, 256, 0, s>>>(*d, V, ns, d->nfull, first, place, desc, col, d->sell_w);
+  GG_CUDA(cudaGetLastError());
+  GG_CUDA(cudaStreamSynchronize(s));
+  return GG_OK;
+}
+
+// A direction without room for its rows is pulled through its lists, as a
+// plain one.
+static int sell_or_plain(gg_graph *g, Dir *d) {
+  const int r = build_sell(g, d);
+  if (r == GG_OK) return r;
+  free_sell(g, d);
+  if (r != GG_ERR_NOMEM) return r;
+  cudaGetLastError();
+  return GG_OK;
+}
+
+// Light bound and chunk size of a hot-source direction unless
+// gg_graph_set_bins chose them.  A light list is one lane's serial walk, about
+// 0.1 us per entry, so the bound grows with the graph (entries / 2^16, a power
+// of two in 32..1024): the longest walk stays below the time the whole pull
+// takes.  Measured, PageRank of 20 iterations with bounds 32 / 128 / 512 /
+// 1024: R-MAT 18 506 / 454 / 546 / 889 us, R-MAT 20 1297 / 1029 / 1041 / 1396
+// us, R-MAT 26 98 / 73 / 69 / 67 ms.
+static void hot_bins(const gg_graph *g, Dir *d) {
+  if (g->bins_set) {
+    d->light = g->out.light;
+    d->chunk = g->out.chunk;
+    return;
+  }
+  uint32_t l = 32;
+  while (l < 1024 && (g->nadj >> 16) >= 2 * (uint64_t)l) l *= 2;
+  d->light = l;
+  d->chunk = 512;
+}
+
 // Frees a renumbered direction and its device bytes.
 static void free_hot_dir(gg_graph *g, Dir *d) {
   const size_t V = g->V;
+  free_sell(g, d);
   free_bins(g, d);
   const size_t npad = (g->nadj + 64) / 64 * 64;
   g->graph_bytes -= sizeof(uint64_t) * (V + 1) + sizeof(uint32_t) * (npad + V + 1) +
@@ -688,9 +864,8 @@ static int transpose_dir(gg_graph *g, const Dir &src, const uint64_t *first, con
     GG_CUDA(cudaGetLastError());
   }
   *dst = Dir();
-  dst->light = src.light;
-  dst->chunk = src.chunk;
   dst->vec = src.vec;
+  hot_bins(g, dst);
   return sort_dir(g, scratch, k0, k1, v0, v0, v1, n, bits, true, dst, false, &ks, &vs);
 }
 
@@ -709,14 +884,18 @@ int hot_out_build(gg_graph *g) {
   return GG_OK;
 }
 
-// The vertices ranked by descending out-degree (equal degrees by id): the
+// The renumbered outgoing adjacency's rows, for pulls over it (BC's
+// backward sweep).
+int hot_out_rows(gg_graph *g) {
+  GG_TRY(hot_out_build(g));
+  return g->pr_out.sell_desc ? GG_OK : sell_or_plain(g, &g->pr_out);
+}
+
+// The vertices ranked by degree_rank_keys: the
 // three tables and the positions of the out-lists taken in that order.
 static int rank_vertices(gg_graph *g, uint64_t *first) {
   const uint32_t V = g->V;
   const int bits = bits_for(V);
-  int dbits = 1;
-  while (dbits < 32 && (1ull << dbits) <= g->nadj) dbits++;
-  const uint32_t dmax = dbits >= 32 ? 0xFFFFFFFFu : (uint32_t)((1ull << dbits) - 1);
   DevScratch tmp;
   uint64_t *k0 = nullptr, *k1 = nullptr, *ks = nullptr;
   uint32_t *v0 = nullptr, *v1 = nullptr, *vs = nullptr;
@@ -724,10 +903,10 @@ static int rank_vertices(gg_graph *g, uint64_t *first) {
   uint64_t *scan = nullptr;
   GG_TRY(tmp.sort_buffers(V, false, &k0, &k1, &v0, &v1, &scratch));
   GG_TRY(tmp.get(&scan, scan_scratch_elems(V)));
-  degree_rank_keys<<<grid_for(V, 256, g->num_sms, 16), 256, 0, g->stream>>>(g->out.deg, V, bits, dmax, k0);
+  degree_rank_keys<<<grid_for(V, 256, g->num_sms, 16), 256, 0, g->stream>>>(g->out.deg, g->in.deg, V, bits, k0);
   GG_CUDA(cudaGetLastError());
-  // the keys start in id order and the sort is stable: the degree bits suffice
-  GG_TRY(radix_sort(g, scratch, k0, k1, SortValues(), V, bits, bits + dbits, &ks, &vs));
+  // the keys start in id order and the sort is stable: the class bits suffice
+  GG_TRY(radix_sort(g, scratch, k0, k1, SortValues(), V, bits, bits + RANK_BITS, &ks, &vs));
   rank_tables<<<grid_for(V, 256, g->num_sms, 16), 256, 0, g->stream>>>(ks, V, bits, g->out.deg, g->pr_id_of_rank,
                                                                       g->pr_rank_of, g->pr_od);
   GG_CUDA(cudaGetLastError());
@@ -762,7 +941,7 @@ int pr_layout_build(gg_graph *g) {
     return status;
   }
   g->pr_ready = true;
-  return GG_OK;
+  return sell_or_plain(g, &g->pr);
 }
 
 void graph_destroy(gg_graph *g) {
