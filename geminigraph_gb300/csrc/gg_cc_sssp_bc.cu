@@ -23,17 +23,26 @@ struct CcPush {
 };
 
 // Dense signal + slot (cc.cpp:60-79): msg = min(dst, labels of all
-// in-neighbours); read from cur, written to nxt.
+// in-neighbours); read from cur, written to nxt.  (A label never exceeds its
+// vertex's id, so the message may start at the label instead of the id.)
+// Every label a gather can return is at least the least id with an out-edge
+// (floor): a vertex that has it is done, and a list that has shown it is too.
+// From the second call on most vertices of a graph with one large component
+// have it, the rest find it at their hottest in-neighbours, which lead the
+// lists of the hot-source layout.  R-MAT 24 (537 M entries): 4.4 ms walking
+// every list in each of three dense calls, 1.15 ms with this and cc_first.
 struct CcPull {
   using Acc = uint32_t;
   const uint32_t *cur;
   uint32_t *nxt;
-  const uint32_t *ids = nullptr;  // hot-source layout: vertex id of each rank (the message starts at dst's id)
+  uint32_t floor = 0;
   uint32_t hot = 0xffffffffu;     // sources below this number are gathered through L1
   __device__ __forceinline__ bool want(uint32_t) const { return true; }
   // no call changes a vertex without in-edges: both buffers hold its label
   __host__ __device__ __forceinline__ bool zero_kept() const { return true; }
-  __device__ __forceinline__ uint32_t identity(uint32_t v) const { return ids ? ids[v] : v; }
+  __device__ __forceinline__ uint32_t identity(uint32_t v) const { return cur[v]; }
+  __device__ __forceinline__ bool skip(uint32_t v) const { return cur[v] <= floor; }
+  __device__ __forceinline__ bool stop(uint32_t acc, float) const { return acc <= floor; }
   __device__ __forceinline__ uint32_t identity_coop() const { return 0xffffffffu; }
   __device__ __forceinline__ uint32_t gather(const Dir &, unsigned long long, uint32_t u) const {
     return ld_gather(cur, u, hot);
@@ -114,6 +123,47 @@ struct SsspPull {
     return false;
   }
 };
+
+// CC's first call, every vertex active with its own id as label: the least
+// in-neighbour, the first entry of the (plain) in-list.  v in the numbering
+// of the labels, id_of its vertex (null: v itself).
+__global__ void __launch_bounds__(PULL_THREADS)
+    cc_first(Dir d, uint32_t V, const uint32_t *__restrict__ id_of, uint32_t *__restrict__ label, ActOut act,
+             Counters *ctr) {
+  Tally t;
+  const size_t groups = ((size_t)V + 31) / 32, nwarps = (size_t)gridDim.x * (PULL_THREADS / 32);
+  for (size_t g = (size_t)blockIdx.x * (PULL_THREADS / 32) + (threadIdx.x >> 5); g < groups; g += nwarps) {
+    const uint32_t v = (uint32_t)(g * 32 + lane_id());
+    bool a = false;
+    if (v < V) {
+      const uint32_t id = id_of ? id_of[v] : v;
+      const unsigned long long b = d.off[id];
+      if (d.off[id + 1] > b) {
+        const uint32_t u = nbr_at(d, b, GG_SITE);
+        a = u < id;
+        if (a) label[v] = u;
+      }
+    }
+    pull_activate(a, v, g, act, t);
+  }
+  t.flush(ctr);
+}
+
+// The least vertex with an out-edge (V if none), by one block over the
+// deg > 0 bitmap.
+__global__ void __launch_bounds__(1024) least_source(const uint32_t *__restrict__ nz, size_t words, uint32_t V,
+                                                     uint32_t *out) {
+  __shared__ uint32_t s_min;
+  if (threadIdx.x == 0) s_min = V;
+  __syncthreads();
+  for (size_t base = 0; base < words; base += blockDim.x) {
+    const size_t i = base + threadIdx.x;
+    const uint32_t w = i < words ? nz[i] : 0u;
+    if (w) atomicMin(&s_min, (uint32_t)(i * 32 + __ffs(w) - 1));
+    if (__syncthreads_or(w != 0)) break;
+  }
+  if (threadIdx.x == 0) *out = s_min;
+}
 
 // Runs the CC / SSSP frontier loop: both toolkits loop while the slots
 // activate something, with a message snapshot for push calls and two state
@@ -240,21 +290,41 @@ static int cc_run(gg_graph *g, uint32_t *label_host, gg_run_stats *st) {
   Launch L(g);
   Trace tr(st, g, "gg_cc");
   cudaStream_t s = g->stream;
+  Counters *ctr = g->ws.ctr;
   GG_TRY(timed_begin(g));
   // label[v] = v over active_in = all (cc.cpp:31-37)
   if (ranked)
     copy_twice<uint32_t><<<grid_for(V, 256, g->num_sms), 256, 0, s>>>(g->pr_id_of_rank, V, lab[0], lab[1]);
   else
     iota_u32<<<grid_for(V, 256, g->num_sms), 256, 0, s>>>(lab[0], V);
-  bitmap_fill<<<grid_for(words, 256, g->num_sms), 256, 0, s>>>(bm[0], words, V);
-  L.launches += 2;
+  L.launches += 1;
   GG_CUDA(cudaGetLastError());
   uint32_t *res = nullptr;
   CcPull pull{};
-  pull.ids = ranked ? g->pr_id_of_rank : nullptr;
   pull.hot = ranked ? g->l1_hot_bytes / 4 : 0xffffffffu;
-  GG_TRY((relax_loop<uint32_t, CcPush, CcPull>(g, dout, din, pull, lab[0], lab[1], q[0], q[1], bm[0], bm[1], V, 0,
-                                               0xffffffffu, false, g->nadj, tr, L, &res)));
+  uint32_t n_act = V;
+  unsigned long long ae = g->nadj;
+  // the first call: dense by the reference's switch (every vertex active)
+  tr.add(1, ae, 0);
+  GG_CUDA(cudaMemsetAsync(bm[0], 0, words * 4, s));
+  GG_TRY(counters_reset(g));
+  least_source<<<1, 1024, 0, s>>>(g->out.nz, words, V, &ctr->aux);
+  ActOut act;
+  act.active_out = bm[0];
+  act.out_deg = dout.deg;
+  GG_TRY(tr.kbegin());
+  cc_first<<<L.pull_grid(), PULL_THREADS, 0, s>>>(g->in, V, ranked ? g->pr_id_of_rank : nullptr, lab[0], act, ctr);
+  GG_TRY(tr.kend());
+  L.launches += 2;
+  GG_CUDA(cudaGetLastError());
+  Counters c;
+  GG_TRY(counters_read(g, &c));
+  tr.set_activated(c.activated);
+  pull.floor = c.aux;
+  n_act = c.activated;
+  ae = c.edges;
+  GG_TRY((relax_loop<uint32_t, CcPush, CcPull>(g, dout, din, pull, lab[0], lab[1], q[0], q[1], bm[0], bm[1], n_act, 0,
+                                               0xffffffffu, false, ae, tr, L, &res)));
   if (ranked) {
     unrank<uint32_t><<<grid_for(V, 256, g->num_sms), 256, 0, s>>>(res, g->pr_rank_of, V, out);
     L.launches += 1;

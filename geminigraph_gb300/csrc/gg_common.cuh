@@ -104,6 +104,7 @@ struct Counters {
   double delta;                 // PageRank delta accumulator
   unsigned int err;             // device-side error flag (bounds checks)
   unsigned int maxdeg;          // largest out_degree among newly activated vertices
+  unsigned int aux;             // a call's own result (CC: the least vertex with an out-edge)
 };
 
 enum WsSlot {

@@ -493,6 +493,14 @@ template <class Op, class = void>
 struct has_dense : std::false_type {};
 template <class Op>
 struct has_dense<Op, std::void_t<decltype(Op::kDense)>> : std::true_type {};
+// Ops that can tell when a list need not be walked (on): skip(v) before its
+// first entry, stop(acc, w) after some of them (acc the result so far, w the
+// weight of the last one).  Their identity(v) is the vertex's own value, so a
+// list left out finishes with it.
+template <class Op, class = void>
+struct has_stop : std::false_type {};
+template <class Op>
+struct has_stop<Op, std::void_t<decltype(&Op::stop)>> : std::true_type {};
 constexpr int ROWS_THREADS = 256;
 constexpr int ROWS_BLOCKS = 4;  // per SM
 constexpr int ROWS_Q = 2;       // columns of four entries in flight per lane
@@ -502,6 +510,7 @@ __global__ void __launch_bounds__(ROWS_THREADS, ROWS_BLOCKS)
   using Acc = typename Op::Acc;
   constexpr bool WT = has_gather_w<Op>::value;
   constexpr bool DENSE = has_dense<Op>::value && sizeof(Acc) == 8;
+  constexpr bool STOP = has_stop<Op>::value;
   constexpr int CH = 8;
   Tally t;
   const uint32_t nwarps = gridDim.x * (ROWS_THREADS / 32);
@@ -513,7 +522,9 @@ __global__ void __launch_bounds__(ROWS_THREADS, ROWS_BLOCKS)
     unsigned long long lo, b, e;
     big_range(d, c, d.chunk, &v, &lo, &b, &e);
     Running<Op> run(op.identity_coop());
-    if (op.want(v)) {
+    bool walk = op.want(v);
+    if constexpr (STOP) walk = walk && !op.skip(v);
+    if (walk) {
       const uint32_t n = (uint32_t)(e - b);
       for (uint32_t k0 = lane; k0 - lane < n; k0 += 32 * CH) {
         uint32_t u[CH];
@@ -531,6 +542,8 @@ __global__ void __launch_bounds__(ROWS_THREADS, ROWS_BLOCKS)
           g[j] = k < n ? op.template value<ALL>(u[j], WT ? wt[WT ? j : 0] : 0.0f) : op.identity_coop();
         }
         run.add(op, combine_tree<CH>(op, g));
+        if constexpr (STOP)
+          if (__any_sync(GG_FULL, op.stop(run.value(), 0.0f))) break;
       }
     }
     const Acc part = op.warp_combine(run.value());
@@ -557,7 +570,9 @@ __global__ void __launch_bounds__(ROWS_THREADS, ROWS_BLOCKS)
     }
     const uint32_t deg = v < V ? d.deg[v] : 0u;
     const bool todo = v < V && deg <= d.light && op.want(v);
-    const uint32_t n = todo ? deg : 0u;
+    uint32_t n = todo ? deg : 0u;
+    if constexpr (STOP)
+      if (n && op.skip(v)) n = 0;
     Running<Op> run(op.identity(v < V ? v : 0u));
     if constexpr (DENSE) {
       uint32_t t4 = 0;
@@ -609,6 +624,8 @@ __global__ void __launch_bounds__(ROWS_THREADS, ROWS_BLOCKS)
             if constexpr (WT) w[q] = ld_once_v4(wcol + 128 * q);
           }
         run.add(op, combine_tree<4 * ROWS_Q>(op, g));
+        if constexpr (STOP)
+          if (op.stop(run.value(), 0.0f)) break;
       }
     }
     const bool a = todo && op.finish(v, run.value(), deg, t);
