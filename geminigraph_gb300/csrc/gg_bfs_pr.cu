@@ -396,6 +396,7 @@ int gg_graph_set_dense_push(gg_graph *g, uint32_t divisor) {
     return GG_ERR_INVALID;
   }
   g->dense_push_div = divisor;
+  g->dense_push_set = 1;
   return GG_OK;
 }
 

@@ -1,5 +1,7 @@
 // CC (toolkits/cc.cpp), SSSP (toolkits/sssp.cpp) and BC (toolkits/bc.cpp,
 // compute) on the device engine.
+#include <math.h>
+
 #include <vector>
 
 #include "gg_engine.cuh"
@@ -41,6 +43,7 @@ struct CcPull {
   // no call changes a vertex without in-edges: both buffers hold its label
   __host__ __device__ __forceinline__ bool zero_kept() const { return true; }
   __device__ __forceinline__ uint32_t identity(uint32_t v) const { return cur[v]; }
+  __device__ __forceinline__ void begin() {}
   __device__ __forceinline__ bool skip(uint32_t v) const { return cur[v] <= floor; }
   __device__ __forceinline__ bool stop(uint32_t acc, float) const { return acc <= floor; }
   __device__ __forceinline__ uint32_t identity_coop() const { return 0xffffffffu; }
@@ -91,15 +94,31 @@ struct SsspPush {
 
 // sssp.cpp:60-80: the dense signal takes the min over ALL in-edges (its
 // active check is commented out, sssp.cpp:64-70); INF = 1e9.
+// On SSSP's layout a list is walked by ascending weight class and only as far
+// as an active source could still lower the vertex: an inactive source cannot
+// (see relax_loop), an active one's candidate is at least fl(lo + w) for the
+// active sources' least distance lo and the least weight w of what is left.
 struct SsspPull {
   using Acc = float;
   const float *cur;
   float *nxt;
+  float wmin = -INFINITY, width = INFINITY;  // of the layout (gg_graph)
+  const unsigned *lo_enc = nullptr;          // ~float_order(lo), written by active_min
+  float lo = -INFINITY;
+  __device__ __forceinline__ void begin() {
+    const uint32_t o = ~*lo_enc;
+    lo = __uint_as_float(o & 0x80000000u ? o & 0x7fffffffu : ~o);
+  }
+  __device__ __forceinline__ bool skip(uint32_t v) const { return __fadd_rn(lo, wmin) >= cur[v]; }
+  __device__ __forceinline__ bool stop(float acc, float w) const {
+    return __fadd_rn(lo, __fsub_rd(w, width)) >= acc;
+  }
   uint32_t hot = 0xffffffffu;  // sources below this number are gathered through L1
   __device__ __forceinline__ bool want(uint32_t) const { return true; }
   // no call changes a vertex without in-edges: both buffers hold its distance
   __host__ __device__ __forceinline__ bool zero_kept() const { return true; }
-  __device__ __forceinline__ float identity(uint32_t) const { return 1e9f; }
+  // the message may start at the distance: only a lower one is written
+  __device__ __forceinline__ float identity(uint32_t v) const { return cur[v]; }
   __device__ __forceinline__ float identity_coop() const { return 1e9f; }
   __device__ __forceinline__ float gather(const Dir &d, unsigned long long k, uint32_t u) const {
     return __fadd_rn(ld_gather(cur, u, hot), d.w[k]);
@@ -123,6 +142,35 @@ struct SsspPull {
     return false;
   }
 };
+
+// The least distance among the active vertices (queue q, or bitmap bm when q
+// is null), as ~float_order in *out (0 before).
+__global__ void active_min(const uint32_t *__restrict__ q, uint32_t n, const uint32_t *__restrict__ bm, size_t words,
+                           const float *__restrict__ dist, unsigned *out) {
+  uint32_t best = 0;
+  auto take = [&](uint32_t v) {
+    const uint32_t u = __float_as_uint(dist[v]);
+    const uint32_t o = ~(u & 0x80000000u ? ~u : u | 0x80000000u);
+    best = o > best ? o : best;
+  };
+  const size_t tid = (size_t)blockIdx.x * blockDim.x + threadIdx.x, stride = (size_t)gridDim.x * blockDim.x;
+  if (q) {
+    for (size_t i = tid; i < n; i += stride) take(q[i]);
+  } else {
+    // a warp per 32 words: each word's vertices by the lanes, coalesced
+    for (size_t g = tid / 32; g * 32 < words; g += stride / 32) {
+      const size_t i = g * 32 + lane_id();
+      const uint32_t w = i < words ? bm[i] : 0u;
+      for (unsigned any = __ballot_sync(GG_FULL, w != 0); any; any &= any - 1) {
+        const int j = __ffs(any) - 1;
+        const uint32_t wj = __shfl_sync(GG_FULL, w, j);
+        if ((wj >> lane_id()) & 1u) take((uint32_t)((g * 32 + j) * 32 + lane_id()));
+      }
+    }
+  }
+  best = __reduce_max_sync(GG_FULL, best);
+  if (lane_id() == 0 && best) atomicMax(out, best);
+}
 
 // CC's first call, every vertex active with its own id as label: the least
 // in-neighbour, the first entry of the (plain) in-list.  v in the numbering
@@ -184,6 +232,11 @@ static int relax_loop(gg_graph *g, const Dir &dout, const Dir &din, const PullOp
   GG_TRY(ws(g, WS_MSG, (size_t)V + 1, &msg));
   GG_TRY(ws(g, WS_STAMP, V, &stamp));
   GG_CUDA(cudaMemsetAsync(stamp, 0, sizeof(uint32_t) * V, s));
+  // A pull that ends its walks early is the faster form down to fewer active
+  // edges: SSSP R-MAT 24, divisors 4 / 8 / 16: 7.2 / 5.9 / 5.7 ms, R-MAT 22:
+  // 2.9 / 2.3 / 2.2 ms (walking every list: 4 was the best).
+  uint32_t push_div = g->dense_push_div;
+  if (has_gather_w<PullOp>::value && din.sell_desc && !g->dense_push_set) push_div = 16;
   int c_i = 0;
   while (n_act > 0) {
     bool sparse = ae < g->E / 20;
@@ -200,7 +253,7 @@ static int relax_loop(gg_graph *g, const Dir &dout, const Dir &din, const PullOp
     // minimum over the active sources' candidates is the dense call's
     // minimum over all in-edges -- the same values and the same activated
     // set (the snapshot keeps every signal before every slot).
-    const bool push = sparse || (g->dense_push_div && ae < g->nadj / g->dense_push_div);
+    const bool push = sparse || (push_div && ae < g->nadj / push_div);
     int nx = c_i ^ 1;
     if (push && ae > 0 && !qvalid) GG_TRY(L.queue_from_bitmap(bm[c_i], dout.nz, q[c_i], &nq));
     GG_CUDA(cudaMemsetAsync(bm[nx], 0, words * 4, s));
@@ -227,6 +280,15 @@ static int relax_loop(gg_graph *g, const Dir &dout, const Dir &din, const PullOp
       PullOp op = pull;
       op.cur = cur;
       op.nxt = nxt;
+      if constexpr (has_gather_w<PullOp>::value) {
+        if (din.sell_desc) {
+          const size_t work = qvalid ? nq : words;
+          active_min<<<grid_for(work, 256, g->num_sms, 8), 256, 0, s>>>(qvalid ? q[c_i] : nullptr, nq, bm[c_i], words,
+                                                                       cur, &ctr->aux);
+          L.launches += 1;
+          op.lo_enc = &ctr->aux;
+        }
+      }
       GG_TRY(L.pull(din, op, a, ctr));
       GG_TRY(tr.kend());
       T *t = cur;
@@ -374,13 +436,10 @@ static int sssp_run(gg_graph *g, uint32_t root, float *dist_host, gg_run_stats *
   // distance d[u] + w is the same sum, and a minimum does not depend on
   // order, so the distances are bit-identical; they map back to vertex order
   // at the end.
-  if (g->pr_layout) {
-    GG_TRY(pr_layout_build(g));
-    if (!g->symmetric) GG_TRY(hot_out_build(g));
-  }
-  const bool ranked = g->pr_layout && g->pr_ready && (g->symmetric || g->pr_out_ready);
-  const Dir &dout = ranked ? (g->symmetric ? g->pr : g->pr_out) : g->out;
-  const Dir &din = ranked ? g->pr : g->in;
+  if (g->pr_layout) GG_TRY(sssp_layout_build(g));
+  const bool ranked = g->pr_layout && g->ps_ready && (g->symmetric || g->pr_out_ready);
+  const Dir &dout = ranked ? (g->symmetric ? g->ps : g->pr_out) : g->out;
+  const Dir &din = ranked ? g->ps : g->in;
   uint32_t start = root;
   float *out = nullptr;
   if (ranked) {
@@ -403,6 +462,8 @@ static int sssp_run(gg_graph *g, uint32_t root, float *dist_host, gg_run_stats *
   float *res = nullptr;
   SsspPull pull{};
   pull.hot = ranked ? g->l1_hot_bytes / 4 : 0xffffffffu;
+  pull.wmin = g->ps_wmin;
+  pull.width = g->ps_width;
   GG_TRY((relax_loop<float, SsspPush, SsspPull>(g, dout, din, pull, dist[0], dist[1], q[0], q[1], bm[0], bm[1], 1,
                                                 1, c.maxdeg, true, c.edges, tr, L, &res)));
   if (ranked) {

@@ -142,6 +142,7 @@ void pools_destroy(gg_graph *g);
 int pr_layout_build(gg_graph *g);
 int hot_out_build(gg_graph *g);
 int hot_out_rows(gg_graph *g);
+int sssp_layout_build(gg_graph *g);
 void pr_layout_free(gg_graph *g);
 
 }  // namespace gg
@@ -190,11 +191,18 @@ struct gg_graph {
   uint32_t *pr_rank_of = nullptr;     // V: new number of vertex v
   uint32_t *pr_id_of_rank = nullptr;  // V: vertex with new number r
   uint32_t *pr_od = nullptr;          // V: out-degree in the new numbering
+  bool ranks_ready = false;           // the three tables above
   bool pr_ready = false;
   // the outgoing adjacency in the same numbering (directed graphs; built on
   // demand by SSSP, whose push steps walk out-lists)
   gg::Dir pr_out;
   bool pr_out_ready = false;
+  // SSSP's incoming adjacency in the same numbering, each list by ascending
+  // weight class (see sssp_layout_build): an entry's weight is at least any
+  // earlier entry's less ps_width; ps_wmin is the least weight
+  gg::Dir ps;
+  bool ps_ready = false;
+  float ps_width = 0.0f, ps_wmin = 0.0f;
   int pr_layout = 1;                  // 0: PageRank pulls the plain incoming adjacency
   // gg_graph_set_bins was called: the hot-source directions take its light
   // bound and chunk size instead of their own (hot_bins)
@@ -236,6 +244,7 @@ struct gg_graph {
   // frontier instead of pulling every in-list (0: always pull; 4 measured
   // best for SSSP on R-MAT 25, neutral for CC on R-MAT 26)
   uint32_t dense_push_div = 4;
+  int dense_push_set = 0;  // gg_graph_set_dense_push was called
   // PageRank's iterations captured as one CUDA graph, replayed while the key
   // (arguments, buffers, events) is unchanged
   cudaGraphExec_t pr_exec[2] = {nullptr, nullptr};  // float, double

@@ -494,9 +494,10 @@ struct has_dense : std::false_type {};
 template <class Op>
 struct has_dense<Op, std::void_t<decltype(Op::kDense)>> : std::true_type {};
 // Ops that can tell when a list need not be walked (on): skip(v) before its
-// first entry, stop(acc, w) after some of them (acc the result so far, w the
-// weight of the last one).  Their identity(v) is the vertex's own value, so a
-// list left out finishes with it.
+// first entry, stop(acc, w) on the way (acc the result so far, w the weight
+// of an entry at or before the next one).  Their identity(v) is the vertex's
+// own value, so a list left out finishes with it; begin() runs once per thread
+// before the first call of either.
 template <class Op, class = void>
 struct has_stop : std::false_type {};
 template <class Op>
@@ -512,6 +513,7 @@ __global__ void __launch_bounds__(ROWS_THREADS, ROWS_BLOCKS)
   constexpr bool DENSE = has_dense<Op>::value && sizeof(Acc) == 8;
   constexpr bool STOP = has_stop<Op>::value;
   constexpr int CH = 8;
+  if constexpr (STOP) op.begin();
   Tally t;
   const uint32_t nwarps = gridDim.x * (ROWS_THREADS / 32);
   // consecutive slices and chunks on different SMs
@@ -521,7 +523,7 @@ __global__ void __launch_bounds__(ROWS_THREADS, ROWS_BLOCKS)
     uint32_t v;
     unsigned long long lo, b, e;
     big_range(d, c, d.chunk, &v, &lo, &b, &e);
-    Running<Op> run(op.identity_coop());
+    Running<Op> run(STOP ? op.identity(v) : op.identity_coop());
     bool walk = op.want(v);
     if constexpr (STOP) walk = walk && !op.skip(v);
     if (walk) {
@@ -535,6 +537,13 @@ __global__ void __launch_bounds__(ROWS_THREADS, ROWS_BLOCKS)
           u[j] = k < n ? nbr_once(d, b + k, GG_SITE) : 0u;
           if constexpr (WT) wt[j] = k < n ? ld_once(d.w + b + k) : 0.0f;
         }
+        if constexpr (STOP) {
+          // lane 0 holds the batch's first entry: with any lane's result
+          const Acc best = op.warp_combine(run.value());
+          float first = 0.0f;
+          if constexpr (WT) first = __shfl_sync(GG_FULL, wt[0], 0);
+          if (op.stop(best, first)) break;
+        }
         Acc g[CH];
 #pragma unroll
         for (int j = 0; j < CH; j++) {
@@ -542,8 +551,6 @@ __global__ void __launch_bounds__(ROWS_THREADS, ROWS_BLOCKS)
           g[j] = k < n ? op.template value<ALL>(u[j], WT ? wt[WT ? j : 0] : 0.0f) : op.identity_coop();
         }
         run.add(op, combine_tree<CH>(op, g));
-        if constexpr (STOP)
-          if (__any_sync(GG_FULL, op.stop(run.value(), 0.0f))) break;
       }
     }
     const Acc part = op.warp_combine(run.value());
@@ -602,6 +609,13 @@ __global__ void __launch_bounds__(ROWS_THREADS, ROWS_BLOCKS)
         }
     } else {
       for (uint32_t k = 0; k < n; k += 4 * ROWS_Q) {
+        if constexpr (STOP) {
+          if (op.stop(run.value(), __uint_as_float(w[0].x))) break;
+          // where the last entry of this step ends the walk, its successors
+          // are not read ahead
+          if (WT && k + 4 * ROWS_Q < n && op.stop(run.value(), __uint_as_float(w[WT ? ROWS_Q - 1 : 0].w)))
+            n = k + 4 * ROWS_Q;
+        }
         col += 128 * ROWS_Q;
         wcol += 128 * ROWS_Q;
         Acc g[4 * ROWS_Q];
@@ -624,8 +638,6 @@ __global__ void __launch_bounds__(ROWS_THREADS, ROWS_BLOCKS)
             if constexpr (WT) w[q] = ld_once_v4(wcol + 128 * q);
           }
         run.add(op, combine_tree<4 * ROWS_Q>(op, g));
-        if constexpr (STOP)
-          if (op.stop(run.value(), 0.0f)) break;
       }
     }
     const bool a = todo && op.finish(v, run.value(), deg, t);

@@ -13,6 +13,7 @@
 // their degree therefore counts both endpoints (core/graph.hpp:393-399).
 #include <errno.h>
 #include <fcntl.h>
+#include <math.h>
 #include <stdarg.h>
 #include <string.h>
 #include <sys/stat.h>
@@ -220,7 +221,8 @@ __global__ void make_keys(const uint32_t *__restrict__ rec, size_t E, int words,
 
 // off[v] = first position whose major id is >= v, for v in [0, V], and nbr =
 // the minor ids, from n sorted keys.  The major id is a key's upper part
-// (low_major: its low `bits` bits).  The vertices between two keys' majors
+// (low_major: its low `bits` bits; bits above both ids are ignored).  The
+// vertices between two keys' majors
 // (and after the last) share one offset: up to GAP_INLINE of them are written
 // by the key's own thread, longer runs go to the gap list in pieces for
 // fill_gaps (a hot-source numbering ends with all vertices without a list: 30
@@ -250,11 +252,11 @@ __global__ void offsets_from_keys(const uint64_t *__restrict__ keys, size_t n, i
   const uint64_t mask = (1ull << bits) - 1;
   for (size_t i = (size_t)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += (size_t)gridDim.x * blockDim.x) {
     const uint64_t k = keys[i];
-    const uint64_t low = k & mask, high = k >> bits;
+    const uint64_t low = k & mask, high = (k >> bits) & mask;
     const uint64_t maj = low_major ? low : high;
     nbr[i] = (uint32_t)(low_major ? high : low);
     uint64_t next = 0;  // first vertex without an offset yet
-    if (i) next = (low_major ? keys[i - 1] & mask : keys[i - 1] >> bits) + 1;
+    if (i) next = ((low_major ? keys[i - 1] : keys[i - 1] >> bits) & mask) + 1;
     if (next <= maj) write_gap(off, next, maj + 1, i, gaps, ngaps);
     if (i == n - 1) write_gap(off, maj + 1, (uint64_t)V + 1, n, gaps, ngaps);
   }
@@ -376,6 +378,7 @@ int bits_for(uint32_t V) {
 static void free_sell(gg_graph *g, Dir *d);
 static int sell_or_plain(gg_graph *g, Dir *d);
 static void hot_bins(const gg_graph *g, Dir *d);
+static int ranks_build(gg_graph *g);
 
 // Degree bins of one direction (see Dir): the long lists (deg > light) with
 // their aligned chunks, split into medium and heavy ones for the BFS pulls.
@@ -472,7 +475,8 @@ int rebuild_bins(gg_graph *g, uint32_t light, uint32_t chunk, uint32_t vec) {
     GG_TRY(build_bins(g, &g->in));
   }
   g->bins_set = 1;
-  Dir *hot[2] = {g->pr_ready ? &g->pr : nullptr, g->pr_out_ready ? &g->pr_out : nullptr};
+  Dir *hot[3] = {g->pr_ready ? &g->pr : nullptr, g->pr_out_ready ? &g->pr_out : nullptr,
+                 g->ps_ready ? &g->ps : nullptr};
   for (Dir *d : hot) {
     if (!d) continue;
     const bool rows = d->sell_desc != nullptr;
@@ -633,6 +637,19 @@ __global__ void rank_tables(const uint64_t *__restrict__ keys, uint32_t V, int b
   }
 }
 
+// Classes of equal width over the weights' range [wmin, wmin + range]
+// (bits = 0: none), for lists ordered by weight.
+constexpr int WEIGHT_BITS = 6;
+struct WeightClass {
+  int bits = 0;
+  float wmin = 0.0f, inv = 0.0f;  // inv: classes per unit of weight
+  __device__ __forceinline__ uint32_t of(float w) const {
+    const float x = __fmul_rn(__fsub_rn(w, wmin), inv);  // monotone in w
+    const float top = (float)((1 << bits) - 1);
+    return x >= top ? (1u << bits) - 1u : x > 0.0f ? (uint32_t)x : 0u;
+  }
+};
+
 // Entry p of the lists taken in the order list_of[0], list_of[1], ... (null:
 // 0, 1, ...), list r at first[r]: keys[p] = (r << bits) | rank_of[its
 // neighbour] (rank_of null: the neighbour), vals[p] = its weight.  Tiles of
@@ -644,7 +661,7 @@ constexpr int EX_TILE = 2048;
 __global__ void __launch_bounds__(EX_THREADS)
     expand_keys(Dir d, const uint64_t *__restrict__ first, uint32_t nlist, const uint32_t *__restrict__ list_of,
                 const uint32_t *__restrict__ rank_of, size_t n, int bits, uint64_t *__restrict__ keys,
-                uint32_t *__restrict__ vals) {
+                uint32_t *__restrict__ vals, WeightClass wc) {
   __shared__ uint64_t s_first[EX_TILE + 1];
   __shared__ uint64_t s_off[EX_TILE + 1];
   __shared__ uint32_t s_lo, s_hi;
@@ -679,8 +696,13 @@ __global__ void __launch_bounds__(EX_THREADS)
       const uint64_t k = staged ? s_off[a] + (p - s_first[a])
                                 : d.off[list_of ? list_of[lo + a] : lo + a] + (p - first[lo + a]);
       const uint32_t u = nbr_at(d, k, GG_SITE);
-      keys[p] = ((uint64_t)(lo + a) << bits) | (rank_of ? rank_of[u] : u);
-      if (vals) vals[p] = __float_as_uint(d.w[k]);
+      uint64_t key = ((uint64_t)(lo + a) << bits) | (rank_of ? rank_of[u] : u);
+      if (vals) {
+        const float w = d.w[k];
+        vals[p] = __float_as_uint(w);
+        if (wc.bits) key |= (uint64_t)wc.of(w) << (2 * bits);
+      }
+      keys[p] = key;
     }
     __syncthreads();
   }
@@ -831,51 +853,60 @@ static void free_hot_dir(gg_graph *g, Dir *d) {
 }
 
 void pr_layout_free(gg_graph *g) {
-  if (!g->pr_ready) return;
+  if (!g->ranks_ready) return;
   cudaStreamSynchronize(g->stream);
-  const size_t V = g->V;
-  g->graph_bytes -= sizeof(uint32_t) * 3 * V;
-  free_hot_dir(g, &g->pr);
+  if (g->pr_ready) free_hot_dir(g, &g->pr);
   if (g->pr_out_ready) free_hot_dir(g, &g->pr_out);
-  g->pr_out_ready = false;
+  if (g->ps_ready) free_hot_dir(g, &g->ps);
+  g->pr_ready = g->pr_out_ready = g->ps_ready = false;
+  g->graph_bytes -= sizeof(uint32_t) * 3 * (size_t)g->V;
   cudaFree(g->pr_rank_of);
   g->pr_rank_of = g->pr_id_of_rank = g->pr_od = nullptr;
-  g->pr_ready = false;
+  g->ranks_ready = false;
 }
 
-// The transpose of src's lists taken in the order of list_of, as a direction:
-// its list r' holds the numbers r of the lists that hold r', ascending.  The
-// expansion walks the lists in ascending number, so one stable sort on the
-// other end's number alone orders both (half the passes of a sort on the
-// pair).  Weights are carried along; duplicate edges keep src's order.
-// first: V + 1 positions of the lists in that order.
-static int transpose_dir(gg_graph *g, const Dir &src, const uint64_t *first, const uint32_t *list_of,
-                         const uint32_t *rank_of, Dir *dst) {
+// The transpose of src's lists taken in rank order, in the hot-source
+// numbering: list r' holds the ranks r of the lists that hold r', ascending
+// (wc: by weight class, then ascending).  The expansion walks the lists in
+// ascending rank, so one stable sort on the other end's rank alone orders
+// both (half the passes of a sort on the pair).  Weights are carried along;
+// duplicate edges keep src's order.
+static int transpose_dir(gg_graph *g, const Dir &src, Dir *dst, WeightClass wc = WeightClass()) {
   const size_t n = g->nadj;
   const int bits = bits_for(g->V);
   DevScratch tmp;
+  uint64_t *first = nullptr, *scan = nullptr;
   uint64_t *k0 = nullptr, *k1 = nullptr, *ks = nullptr;
   uint32_t *v0 = nullptr, *v1 = nullptr, *vs = nullptr;
   void *scratch = nullptr;
+  GG_TRY(tmp.get(&first, (size_t)g->V + 1 + scan_scratch_elems(g->V)));
+  scan = first + g->V + 1;
   GG_TRY(tmp.sort_buffers(n, g->weighted != 0, &k0, &k1, &v0, &v1, &scratch));
+  GG_CUDA((exclusive_scan<unsigned long long, QueueDegreeIn>(QueueDegreeIn{g->pr_id_of_rank, src.deg}, g->V,
+                                                             (unsigned long long *)first, (unsigned long long *)scan,
+                                                             g->stream, nullptr)));
   if (n) {
     expand_keys<<<grid_for((n + EX_TILE - 1) / EX_TILE * EX_THREADS, EX_THREADS, g->num_sms, 6), EX_THREADS, 0,
-                  g->stream>>>(src, first, g->V, list_of, rank_of, n, bits, k0, v0);
+                  g->stream>>>(src, first, g->V, g->pr_id_of_rank, g->pr_rank_of, n, bits, k0, v0, wc);
     GG_CUDA(cudaGetLastError());
   }
   *dst = Dir();
   dst->vec = src.vec;
   hot_bins(g, dst);
-  return sort_dir(g, scratch, k0, k1, v0, v0, v1, n, bits, true, dst, false, &ks, &vs);
+  uint64_t *ka = k0;
+  uint32_t *va = v0;
+  if (wc.bits) {
+    const SortValues v{v0, v0, v1, nullptr};
+    GG_TRY(radix_sort(g, scratch, k0, k1, v, n, 2 * bits, 2 * bits + wc.bits, &ka, &va));
+  }
+  return sort_dir(g, scratch, ka, ka == k0 ? k1 : k0, va, va, va == v0 ? v1 : v0, n, bits, true, dst, false, &ks, &vs);
 }
 
-// The outgoing adjacency in the hot-source numbering: the transpose of the
-// renumbered incoming one.
+// The outgoing adjacency in the hot-source numbering.
 int hot_out_build(gg_graph *g) {
   if (g->pr_out_ready) return GG_OK;
-  GG_TRY(pr_layout_build(g));
-  GG_CUDA(cudaSetDevice(g->device));
-  const int s = transpose_dir(g, g->pr, g->pr.off, nullptr, nullptr, &g->pr_out);
+  GG_TRY(ranks_build(g));
+  const int s = transpose_dir(g, g->in, &g->pr_out);
   if (s != GG_OK) {
     free_hot_dir(g, &g->pr_out);
     return s;
@@ -891,57 +922,122 @@ int hot_out_rows(gg_graph *g) {
   return g->pr_out.sell_desc ? GG_OK : sell_or_plain(g, &g->pr_out);
 }
 
-// The vertices ranked by degree_rank_keys: the
-// three tables and the positions of the out-lists taken in that order.
-static int rank_vertices(gg_graph *g, uint64_t *first) {
+// The vertices ranked by degree_rank_keys: the numbering's three tables.
+static int ranks_build(gg_graph *g) {
+  if (g->ranks_ready) return GG_OK;
+  GG_CUDA(cudaSetDevice(g->device));
   const uint32_t V = g->V;
   const int bits = bits_for(V);
   DevScratch tmp;
   uint64_t *k0 = nullptr, *k1 = nullptr, *ks = nullptr;
   uint32_t *v0 = nullptr, *v1 = nullptr, *vs = nullptr;
   void *scratch = nullptr;
-  uint64_t *scan = nullptr;
   GG_TRY(tmp.sort_buffers(V, false, &k0, &k1, &v0, &v1, &scratch));
-  GG_TRY(tmp.get(&scan, scan_scratch_elems(V)));
   degree_rank_keys<<<grid_for(V, 256, g->num_sms, 16), 256, 0, g->stream>>>(g->out.deg, g->in.deg, V, bits, k0);
   GG_CUDA(cudaGetLastError());
   // the keys start in id order and the sort is stable: the class bits suffice
   GG_TRY(radix_sort(g, scratch, k0, k1, SortValues(), V, bits, bits + RANK_BITS, &ks, &vs));
+  uint32_t *tables = nullptr;
+  GG_CUDA(cudaMalloc(&tables, sizeof(uint32_t) * 3 * (size_t)V));
+  g->pr_rank_of = tables;
+  g->pr_id_of_rank = tables + V;
+  g->pr_od = tables + 2 * (size_t)V;
+  g->graph_bytes += sizeof(uint32_t) * 3 * (size_t)V;
+  g->ranks_ready = true;
   rank_tables<<<grid_for(V, 256, g->num_sms, 16), 256, 0, g->stream>>>(ks, V, bits, g->out.deg, g->pr_id_of_rank,
                                                                       g->pr_rank_of, g->pr_od);
   GG_CUDA(cudaGetLastError());
-  GG_CUDA((exclusive_scan<uint64_t, U32AsU64>(U32AsU64{g->pr_od}, V, first, scan, g->stream, nullptr)));
   GG_CUDA(cudaStreamSynchronize(g->stream));
   return GG_OK;
 }
 
+// The incoming adjacency renumbered, with its rows.
 int pr_layout_build(gg_graph *g) {
   if (g->pr_ready) return GG_OK;
-  GG_CUDA(cudaSetDevice(g->device));
-  const uint32_t V = g->V;
-  GG_CUDA(cudaMalloc(&g->pr_rank_of, sizeof(uint32_t) * 3 * (size_t)V));
-  g->pr_id_of_rank = g->pr_rank_of + V;
-  g->pr_od = g->pr_id_of_rank + V;
-  g->graph_bytes += sizeof(uint32_t) * 3 * (size_t)V;
-  DevScratch tmp;
-  uint64_t *first = nullptr;
-  int status = tmp.get(&first, (size_t)V + 1);
-  if (status == GG_OK) status = rank_vertices(g, first);
-  // the incoming adjacency renumbered (the transpose of the out-lists in
-  // rank order), with its weights when the graph has them (SSSP's pulls
-  // gather them)
-  if (status == GG_OK) {
-    status = transpose_dir(g, g->out, first, g->pr_id_of_rank, g->pr_rank_of, &g->pr);
-    if (status != GG_OK) free_hot_dir(g, &g->pr);
-  }
-  if (status != GG_OK) {
-    cudaFree(g->pr_rank_of);
-    g->graph_bytes -= sizeof(uint32_t) * 3 * (size_t)V;
-    g->pr_rank_of = g->pr_id_of_rank = g->pr_od = nullptr;
-    return status;
+  GG_TRY(ranks_build(g));
+  const int s = transpose_dir(g, g->out, &g->pr);
+  if (s != GG_OK) {
+    free_hot_dir(g, &g->pr);
+    return s;
   }
   g->pr_ready = true;
   return sell_or_plain(g, &g->pr);
+}
+
+// Least and largest weight (NaN weights left out), as ordered integers.
+__device__ __forceinline__ uint32_t float_order(float x) {
+  const uint32_t u = __float_as_uint(x);
+  return u & 0x80000000u ? ~u : u | 0x80000000u;
+}
+__global__ void weight_range(const float *__restrict__ w, size_t n, uint32_t *range) {
+  uint32_t lo = 0xffffffffu, hi = 0;
+  for (size_t i = (size_t)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += (size_t)gridDim.x * blockDim.x) {
+    const float x = w[i];
+    if (x != x) continue;
+    const uint32_t o = float_order(x);
+    lo = o < lo ? o : lo;
+    hi = o > hi ? o : hi;
+  }
+  lo = __reduce_min_sync(GG_FULL, lo);
+  hi = __reduce_max_sync(GG_FULL, hi);
+  if (lane_id() == 0) {
+    if (lo != 0xffffffffu) atomicMin(range, lo);
+    if (hi) atomicMax(range + 1, hi);
+  }
+}
+static float float_of_order(uint32_t o) {
+  const uint32_t u = o & 0x80000000u ? o & 0x7fffffffu : ~o;
+  float f;
+  memcpy(&f, &u, sizeof f);
+  return f;
+}
+
+// SSSP's layout: the incoming adjacency renumbered, each list by ascending
+// weight class (64 classes of equal width), with its rows, and for a directed
+// graph the outgoing adjacency.  A dense call relaxes only what an active
+// source can improve: with the active sources' least distance, a list's walk
+// ends where that distance plus the next weight reaches the vertex's own.  On
+// R-MAT graphs with weights in [0, 1) a hub settles near the least active
+// distance, so most of its list is never gathered.  R-MAT 24, 268 M entries:
+// 11.1 ms walking every list, 5.7 ms so; the class pass adds 2.4 ms to the
+// layout's build.
+int sssp_layout_build(gg_graph *g) {
+  GG_TRY(ranks_build(g));
+  if (!g->ps_ready) {
+    WeightClass wc;
+    g->ps_width = INFINITY;
+    g->ps_wmin = -INFINITY;
+    if (g->nadj && 2 * bits_for(g->V) + WEIGHT_BITS <= 64) {
+      DevScratch tmp;
+      uint32_t *dev = nullptr, h[2] = {0xffffffffu, 0u};
+      GG_TRY(tmp.get(&dev, 2));
+      GG_CUDA(cudaMemcpyAsync(dev, h, sizeof(h), cudaMemcpyHostToDevice, g->stream));
+      weight_range<<<grid_for(g->nadj, 256, g->num_sms, 8), 256, 0, g->stream>>>(g->in.w, g->nadj, dev);
+      GG_CUDA(cudaGetLastError());
+      GG_CUDA(cudaMemcpyAsync(h, dev, sizeof(h), cudaMemcpyDeviceToHost, g->stream));
+      GG_CUDA(cudaStreamSynchronize(g->stream));
+      const float lo = float_of_order(h[0]), hi = float_of_order(h[1]), range = hi - lo;
+      if (h[0] <= h[1] && isfinite(lo) && isfinite(hi) && isfinite(range)) {
+        g->ps_wmin = lo;
+        wc.wmin = lo;
+        const float classes = (float)(1 << WEIGHT_BITS);
+        if (range > 0.0f && isfinite(classes / range)) {
+          wc.bits = WEIGHT_BITS;
+          wc.inv = classes / range;
+          // a class's width and the rounding of its bounds (see WeightClass)
+          g->ps_width = range / classes * 1.001f + 1e-6f * fmaxf(fabsf(lo), fabsf(hi));
+        }
+      }
+    }
+    const int s = transpose_dir(g, g->out, &g->ps, wc);
+    if (s != GG_OK) {
+      free_hot_dir(g, &g->ps);
+      return s;
+    }
+    g->ps_ready = true;
+    GG_TRY(sell_or_plain(g, &g->ps));
+  }
+  return g->symmetric ? GG_OK : hot_out_build(g);
 }
 
 void graph_destroy(gg_graph *g) {

@@ -447,8 +447,9 @@ int gg_graph_set_l1_hot(gg_graph *g, uint32_t l1_bytes);
  * adjacency entries / divisor; 0 always pulls.  A source that is not active
  * cannot lower a neighbour's label or distance, so both forms give the same
  * values, the same activated set and the same per-call trace (which records
- * the reference's mode).  Default 4 (measured on R-MAT 25 SSSP: 131 -> 145
- * GTEPS; CC on R-MAT 26 unchanged). */
+ * the reference's mode).  Default 4; until this is called, gg_sssp on the
+ * hot-source layout uses 16, since its pulls there end most lists early
+ * (R-MAT 24: 7.2 ms with 4, 5.7 ms with 16). */
 int gg_graph_set_dense_push(gg_graph *g, uint32_t divisor);
 
 /* Kernel choice of gg_bfs / gg_bfs_many (the reference's dense mode is the
