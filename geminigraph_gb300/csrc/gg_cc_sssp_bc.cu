@@ -5,6 +5,7 @@
 #include <vector>
 
 #include "gg_engine.cuh"
+#include "gg_resident.cuh"
 
 namespace gg {
 
@@ -175,10 +176,8 @@ __global__ void active_min(const uint32_t *__restrict__ q, uint32_t n, const uin
 // CC's first call, every vertex active with its own id as label: the least
 // in-neighbour, the first entry of the (plain) in-list.  v in the numbering
 // of the labels, id_of its vertex (null: v itself).
-__global__ void __launch_bounds__(PULL_THREADS)
-    cc_first(Dir d, uint32_t V, const uint32_t *__restrict__ id_of, uint32_t *__restrict__ label, ActOut act,
-             Counters *ctr) {
-  Tally t;
+__device__ __forceinline__ void cc_first_walk(const Dir &d, uint32_t V, const uint32_t *id_of, uint32_t *label,
+                                              const ActOut &act, Tally &t) {
   const size_t groups = ((size_t)V + 31) / 32, nwarps = (size_t)gridDim.x * (PULL_THREADS / 32);
   for (size_t g = (size_t)blockIdx.x * (PULL_THREADS / 32) + (threadIdx.x >> 5); g < groups; g += nwarps) {
     const uint32_t v = (uint32_t)(g * 32 + lane_id());
@@ -194,13 +193,19 @@ __global__ void __launch_bounds__(PULL_THREADS)
     }
     pull_activate(a, v, g, act, t);
   }
+}
+__global__ void __launch_bounds__(PULL_THREADS)
+    cc_first(Dir d, uint32_t V, const uint32_t *__restrict__ id_of, uint32_t *__restrict__ label, ActOut act,
+             Counters *ctr) {
+  Tally t;
+  cc_first_walk(d, V, id_of, label, act, t);
   t.flush(ctr);
 }
 
 // The least vertex with an out-edge (V if none), by one block over the
 // deg > 0 bitmap.
-__global__ void __launch_bounds__(1024) least_source(const uint32_t *__restrict__ nz, size_t words, uint32_t V,
-                                                     uint32_t *out) {
+__device__ __forceinline__ void least_source_block(const uint32_t *__restrict__ nz, size_t words, uint32_t V,
+                                                   uint32_t *out) {
   __shared__ uint32_t s_min;
   if (threadIdx.x == 0) s_min = V;
   __syncthreads();
@@ -212,13 +217,343 @@ __global__ void __launch_bounds__(1024) least_source(const uint32_t *__restrict_
   }
   if (threadIdx.x == 0) *out = s_min;
 }
+__global__ void __launch_bounds__(1024) least_source(const uint32_t *__restrict__ nz, size_t words, uint32_t V,
+                                                     uint32_t *out) {
+  least_source_block(nz, words, V, out);
+}
+
+// ------------------------------------------------------------------ resident CC / SSSP
+// What a resident run needs of the two toolkits.
+struct CcRun {
+  using T = uint32_t;
+  using Pull = CcPull;
+  static constexpr bool kWeighted = false;
+  // largest graph (entries) run whole: R-MAT 18 / 20 / 22 / 24 (2^27 to 2^29
+  // entries the last two) 293 / 323 / 497 / 1153 us from the host, 160 / 189 /
+  // 358 / 1235 so
+  static constexpr unsigned long long kWhole = 1ull << 28;
+  static __device__ __forceinline__ T cand(T msg, float) { return msg; }
+  static __device__ __forceinline__ T amin(T *p, T x) { return atomicMin(p, x); }
+};
+struct SsspRun {
+  using T = float;
+  using Pull = SsspPull;
+  static constexpr bool kWeighted = true;
+  // R-MAT 16 / 18 / 20 / 24: 834 / 928 / 1519 / 5740 us from the host, 446 /
+  // 601 / 1501 / 12400 so (its pulls have fewer warps than the host's kernels)
+  static constexpr unsigned long long kWhole = 1ull << 24;
+  static __device__ __forceinline__ T cand(T msg, float w) { return __fadd_rn(msg, w); }
+  // write_min, returning the value before (see atomic_min_float)
+  static __device__ __forceinline__ T amin(T *p, T x) {
+    if (!(x < 0.0f)) return __int_as_float(atomicMin((int *)p, __float_as_int(x)));
+    return __uint_as_float(atomicMax((unsigned *)p, __float_as_uint(x)));
+  }
+};
+
+struct RelaxArgs {
+  Dir out, in;                    // the run's numbering; in.sell_desc: pulls can run here
+  Dir plain_in;                   // CC's first call
+  const uint32_t *plain_nz;
+  const uint32_t *id_of, *rank_of;  // null: the run is in vertex order
+  uint32_t *q[2], *bm[2];
+  void *a[2], *result, *partials;
+  ResTally *slots;                // three
+  uint32_t *word;                 // one value between the run's start and its first call
+  ResRow *rows;                   // the calls' rows while the run goes on
+  ResOut *out_host;               // mapped host memory
+  void *result_host;              // also the result, when it fits (mapped)
+  unsigned long long edges_lim;   // edges / 20
+  unsigned long long nadj;
+  uint32_t V, push_div, root;
+  uint32_t init;                  // 1: start of a traversal; 2: continued by another launch; 0: entered from the host loop
+  uint32_t whole;                 // no call is too large
+};
+
+// Consecutive calls of the CC / SSSP loop.  Two state arrays: at the start of
+// a call every vertex's value is in the one to read (R); slots lower the other
+// (W).  Every message is read from R, which no slot of the call writes, so
+// all signals precede all slots without a snapshot.  For W to become the next
+// call's R, every vertex that R had right and W not is brought up to date
+// during the call: those are the active ones (changed in the previous call,
+// which wrote what is now R), each by the thread that expands it.  A slot that
+// lowers W[dst] below R[dst] is the first of the call to do so exactly if W
+// held R's value or more before: it appends dst to the next queue.
+template <class Run>
+__global__ void __launch_bounds__(RES_THREADS, RES_BLOCKS) relax_run(RelaxArgs p, typename Run::Pull pull, ResState st) {
+  using T = typename Run::T;
+  cooperative_groups::grid_group grid = cooperative_groups::this_grid();
+  const uint32_t V = p.V, cap = V + 1;
+  const size_t words = 2 * ((size_t)V / 64 + 1);
+  const uint32_t nthreads = gridDim.x * RES_THREADS, tid = blockIdx.x * RES_THREADS + threadIdx.x;
+  const bool first_thread = tid == 0;
+  T *a0 = (T *)p.a[0], *a1 = (T *)p.a[1];
+  __shared__ ResStage s_stage;
+  res_stage_init(s_stage);
+  uint32_t step = st.step;
+  auto slot = [&]() { return p.slots + step % 3; };
+  auto begin_step = [&]() { res_clear(p.slots + (step + 1) % 3); };
+  st.calls = 0;
+  if (p.init == 1) {
+    for (uint32_t i = tid; i < words; i += nthreads) p.bm[0][i] = p.bm[1][i] = 0u;
+    if constexpr (Run::kWeighted) {
+      const uint32_t start = p.rank_of ? p.rank_of[p.root] : p.root;
+      for (uint32_t v = tid; v < V; v += nthreads) a0[v] = a1[v] = v == start ? 0.0f : 1e9f;
+      st.ae = p.out.deg[start];
+      st.n_act = 1;
+      st.n = st.ae > RES_HUB ? 0 : 1;
+      st.hubs = 1 - st.n;
+      st.qvalid = 1;
+      if (first_thread) p.q[0][st.n ? 0 : cap - 1] = start;
+    } else {
+      for (uint32_t v = tid; v < V; v += nthreads) a0[v] = a1[v] = p.id_of ? p.id_of[v] : v;
+      st.ae = p.nadj;
+      st.n_act = V;
+      if (blockIdx.x == 0) least_source_block(p.plain_nz, words, V, p.word);
+    }
+    grid.sync();
+    if constexpr (!Run::kWeighted) pull.floor = res_read(p.word);
+  } else if (p.init == 0) {
+    const T *from = (const T *)p.a[st.role];
+    T *to = (T *)p.a[st.role ^ 1];
+    for (uint32_t v = tid; v < V; v += nthreads) to[v] = from[v];
+    // the queue with its hubs apart
+    begin_step();
+    for (uint32_t i = tid; i < st.n; i += nthreads) {
+      const uint32_t v = p.q[st.q][i];
+      res_append(v, p.out.deg[v], p.q[st.q ^ 1], cap, slot());
+    }
+    grid.sync();
+    st.n = (uint32_t)res_read(&slot()->app);
+    st.hubs = (uint32_t)res_read(&slot()->happ);
+    st.q ^= 1;
+    step++;
+  }
+  bool opening = p.init == 1 && !Run::kWeighted;
+  while (st.n_act > 0 && st.calls < RES_CALLS) {
+    const bool sparse = st.ae < p.edges_lim;
+    const bool push = sparse || (p.push_div && st.ae < p.nadj / p.push_div);
+    if (!push && !p.in.sell_desc) break;
+    if (!p.whole && (!sparse || st.n + st.hubs > RES_MAX_QUEUE || st.ae > RES_MAX_AE)) break;
+    const unsigned long long ae = st.ae;
+    const T *R = (const T *)p.a[st.role];
+    T *W = (T *)p.a[st.role ^ 1];
+    if (push) {
+      if (!st.qvalid) {
+        begin_step();
+        res_queue_from_bitmap(p.bm[st.bm], words, p.out.deg, p.q[st.q], cap, slot());
+        grid.sync();
+        st.n = (uint32_t)res_read(&slot()->app);
+        st.hubs = (uint32_t)res_read(&slot()->happ);
+        step++;
+      }
+      begin_step();
+      ResTally *sl = slot();
+      uint32_t *qn = p.q[st.q ^ 1];
+      res_expand(
+          p.out, p.q[st.q], st.n, st.hubs, st.ae, cap,
+          [&](uint32_t src, bool lead) {
+            const T msg = R[src];
+            if (lead) Run::amin(W + src, msg);
+            return msg;
+          },
+          [&](T msg, uint32_t, unsigned long long k) {
+            const uint32_t dst = nbr_at(p.out, k, GG_SITE);
+            const T x = Run::cand(msg, Run::kWeighted ? p.out.w[k] : 0.0f);
+            const T r = R[dst];
+            if (x < r) {
+              const uint32_t od = p.out.deg[dst];
+              if (!(Run::amin(W + dst, x) < r)) res_stage(dst, od, s_stage, qn, cap, sl);
+            }
+          });
+      res_stage_flush(s_stage, qn, sl);
+      grid.sync();
+      const unsigned long long app = res_read(&sl->app), happ = res_read(&sl->happ);
+      step++;
+      st.n = (uint32_t)app;
+      st.hubs = (uint32_t)happ;
+      st.n_act = st.n + st.hubs;
+      st.ae = (app >> 32) + (happ >> 32);
+      st.q ^= 1;
+      st.qvalid = 1;
+      st.role ^= 1;
+    } else {
+      typename Run::Pull op = pull;
+      op.cur = R;
+      op.nxt = W;
+      // the least active distance, which ends the walks of large graphs early;
+      // below 2^22 entries finding it takes longer (R-MAT 16 and 18: 446 and
+      // 601 us without, 556 and 745 with; R-MAT 20: 1632 and 1501)
+      if (Run::kWeighted && p.nadj > (1ull << 22)) {
+        begin_step();
+        uint32_t best = 0;
+        auto take = [&](uint32_t v) {
+          const uint32_t u = __float_as_uint((float)R[v]);
+          const uint32_t o = ~(u & 0x80000000u ? ~u : u | 0x80000000u);
+          best = o > best ? o : best;
+        };
+        if (st.qvalid) {
+          for (uint32_t i = tid; i < st.n + st.hubs; i += nthreads)
+            take(i < st.n ? p.q[st.q][i] : p.q[st.q][cap - 1 - (i - st.n)]);
+        } else {
+          for (uint32_t i = tid; i < words * 32; i += nthreads)
+            if ((p.bm[st.bm][i >> 5] >> (i & 31)) & 1u) take(i);
+        }
+        best = __reduce_max_sync(GG_FULL, best);
+        if (lane_id() == 0 && best) atomicMax(&slot()->c.aux, best);
+        grid.sync();
+        if constexpr (Run::kWeighted) op.lo_enc = &slot()->c.aux;
+        op.begin();
+        step++;
+      }
+      begin_step();
+      ActOut act;
+      act.active_out = p.bm[st.bm ^ 1];
+      act.out_deg = p.out.deg;
+      Tally t;
+      if (opening) {
+        // label[v] = v: in place, both arrays agree on what it leaves alone
+        cc_first_walk(p.plain_in, V, p.id_of, (uint32_t *)W, act, t);
+      } else {
+        const uint32_t warp = (threadIdx.x >> 5) * gridDim.x + blockIdx.x, nwarps = gridDim.x * (RES_THREADS / 32);
+        const bool parts = p.in.nheavy > 0;
+        if (!parts) long_lists<typename Run::Pull, true>(p.in, op, act, t, warp, nwarps);
+        rows_walk<typename Run::Pull, true, true>(p.in, V, op, act, t, parts ? (T *)p.partials : nullptr, warp, nwarps);
+        // the set this call was entered with has no reader any more; the next
+        // pull sets its bits there
+        for (uint32_t i = tid; i < words; i += nthreads) p.bm[st.bm][i] = 0u;
+        if (parts) {
+          grid.sync();
+          big_finish<typename Run::Pull, 8, true>(p.in, op, (const T *)p.partials, act, t);
+        }
+      }
+      t.flush(&slot()->c);
+      grid.sync();
+      st.n_act = res_read(&slot()->c.activated);
+      st.ae = res_read(&slot()->c.edges);
+      step++;
+      st.bm ^= 1;
+      st.qvalid = 0;
+      st.role ^= 1;
+      opening = false;
+    }
+    if (first_thread) p.rows[st.calls] = ResRow{ae, st.n_act, sparse ? 0u : 1u};
+    st.calls++;
+  }
+  if (st.n_act == 0) {
+    const T *R = (const T *)p.a[st.role];
+    T *out = (T *)p.result, *host = (T *)p.result_host;
+    for (uint32_t v = tid; v < V; v += nthreads) {
+      const T x = R[p.rank_of ? p.rank_of[v] : v];
+      if (p.rank_of) out[v] = x;
+      if (host) host[v] = x;
+    }
+  } else if (st.qvalid && st.calls < RES_CALLS) {
+    // back to the host loop: its queues hold vertices with out-edges only
+    begin_step();
+    res_plain_queue(p.q[st.q], st.n, st.hubs, cap, p.out.deg, p.q[st.q ^ 1], slot());
+    grid.sync();
+    st.n = (uint32_t)res_read(&slot()->app);
+    st.hubs = 0;
+    st.q ^= 1;
+    step++;
+  }
+  st.step = step % 3;
+  res_report(st, p.rows, p.out_host);
+}
+
+// A dense call pushes below this fraction of the adjacency.  A pull that ends
+// its walks early is the faster form down to fewer active edges: SSSP R-MAT
+// 24, divisors 4 / 8 / 16: 7.2 / 5.9 / 5.7 ms, R-MAT 22: 2.9 / 2.3 / 2.2 ms
+// (walking every list: 4 was the best).
+template <class PullOp>
+static uint32_t relax_push_div(const gg_graph *g, const Dir &din) {
+  return has_gather_w<PullOp>::value && din.sell_desc && !g->dense_push_set ? 16 : g->dense_push_div;
+}
+
+template <class Run>
+static int relax_args(gg_graph *g, const Dir &dout, const Dir &din, void *a0, void *a1, uint32_t *const *q,
+                      uint32_t *const *bm, RelaxArgs *p) {
+  *p = RelaxArgs{};
+  p->out = dout;
+  p->in = din;
+  p->q[0] = q[0];
+  p->q[1] = q[1];
+  p->bm[0] = bm[0];
+  p->bm[1] = bm[1];
+  p->a[0] = a0;
+  p->a[1] = a1;
+  typename Run::T *part = nullptr;
+  GG_TRY(ws(g, WS_PARTIAL, din.nbigchunks, &part));
+  p->partials = part;
+  GG_TRY(res_buffers(g, &p->slots, &p->rows, &p->word));
+  p->out_host = (ResOut *)g->ws.stage;
+  p->edges_lim = g->E / 20;
+  p->nadj = g->nadj;
+  p->V = g->V;
+  p->push_div = relax_push_div<typename Run::Pull>(g, din);
+  return GG_OK;
+}
+
+// One launch of relax_run; *st is where it stopped.
+template <class Run>
+static int relax_launch(gg_graph *g, RelaxArgs &p, typename Run::Pull pull, ResState *st, Launch &L, Trace &tr) {
+  ResState in = *st;
+  void *args[] = {&p, &pull, &in};
+  GG_TRY(res_launch(g, (const void *)relax_run<Run>, p.whole ? res_blocks(g) : (unsigned)g->num_sms, args, &in, &L));
+  *st = ((const ResOut *)g->ws.stage)->st;
+  res_trace(g, tr);
+  return GG_OK;
+}
+
+// A whole CC / SSSP traversal on the device; *ran = false where it has to run
+// from the host: a large graph (there the calls are long enough to launch one
+// by one, with kernels of their own), no rows to pull, gathers by source
+// number, or per-call times asked for.
+template <class Run>
+static int relax_whole(gg_graph *g, const Dir &dout, const Dir &din, const typename Run::Pull &pull, bool ranked,
+                       uint32_t root, void *const *a, uint32_t *const *q, uint32_t *const *bm, void *result,
+                       size_t result_bytes, Launch &L, Trace &tr, const gg_run_stats *stats, bool *ran, void **dev,
+                       const void **host) {
+  *ran = false;
+  if (g->nadj > Run::kWhole || !din.sell_desc || !pull.gathers_all(g->V) || (stats && stats->call_ms) || !L.coop_ok() ||
+      !g->ws.stage)
+    return GG_OK;
+  RelaxArgs p;
+  GG_TRY((relax_args<Run>(g, dout, din, a[0], a[1], q, bm, &p)));
+  p.plain_in = g->in;
+  p.plain_nz = g->out.nz;
+  p.id_of = ranked ? g->pr_id_of_rank : nullptr;
+  p.rank_of = ranked ? g->pr_rank_of : nullptr;
+  p.result = result;
+  p.result_host = result_bytes <= RES_RESULT_BYTES ? (char *)g->ws.stage + RES_OUT_BYTES : nullptr;
+  p.root = root;
+  p.whole = 1;
+  if (!g->dense_push_set) {
+    // CC's pulls over rows end at the floor and beat its pushes, which all
+    // lower the same hubs (R-MAT 16 / 18, a late dense call: 45 / 184 us
+    // pushing, 15 / 18 pulling; at R-MAT 24, 537 M entries, from the host,
+    // the vertices that a pull looks at are the greater cost)
+    if (!Run::kWeighted) p.push_div = 0;
+    if (Run::kWeighted && g->nadj <= RES_PUSH_ALL) p.push_div = 1;
+  }
+  p.init = 1;
+  ResState st;
+  do {
+    GG_TRY((relax_launch<Run>(g, p, pull, &st, L, tr)));
+    p.init = 2;
+  } while (st.n_act > 0);
+  *ran = true;
+  *dev = ranked ? result : a[st.role];
+  *host = p.result_host;
+  return GG_OK;
+}
 
 // Runs the CC / SSSP frontier loop: both toolkits loop while the slots
 // activate something, with a message snapshot for push calls and two state
 // buffers for pull calls.
-template <typename T, class PushOp, class PullOp>
+template <class Run, typename T, class PushOp, class PullOp>
 static int relax_loop(gg_graph *g, const Dir &dout, const Dir &din, const PullOp &pull, T *state0, T *state1,
-                      uint32_t *q0, uint32_t *q1, uint32_t *bm0, uint32_t *bm1, uint32_t n_act, uint32_t nq, uint32_t md,
+                      uint32_t *q0, uint32_t *q1, uint32_t *bm0, uint32_t *bm1, uint32_t n_act, uint32_t nq,
                       bool qvalid, unsigned long long ae, Trace &tr, Launch &L, T **result) {
   const uint32_t V = g->V;
   const size_t words = bitmap_words32(V);
@@ -228,22 +563,34 @@ static int relax_loop(gg_graph *g, const Dir &dout, const Dir &din, const PullOp
   uint32_t *q[2] = {q0, q1};
   uint32_t *bm[2] = {bm0, bm1};
   T *msg;
-  uint32_t *stamp;
   GG_TRY(ws(g, WS_MSG, (size_t)V + 1, &msg));
-  GG_TRY(ws(g, WS_STAMP, V, &stamp));
-  GG_CUDA(cudaMemsetAsync(stamp, 0, sizeof(uint32_t) * V, s));
   // A pull that ends its walks early is the faster form down to fewer active
   // edges: SSSP R-MAT 24, divisors 4 / 8 / 16: 7.2 / 5.9 / 5.7 ms, R-MAT 22:
   // 2.9 / 2.3 / 2.2 ms (walking every list: 4 was the best).
-  uint32_t push_div = g->dense_push_div;
-  if (has_gather_w<PullOp>::value && din.sell_desc && !g->dense_push_set) push_div = 16;
+  const uint32_t push_div = relax_push_div<PullOp>(g, din);
   int c_i = 0;
   while (n_act > 0) {
     bool sparse = ae < g->E / 20;
-    if (sparse && qvalid && Launch::small_ok(nq, ae, md)) {
+    if (sparse && qvalid && nq <= RES_MAX_QUEUE && ae <= RES_MAX_AE && ae > 0 && L.coop_ok()) {
       // consecutive small sparse calls run on the device without host round trips
-      GG_TRY((L.small_run<PushOp, false, T>(dout, PushOp{cur, msg}, q, &c_i, &nq, &ae, &md, &n_act, nullptr, nullptr,
-                                            cur, msg, tr, stamp)));
+      RelaxArgs p;
+      GG_TRY((relax_args<Run>(g, dout, din, cur, nxt, q, bm, &p)));
+      ResState st;
+      st.ae = ae;
+      st.n_act = n_act;
+      st.n = nq;
+      st.qvalid = 1;
+      st.q = (uint32_t)c_i;
+      GG_TRY((relax_launch<Run>(g, p, pull, &st, L, tr)));
+      ae = st.ae;
+      n_act = st.n_act;
+      nq = st.n;
+      c_i = (int)st.q;
+      if (st.role) {
+        T *t = cur;
+        cur = nxt;
+        nxt = t;
+      }
       continue;
     }
     tr.add(sparse ? 0 : 1, ae, 0);
@@ -300,7 +647,6 @@ static int relax_loop(gg_graph *g, const Dir &dout, const Dir &din, const PullOp
     GG_TRY(counters_read(g, &c));
     n_act = c.activated;
     nq = c.qlen;
-    md = c.maxdeg;
     qvalid = push;
     ae = c.edges;
     tr.set_activated(c.activated);
@@ -326,6 +672,19 @@ __global__ void unrank(const T *__restrict__ by_rank, const uint32_t *__restrict
                        T *__restrict__ out) {
   for (size_t v = (size_t)blockIdx.x * blockDim.x + threadIdx.x; v < V; v += (size_t)gridDim.x * blockDim.x)
     out[v] = by_rank[rank_of[v]];
+}
+
+// The end of a whole run: its time and its result.
+static int relax_done(gg_graph *g, gg_run_stats *st, const Launch &L, void *user, const void *dev, const void *host,
+                      size_t bytes) {
+  GG_TRY(timed_read(g, st, L.launches));
+  if (user && host)
+    memcpy(user, host, bytes);
+  else if (user)
+    GG_CUDA(cudaMemcpy(user, dev, bytes, cudaMemcpyDeviceToHost));
+  g->result[0] = dev;
+  g->result[1] = nullptr;
+  return GG_OK;
 }
 
 static int cc_run(gg_graph *g, uint32_t *label_host, gg_run_stats *st) {
@@ -354,6 +713,15 @@ static int cc_run(gg_graph *g, uint32_t *label_host, gg_run_stats *st) {
   cudaStream_t s = g->stream;
   Counters *ctr = g->ws.ctr;
   GG_TRY(timed_begin(g));
+  CcPull pull{};
+  pull.hot = ranked ? g->l1_hot_bytes / 4 : 0xffffffffu;
+  bool whole = false;
+  void *dev = nullptr;
+  const void *host = nullptr;
+  void *const states[2] = {lab[0], lab[1]};
+  GG_TRY((relax_whole<CcRun>(g, dout, din, pull, ranked, 0, states, q, bm, out, sizeof(uint32_t) * V, L, tr, st, &whole,
+                             &dev, &host)));
+  if (whole) return relax_done(g, st, L, label_host, dev, host, sizeof(uint32_t) * V);
   // label[v] = v over active_in = all (cc.cpp:31-37)
   if (ranked)
     copy_twice<uint32_t><<<grid_for(V, 256, g->num_sms), 256, 0, s>>>(g->pr_id_of_rank, V, lab[0], lab[1]);
@@ -362,8 +730,6 @@ static int cc_run(gg_graph *g, uint32_t *label_host, gg_run_stats *st) {
   L.launches += 1;
   GG_CUDA(cudaGetLastError());
   uint32_t *res = nullptr;
-  CcPull pull{};
-  pull.hot = ranked ? g->l1_hot_bytes / 4 : 0xffffffffu;
   uint32_t n_act = V;
   unsigned long long ae = g->nadj;
   // the first call: dense by the reference's switch (every vertex active)
@@ -385,8 +751,8 @@ static int cc_run(gg_graph *g, uint32_t *label_host, gg_run_stats *st) {
   pull.floor = c.aux;
   n_act = c.activated;
   ae = c.edges;
-  GG_TRY((relax_loop<uint32_t, CcPush, CcPull>(g, dout, din, pull, lab[0], lab[1], q[0], q[1], bm[0], bm[1], n_act, 0,
-                                               0xffffffffu, false, ae, tr, L, &res)));
+  GG_TRY((relax_loop<CcRun, uint32_t, CcPush, CcPull>(g, dout, din, pull, lab[0], lab[1], q[0], q[1], bm[0], bm[1], n_act, 0,
+                                               false, ae, tr, L, &res)));
   if (ranked) {
     unrank<uint32_t><<<grid_for(V, 256, g->num_sms), 256, 0, s>>>(res, g->pr_rank_of, V, out);
     L.launches += 1;
@@ -442,14 +808,23 @@ static int sssp_run(gg_graph *g, uint32_t root, float *dist_host, gg_run_stats *
   const Dir &din = ranked ? g->ps : g->in;
   uint32_t start = root;
   float *out = nullptr;
-  if (ranked) {
-    GG_CUDA(cudaMemcpy(&start, g->pr_rank_of + root, sizeof(uint32_t), cudaMemcpyDeviceToHost));
-    GG_TRY(ws(g, WS_S2, V, &out));
-  }
+  if (ranked) GG_TRY(ws(g, WS_S2, V, &out));
   Launch L(g);
   Trace tr(st, g, "gg_sssp");
   cudaStream_t s = g->stream;
+  SsspPull pull{};
+  pull.hot = ranked ? g->l1_hot_bytes / 4 : 0xffffffffu;
+  pull.wmin = g->ps_wmin;
+  pull.width = g->ps_width;
   GG_TRY(timed_begin(g));
+  bool whole = false;
+  void *dev = nullptr;
+  const void *host = nullptr;
+  void *const states[2] = {dist[0], dist[1]};
+  GG_TRY((relax_whole<SsspRun>(g, dout, din, pull, ranked, root, states, q, bm, out, sizeof(float) * V, L, tr, st, &whole,
+                               &dev, &host)));
+  if (whole) return relax_done(g, st, L, dist_host, dev, host, sizeof(float) * V);
+  if (ranked) GG_CUDA(cudaMemcpy(&start, g->pr_rank_of + root, sizeof(uint32_t), cudaMemcpyDeviceToHost));
   GG_CUDA(cudaMemsetAsync(bm[0], 0, words * 4, s));
   GG_TRY(counters_reset(g));
   fill_kernel<float><<<grid_for(V, 256, g->num_sms), 256, 0, s>>>(dist[0], V, 1e9f);
@@ -460,12 +835,8 @@ static int sssp_run(gg_graph *g, uint32_t root, float *dist_host, gg_run_stats *
   Counters c;
   GG_TRY(counters_read(g, &c));
   float *res = nullptr;
-  SsspPull pull{};
-  pull.hot = ranked ? g->l1_hot_bytes / 4 : 0xffffffffu;
-  pull.wmin = g->ps_wmin;
-  pull.width = g->ps_width;
-  GG_TRY((relax_loop<float, SsspPush, SsspPull>(g, dout, din, pull, dist[0], dist[1], q[0], q[1], bm[0], bm[1], 1,
-                                                1, c.maxdeg, true, c.edges, tr, L, &res)));
+  GG_TRY((relax_loop<SsspRun, float, SsspPush, SsspPull>(g, dout, din, pull, dist[0], dist[1], q[0], q[1], bm[0], bm[1], 1,
+                                                1, true, c.edges, tr, L, &res)));
   if (ranked) {
     unrank<float><<<grid_for(V, 256, g->num_sms), 256, 0, s>>>(res, g->pr_rank_of, V, out);
     L.launches += 1;

@@ -118,7 +118,7 @@ enum WsSlot {
   WS_PARTIAL,                           // per-chunk partial results of heavy lists
   WS_PIPE,                              // second result buffer of the pipelined calls
   WS_QPOS,                              // per-word queue positions (queue_from_bitmap)
-  WS_STAMP,                             // per-vertex activation stamps (small sparse runs)
+  WS_RES,                               // resident runs: tally slots and call rows
   WS_SMALL,                             // SmallRun state and its trace rows
   WS_MS_VISIT, WS_MS_FRONT, WS_MS_NEXT, // batched traversals: lane masks
   WS_MS_LVL, WS_MS_PAR, WS_MS_DIST,     // batched traversals: per-lane state (vertex-major)
@@ -245,6 +245,7 @@ struct gg_graph {
   // best for SSSP on R-MAT 25, neutral for CC on R-MAT 26)
   uint32_t dense_push_div = 4;
   int dense_push_set = 0;  // gg_graph_set_dense_push was called
+  int res_step = -1;       // tally slot of the next resident launch (-1: the slots are not clear)
   // PageRank's iterations captured as one CUDA graph, replayed while the key
   // (arguments, buffers, events) is unchanged
   cudaGraphExec_t pr_exec[2] = {nullptr, nullptr};  // float, double
@@ -366,6 +367,7 @@ struct Trace {
 int check_status(gg_graph *g);
 int timed_begin(gg_graph *g);
 int timed_end(gg_graph *g, gg_run_stats *st, int launches);
+int timed_read(gg_graph *g, gg_run_stats *st, int launches);  // the end is recorded and reached
 
 // ---------------------------------------------------------------- device helpers
 __device__ __forceinline__ bool bm_test(const uint32_t *bm, uint32_t v) {

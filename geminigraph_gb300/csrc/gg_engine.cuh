@@ -88,11 +88,16 @@ __device__ __forceinline__ void push_activate(bool pred, uint32_t v, const ActOu
 }
 
 // Pull activation: the warp owns bitmap word g (vertices 32g..32g+31), so the
-// word is written with plain stores.  All lanes must call.
+// word is written with plain stores (SHARED: with an atomic, where other
+// warps set bits of the word too).  All lanes must call.
+template <bool SHARED = false>
 __device__ __forceinline__ void pull_activate(bool act, uint32_t v, size_t g, const ActOut &a, Tally &t) {
   unsigned bits = __ballot_sync(GG_FULL, act);
   if (lane_id() == 0 && bits) {
-    a.active_out[g] = bits;
+    if (SHARED)
+      atomicOr(a.active_out + g, bits);
+    else
+      a.active_out[g] = bits;
     if (a.visited) a.visited[g] |= bits;
   }
   if (act) {
@@ -415,10 +420,9 @@ struct Running<Op, std::enable_if_t<Op::kCompensated>> {
 // longest lists lead, and 32 of them in one warp are combined one after
 // another (R-MAT 20: 32 us of a 75-us iteration).
 template <class Op, uint32_t SERIAL, bool SPREAD>
-__global__ void __launch_bounds__(PULL_THREADS)
-    pull_big_finish(Dir d, Op op, const typename Op::Acc *__restrict__ partials, ActOut act, Counters *ctr) {
+__device__ __forceinline__ void big_finish(const Dir &d, const Op &op, const typename Op::Acc *partials,
+                                           const ActOut &act, Tally &t) {
   using Acc = typename Op::Acc;
-  Tally t;
   const size_t stride = (size_t)gridDim.x * PULL_THREADS;
   const size_t n = SPREAD ? ((size_t)d.nbig + stride - 1) / stride * stride : ((size_t)d.nbig + 31) / 32 * 32;
   const unsigned lane = lane_id();
@@ -458,6 +462,12 @@ __global__ void __launch_bounds__(PULL_THREADS)
     const bool a = todo && op.finish(v, acc, d.deg[v], t);
     if (act.active_out) push_activate(a, v, act, t);
   }
+}
+template <class Op, uint32_t SERIAL, bool SPREAD>
+__global__ void __launch_bounds__(PULL_THREADS)
+    pull_big_finish(Dir d, Op op, const typename Op::Acc *partials, ActOut act, Counters *ctr) {
+  Tally t;
+  big_finish<Op, SERIAL, SPREAD>(d, op, partials, act, t);
   pull_flush<Op, PULL_THREADS>(t, act.active_out != nullptr, ctr);
 }
 
@@ -505,55 +515,62 @@ struct has_stop<Op, std::void_t<decltype(&Op::stop)>> : std::true_type {};
 constexpr int ROWS_THREADS = 256;
 constexpr int ROWS_BLOCKS = 4;  // per SM
 constexpr int ROWS_Q = 2;       // columns of four entries in flight per lane
+// walk_list: entries [b, e) of vertex v's list by a warp, the combined result
+// in all lanes.
 template <class Op, bool ALL>
-__global__ void __launch_bounds__(ROWS_THREADS, ROWS_BLOCKS)
-    pull_rows(Dir d, uint32_t V, Op op, ActOut act, Counters *ctr, typename Op::Acc *__restrict__ partials) {
+__device__ __forceinline__ typename Op::Acc walk_list(const Dir &d, const Op &op, uint32_t v, unsigned long long b,
+                                                      unsigned long long e) {
+  using Acc = typename Op::Acc;
+  constexpr bool WT = has_gather_w<Op>::value;
+  constexpr bool STOP = has_stop<Op>::value;
+  constexpr int CH = 8;
+  const unsigned lane = lane_id();
+  Running<Op> run(STOP ? op.identity(v) : op.identity_coop());
+  const uint32_t n = (uint32_t)(e - b);
+  for (uint32_t k0 = lane; k0 - lane < n; k0 += 32 * CH) {
+    uint32_t u[CH];
+    float wt[WT ? CH : 1];
+#pragma unroll
+    for (int j = 0; j < CH; j++) {
+      const uint32_t k = k0 + 32 * j;
+      u[j] = k < n ? nbr_once(d, b + k, GG_SITE) : 0u;
+      if constexpr (WT) wt[j] = k < n ? ld_once(d.w + b + k) : 0.0f;
+    }
+    if constexpr (STOP) {
+      // lane 0 holds the batch's first entry: with any lane's result
+      const Acc best = op.warp_combine(run.value());
+      float first = 0.0f;
+      if constexpr (WT) first = __shfl_sync(GG_FULL, wt[0], 0);
+      if (op.stop(best, first)) break;
+    }
+    Acc g[CH];
+#pragma unroll
+    for (int j = 0; j < CH; j++) {
+      const uint32_t k = k0 + 32 * j;
+      g[j] = k < n ? op.template value<ALL>(u[j], WT ? wt[WT ? j : 0] : 0.0f) : op.identity_coop();
+    }
+    run.add(op, combine_tree<CH>(op, g));
+  }
+  return op.warp_combine(run.value());
+}
+
+// rows_walk: the part of warp `warp` of `nwarps`; partials null: the long
+// lists are somebody else's (SHARED: in the same step).
+template <class Op, bool ALL, bool SHARED>
+__device__ __forceinline__ void rows_walk(const Dir &d, uint32_t V, const Op &op, const ActOut &act, Tally &t,
+                                          typename Op::Acc *partials, uint32_t warp, uint32_t nwarps) {
   using Acc = typename Op::Acc;
   constexpr bool WT = has_gather_w<Op>::value;
   constexpr bool DENSE = has_dense<Op>::value && sizeof(Acc) == 8;
   constexpr bool STOP = has_stop<Op>::value;
-  constexpr int CH = 8;
-  if constexpr (STOP) op.begin();
-  Tally t;
-  const uint32_t nwarps = gridDim.x * (ROWS_THREADS / 32);
-  // consecutive slices and chunks on different SMs
-  const uint32_t warp = (threadIdx.x >> 5) * gridDim.x + blockIdx.x;
   const unsigned lane = lane_id();
-  for (uint32_t c = warp; c < d.nbigchunks; c += nwarps) {
+  for (uint32_t c = warp; partials && c < d.nbigchunks; c += nwarps) {
     uint32_t v;
     unsigned long long lo, b, e;
     big_range(d, c, d.chunk, &v, &lo, &b, &e);
-    Running<Op> run(STOP ? op.identity(v) : op.identity_coop());
     bool walk = op.want(v);
     if constexpr (STOP) walk = walk && !op.skip(v);
-    if (walk) {
-      const uint32_t n = (uint32_t)(e - b);
-      for (uint32_t k0 = lane; k0 - lane < n; k0 += 32 * CH) {
-        uint32_t u[CH];
-        float wt[WT ? CH : 1];
-#pragma unroll
-        for (int j = 0; j < CH; j++) {
-          const uint32_t k = k0 + 32 * j;
-          u[j] = k < n ? nbr_once(d, b + k, GG_SITE) : 0u;
-          if constexpr (WT) wt[j] = k < n ? ld_once(d.w + b + k) : 0.0f;
-        }
-        if constexpr (STOP) {
-          // lane 0 holds the batch's first entry: with any lane's result
-          const Acc best = op.warp_combine(run.value());
-          float first = 0.0f;
-          if constexpr (WT) first = __shfl_sync(GG_FULL, wt[0], 0);
-          if (op.stop(best, first)) break;
-        }
-        Acc g[CH];
-#pragma unroll
-        for (int j = 0; j < CH; j++) {
-          const uint32_t k = k0 + 32 * j;
-          g[j] = k < n ? op.template value<ALL>(u[j], WT ? wt[WT ? j : 0] : 0.0f) : op.identity_coop();
-        }
-        run.add(op, combine_tree<CH>(op, g));
-      }
-    }
-    const Acc part = op.warp_combine(run.value());
+    const Acc part = walk ? walk_list<Op, ALL>(d, op, v, b, e) : op.identity_coop();
     if (lane == 0) partials[c] = part;
   }
   const uint32_t nsl = op.zero_kept() ? d.nfull : d.nslices;
@@ -641,9 +658,32 @@ __global__ void __launch_bounds__(ROWS_THREADS, ROWS_BLOCKS)
       }
     }
     const bool a = todo && op.finish(v, run.value(), deg, t);
-    if (act.active_out) pull_activate(a, v, ds.x, act, t);
+    if (act.active_out) pull_activate<SHARED>(a, v, ds.x, act, t);
     ds = dn;
   }
+}
+// The long lists by a warp each, finished at once: for graphs whose lists are
+// short enough that a barrier and partial results take longer.
+template <class Op, bool ALL>
+__device__ __forceinline__ void long_lists(const Dir &d, const Op &op, const ActOut &act, Tally &t, uint32_t warp,
+                                           uint32_t nwarps) {
+  for (uint32_t i = warp; i < d.nbig; i += nwarps) {
+    const uint32_t v = d.big[i];
+    bool walk = op.want(v);
+    if constexpr (has_stop<Op>::value) walk = walk && !op.skip(v);
+    const typename Op::Acc part = walk ? walk_list<Op, ALL>(d, op, v, d.off[v], d.off[v + 1]) : op.identity_coop();
+    const bool a = lane_id() == 0 && op.want(v) && op.finish(v, op.combine(op.identity(v), part), d.deg[v], t);
+    if (act.active_out) push_activate(a, v, act, t);
+  }
+}
+template <class Op, bool ALL>
+__global__ void __launch_bounds__(ROWS_THREADS, ROWS_BLOCKS)
+    pull_rows(Dir d, uint32_t V, Op op, ActOut act, Counters *ctr, typename Op::Acc *partials) {
+  if constexpr (has_stop<Op>::value) op.begin();
+  Tally t;
+  // consecutive slices and chunks on different SMs
+  rows_walk<Op, ALL, false>(d, V, op, act, t, partials, (threadIdx.x >> 5) * gridDim.x + blockIdx.x,
+                            gridDim.x * (ROWS_THREADS / 32));
   pull_flush<Op, ROWS_THREADS>(t, act.active_out != nullptr, ctr);
 }
 
