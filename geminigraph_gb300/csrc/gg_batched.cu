@@ -1466,7 +1466,7 @@ __global__ void ms_advance(MsState *st, const MsCounters *mc, int bfs, cudaGraph
 
 static bool same_dir(const Dir &a, const Dir &b) {
   return a.light == b.light && a.chunk == b.chunk && a.vec == b.vec && a.off == b.off && a.nbr == b.nbr &&
-         a.w == b.w && a.deg == b.deg && a.nz == b.nz && a.med == b.med && a.nmed == b.nmed && a.heavy == b.heavy &&
+         a.w == b.w && a.deg == b.deg && a.nz == b.nz && a.heavy == b.heavy &&
          a.nheavy == b.nheavy && a.heavy_chunk == b.heavy_chunk && a.chunk_owner == b.chunk_owner &&
          a.nchunks == b.nchunks && a.big == b.big && a.nbig == b.nbig && a.big_chunk == b.big_chunk &&
          a.big_owner == b.big_owner && a.nbigchunks == b.nbigchunks && a.nv == b.nv && a.ne == b.ne &&

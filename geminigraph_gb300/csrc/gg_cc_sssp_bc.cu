@@ -282,9 +282,10 @@ template <class Run>
 __global__ void __launch_bounds__(RES_THREADS, RES_BLOCKS) relax_run(RelaxArgs p, typename Run::Pull pull, ResState st) {
   using T = typename Run::T;
   cooperative_groups::grid_group grid = cooperative_groups::this_grid();
-  const uint32_t V = p.V, cap = V + 1;
+  const uint32_t V = p.V;
+  const size_t cap = (size_t)V + 1;
   const size_t words = 2 * ((size_t)V / 64 + 1);
-  const uint32_t nthreads = gridDim.x * RES_THREADS, tid = blockIdx.x * RES_THREADS + threadIdx.x;
+  const size_t nthreads = (size_t)gridDim.x * RES_THREADS, tid = (size_t)blockIdx.x * RES_THREADS + threadIdx.x;
   const bool first_thread = tid == 0;
   T *a0 = (T *)p.a[0], *a1 = (T *)p.a[1];
   __shared__ ResStage s_stage;
@@ -294,10 +295,10 @@ __global__ void __launch_bounds__(RES_THREADS, RES_BLOCKS) relax_run(RelaxArgs p
   auto begin_step = [&]() { res_clear(p.slots + (step + 1) % 3); };
   st.calls = 0;
   if (p.init == 1) {
-    for (uint32_t i = tid; i < words; i += nthreads) p.bm[0][i] = p.bm[1][i] = 0u;
+    for (size_t i = tid; i < words; i += nthreads) p.bm[0][i] = p.bm[1][i] = 0u;
     if constexpr (Run::kWeighted) {
       const uint32_t start = p.rank_of ? p.rank_of[p.root] : p.root;
-      for (uint32_t v = tid; v < V; v += nthreads) a0[v] = a1[v] = v == start ? 0.0f : 1e9f;
+      for (size_t v = tid; v < V; v += nthreads) a0[v] = a1[v] = v == start ? 0.0f : 1e9f;
       st.ae = p.out.deg[start];
       st.n_act = 1;
       st.n = st.ae > RES_HUB ? 0 : 1;
@@ -305,7 +306,7 @@ __global__ void __launch_bounds__(RES_THREADS, RES_BLOCKS) relax_run(RelaxArgs p
       st.qvalid = 1;
       if (first_thread) p.q[0][st.n ? 0 : cap - 1] = start;
     } else {
-      for (uint32_t v = tid; v < V; v += nthreads) a0[v] = a1[v] = p.id_of ? p.id_of[v] : v;
+      for (size_t v = tid; v < V; v += nthreads) a0[v] = a1[v] = p.id_of ? p.id_of[v] : (uint32_t)v;
       st.ae = p.nadj;
       st.n_act = V;
       if (blockIdx.x == 0) least_source_block(p.plain_nz, words, V, p.word);
@@ -313,12 +314,9 @@ __global__ void __launch_bounds__(RES_THREADS, RES_BLOCKS) relax_run(RelaxArgs p
     grid.sync();
     if constexpr (!Run::kWeighted) pull.floor = res_read(p.word);
   } else if (p.init == 0) {
-    const T *from = (const T *)p.a[st.role];
-    T *to = (T *)p.a[st.role ^ 1];
-    for (uint32_t v = tid; v < V; v += nthreads) to[v] = from[v];
-    // the queue with its hubs apart
+    // the queue with its hubs apart (the host has copied R to W)
     begin_step();
-    for (uint32_t i = tid; i < st.n; i += nthreads) {
+    for (size_t i = tid; i < st.n; i += nthreads) {
       const uint32_t v = p.q[st.q][i];
       res_append(v, p.out.deg[v], p.q[st.q ^ 1], cap, slot());
     }
@@ -392,11 +390,11 @@ __global__ void __launch_bounds__(RES_THREADS, RES_BLOCKS) relax_run(RelaxArgs p
           best = o > best ? o : best;
         };
         if (st.qvalid) {
-          for (uint32_t i = tid; i < st.n + st.hubs; i += nthreads)
+          for (size_t i = tid; i < st.n + st.hubs; i += nthreads)
             take(i < st.n ? p.q[st.q][i] : p.q[st.q][cap - 1 - (i - st.n)]);
         } else {
-          for (uint32_t i = tid; i < words * 32; i += nthreads)
-            if ((p.bm[st.bm][i >> 5] >> (i & 31)) & 1u) take(i);
+          for (size_t i = tid; i < words * 32; i += nthreads)
+            if ((p.bm[st.bm][i >> 5] >> (i & 31)) & 1u) take((uint32_t)i);
         }
         best = __reduce_max_sync(GG_FULL, best);
         if (lane_id() == 0 && best) atomicMax(&slot()->c.aux, best);
@@ -420,7 +418,7 @@ __global__ void __launch_bounds__(RES_THREADS, RES_BLOCKS) relax_run(RelaxArgs p
         rows_walk<typename Run::Pull, true, true>(p.in, V, op, act, t, parts ? (T *)p.partials : nullptr, warp, nwarps);
         // the set this call was entered with has no reader any more; the next
         // pull sets its bits there
-        for (uint32_t i = tid; i < words; i += nthreads) p.bm[st.bm][i] = 0u;
+        for (size_t i = tid; i < words; i += nthreads) p.bm[st.bm][i] = 0u;
         if (parts) {
           grid.sync();
           big_finish<typename Run::Pull, 8, true>(p.in, op, (const T *)p.partials, act, t);
@@ -442,7 +440,7 @@ __global__ void __launch_bounds__(RES_THREADS, RES_BLOCKS) relax_run(RelaxArgs p
   if (st.n_act == 0) {
     const T *R = (const T *)p.a[st.role];
     T *out = (T *)p.result, *host = (T *)p.result_host;
-    for (uint32_t v = tid; v < V; v += nthreads) {
+    for (size_t v = tid; v < V; v += nthreads) {
       const T x = R[p.rank_of ? p.rank_of[v] : v];
       if (p.rank_of) out[v] = x;
       if (host) host[v] = x;
@@ -581,7 +579,13 @@ static int relax_loop(gg_graph *g, const Dir &dout, const Dir &din, const PullOp
       st.n = nq;
       st.qvalid = 1;
       st.q = (uint32_t)c_i;
+      GG_CUDA(cudaMemcpyAsync(nxt, cur, sizeof(T) * V, cudaMemcpyDeviceToDevice, s));
       GG_TRY((relax_launch<Run>(g, p, pull, &st, L, tr)));
+      // as many calls as fit one launch: the arrays and the queue are the kernel's still
+      while (st.n_act > 0 && st.calls == RES_CALLS) {
+        p.init = 2;
+        GG_TRY((relax_launch<Run>(g, p, pull, &st, L, tr)));
+      }
       ae = st.ae;
       n_act = st.n_act;
       nq = st.n;

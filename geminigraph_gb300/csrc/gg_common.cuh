@@ -66,8 +66,6 @@ struct Dir {
   float *w = nullptr;
   uint32_t *deg = nullptr;
   uint32_t *nz = nullptr;           // bitmap: deg > 0
-  uint32_t *med = nullptr;          // LIGHT_DEG < deg <= HEAVY_DEG, ascending
-  uint32_t nmed = 0;
   uint32_t *heavy = nullptr;        // deg > HEAVY_DEG, ascending
   uint32_t nheavy = 0;
   uint32_t *heavy_chunk = nullptr;  // nheavy+1: prefix of per-vertex chunk counts
@@ -79,7 +77,7 @@ struct Dir {
   uint32_t *big_owner = nullptr;    // nbigchunks: index into big of each chunk
   uint32_t nbigchunks = 0;
   uint32_t *bins_mem = nullptr;     // the allocations of the bins: big, big_chunk;
-  uint32_t *owner_mem = nullptr;    // the owners, med, heavy and heavy_chunk
+  uint32_t *owner_mem = nullptr;    // the owners, heavy and heavy_chunk
   size_t owner_words = 0;
   // Rows of a hot-source direction (see pull_rows): 32 consecutive vertices
   // make a slice whose light lists are stored column-major, four entries per
@@ -119,7 +117,7 @@ enum WsSlot {
   WS_PIPE,                              // second result buffer of the pipelined calls
   WS_QPOS,                              // per-word queue positions (queue_from_bitmap)
   WS_RES,                               // resident runs: tally slots and call rows
-  WS_SMALL,                             // SmallRun state and its trace rows
+  WS_SMALL,                             // small BFS pushes: state, tallies and call rows
   WS_MS_VISIT, WS_MS_FRONT, WS_MS_NEXT, // batched traversals: lane masks
   WS_MS_LVL, WS_MS_PAR, WS_MS_DIST,     // batched traversals: per-lane state (vertex-major)
   WS_MS_MISC, WS_MS_ROOTS,              // batched traversals: counters, roots

@@ -122,6 +122,13 @@ __device__ __forceinline__ uint32_t upper_bound_idx(const T *P, uint32_t lo, uin
   return lo;
 }
 
+// Ops whose result depends on which edge comes first (BFS's parents): their
+// tiles keep the timing they have, one thread's searches included.
+template <class Op, class = void>
+struct has_claims : std::false_type {};
+template <class Op>
+struct has_claims<Op, std::void_t<decltype(Op::kClaims)>> : std::true_type {};
+
 // The queue entry holding edge e0 of the prefix P and one past the entry
 // holding edge e1 - 1, by the block's first two warps (one thread's two
 // binary searches are 40 dependent loads for a queue of a million).
@@ -161,7 +168,15 @@ __global__ void __launch_bounds__(PUSH_THREADS)
   for (unsigned long long tile = blockIdx.x; tile < ntiles; tile += gridDim.x) {
     unsigned long long e0 = tile * PUSH_TILE;
     unsigned long long e1 = e0 + PUSH_TILE < total ? e0 + PUSH_TILE : total;
-    tile_bounds(P, n, e0, e1, &s_lo, &s_hi);
+    if constexpr (has_claims<Op>::value) {
+      if (threadIdx.x == 0) {
+        uint32_t lo = upper_bound_idx<unsigned long long>(P, 0, n + 1, e0) - 1;
+        s_lo = lo;
+        s_hi = upper_bound_idx<unsigned long long>(P, lo, n + 1, e1 - 1);  // one past the entry holding e1-1
+      }
+    } else {
+      tile_bounds(P, n, e0, e1, &s_lo, &s_hi);
+    }
     __syncthreads();
     const uint32_t lo = s_lo, hi = s_hi, cnt = hi - lo;
     const bool staged = cnt <= (uint32_t)PUSH_STAGE;
@@ -693,118 +708,117 @@ __global__ void __launch_bounds__(ROWS_THREADS, ROWS_BLOCKS)
 // that order: lanes scan their own list in order; a warp takes the lowest
 // lane of the first 32-wide chunk with a hit; heavy chunks record the index
 // of their first hit and the finish takes the lowest.
-static __global__ void __launch_bounds__(PULL_THREADS, 8)
-    bfs_pull_light(Dir d, uint32_t V, const uint32_t *__restrict__ active_in, uint32_t *parent, ActOut act,
-                   Counters *ctr) {
-  Tally t;
-  const size_t nwarps = (size_t)gridDim.x * (PULL_THREADS / 32);
+//
+// bfs_walk: a warp per 32 consecutive vertices (the word of the bitmaps it
+// owns).  What has to be read of a vertex is what bounds it (R-MAT 24: 511 MB
+// of offsets, degrees and first entries): vertices that are visited or have
+// no in-list cost two bits, the offsets of the others are read one group and
+// their bits two groups ahead, degrees only of vertices reached.  A list
+// without a hit in its first d.light entries goes on in the same warp, 32
+// entries at a time, up to HEAVY_DEG entries (a kernel of a warp per such list
+// took 237 us a call at R-MAT 26, nearly all of it finding visited vertices).
+// HEAVY lists are bfs_heavy_first's from the start.
+__device__ __forceinline__ void bfs_walk(const Dir &d, uint32_t V, const uint32_t *active_in, uint32_t *parent,
+                                         const ActOut &act, Tally &t, size_t warp, size_t nwarps) {
   const size_t groups = ((size_t)V + 31) / 32;
   const unsigned lane = lane_id();
-  // Software-pipelined over the warp's groups: the visited word, offsets and
-  // out-degree of group g + nwarps are loaded before group g is scanned.
-  size_t g = (size_t)blockIdx.x * (PULL_THREADS / 32) + (threadIdx.x >> 5);
-  uint32_t vis = 0, od = 0;
-  unsigned long long b = 0, e = 0;
-  bool todo = false;
-  if (g < groups) {
-    uint32_t v = (uint32_t)(g * 32 + lane);
-    vis = act.visited[g];
-    todo = v < V && !((vis >> lane) & 1u);
-    if (todo) {
-      b = d.off[v];
-      e = d.off[v + 1];
-      od = act.out_deg[v];
+  auto words = [&](size_t g, uint32_t &vis, uint32_t &todo) {
+    vis = todo = 0;
+    if (g < groups) {
+      vis = act.visited[g];
+      todo = d.nz[g] & ~vis;
     }
-  }
-  while (g < groups) {
-    const size_t gn = g + nwarps;
-    uint32_t visn = 0, odn = 0;
-    unsigned long long bn = 0, en = 0;
-    bool todon = false;
-    if (gn < groups) {
-      uint32_t vn = (uint32_t)(gn * 32 + lane);
-      visn = act.visited[gn];
-      todon = vn < V && !((visn >> lane) & 1u);
-      if (todon) {
-        bn = d.off[vn];
-        en = d.off[vn + 1];
-        odn = act.out_deg[vn];
+  };
+  auto bounds = [&](size_t g, uint32_t todo, unsigned long long &b, unsigned long long &e) {
+    b = e = 0;
+    if ((todo >> lane) & 1u) {
+      b = d.off[g * 32 + lane];
+      e = d.off[g * 32 + lane + 1];
+    }
+  };
+  uint32_t vis, todo, vis1, todo1;
+  unsigned long long b, e;
+  words(warp, vis, todo);
+  words(warp + nwarps, vis1, todo1);
+  bounds(warp, todo, b, e);
+  for (size_t g = warp; g < groups; g += nwarps) {
+    uint32_t vis2, todo2;
+    unsigned long long b1, e1;
+    words(g + 2 * nwarps, vis2, todo2);
+    bounds(g + nwarps, todo1, b1, e1);
+    if (todo) {  // uniform
+      uint32_t found = NONE32;
+      const unsigned long long n = e - b;
+      const bool heavy = n > HEAVY_DEG;
+      const unsigned long long lim = heavy ? b : n <= d.light ? e : b + d.light;
+      constexpr int STEP = 4;
+      for (unsigned long long k = b; k < lim && found == NONE32; k += STEP) {
+        uint32_t u[STEP];
+#pragma unroll
+        for (int j = 0; j < STEP; j++) u[j] = k + j < lim ? nbr_at(d, k + j, GG_SITE) : NONE32;
+        unsigned hits = 0;
+#pragma unroll
+        for (int j = 0; j < STEP; j++) hits |= (u[j] != NONE32 && bm_test(active_in, u[j])) ? 1u << j : 0u;
+#pragma unroll
+        for (int j = STEP - 1; j >= 0; j--)
+          if ((hits >> j) & 1u) found = u[j];
+      }
+      for (unsigned rest = __ballot_sync(GG_FULL, found == NONE32 && n > d.light && !heavy); rest; rest &= rest - 1) {
+        const int j = __ffs(rest) - 1;
+        const unsigned long long ej = __shfl_sync(GG_FULL, e, j);
+        uint32_t hit = NONE32;
+        for (unsigned long long base = __shfl_sync(GG_FULL, lim, j); base < ej && hit == NONE32; base += 64) {
+          const unsigned long long k = base + lane;
+          uint32_t s0 = 0, s1 = 0;
+          bool h0 = false, h1 = false;
+          if (k < ej) s0 = nbr_at(d, k, GG_SITE);
+          if (k + 32 < ej) s1 = nbr_at(d, k + 32, GG_SITE);
+          if (k < ej) h0 = bm_test(active_in, s0);
+          if (k + 32 < ej) h1 = bm_test(active_in, s1);
+          const unsigned m0 = __ballot_sync(GG_FULL, h0), m1 = __ballot_sync(GG_FULL, h1);
+          if (m0)
+            hit = __shfl_sync(GG_FULL, s0, __ffs(m0) - 1);
+          else if (m1)
+            hit = __shfl_sync(GG_FULL, s1, __ffs(m1) - 1);
+        }
+        if ((int)lane == j) found = hit;
+      }
+      const bool a = found != NONE32;
+      const unsigned bits = __ballot_sync(GG_FULL, a);
+      if (lane == 0 && bits) {
+        act.active_out[g] = bits;
+        act.visited[g] = vis | bits;
+      }
+      if (a) {
+        const uint32_t v = (uint32_t)(g * 32 + lane), od = act.out_deg[v];
+        parent[v] = found;
+        t.activated += 1;
+        t.edges += od;
+        t.maxdeg = od > t.maxdeg ? od : t.maxdeg;
       }
     }
-    // the first LIGHT_DEG entries of every list, four independent loads at a
-    // time; longer lists without a hit there go on in the medium / heavy kernels
-    const uint32_t v = (uint32_t)(g * 32 + lane);
-    uint32_t found = NONE32;
-    if (todo) {
-      unsigned long long lim = e - b <= d.light ? e : b + d.light;
-      for (unsigned long long k = b; k < lim && found == NONE32; k += 4) {
-        uint32_t s0 = nbr_at(d, k, GG_SITE);
-        uint32_t s1 = k + 1 < lim ? nbr_at(d, k + 1, GG_SITE) : s0;
-        uint32_t s2 = k + 2 < lim ? nbr_at(d, k + 2, GG_SITE) : s0;
-        uint32_t s3 = k + 3 < lim ? nbr_at(d, k + 3, GG_SITE) : s0;
-        bool h0 = bm_test_ldg(active_in, s0), h1 = bm_test_ldg(active_in, s1);
-        bool h2 = bm_test_ldg(active_in, s2), h3 = bm_test_ldg(active_in, s3);
-        found = h0 ? s0 : h1 ? s1 : h2 ? s2 : h3 ? s3 : NONE32;
-      }
-    }
-    const bool a = found != NONE32;
-    if (a) parent[v] = found;
-    const unsigned bits = __ballot_sync(GG_FULL, a);
-    if (lane == 0 && bits) {
-      act.active_out[g] = bits;
-      act.visited[g] = vis | bits;
-    }
-    if (a) {
-      t.activated += 1;
-      t.edges += od;
-      t.maxdeg = od > t.maxdeg ? od : t.maxdeg;
-    }
-    g = gn;
-    vis = visn;
-    todo = todon;
-    b = bn;
-    e = en;
-    od = odn;
+    vis = vis1;
+    todo = todo1;
+    vis1 = vis2;
+    todo1 = todo2;
+    b = b1;
+    e = e1;
   }
-  t.flush(ctr);
 }
-
-static __global__ void __launch_bounds__(PULL_THREADS)
-    bfs_pull_medium(Dir d, const uint32_t *__restrict__ active_in, uint32_t *parent, ActOut act, Counters *ctr) {
+// Six blocks of 256 threads per SM (R-MAT 26: 2.35 ms a BFS; eight, with
+// spills, 3.25) and four entries a step (eight: 2.60).
+constexpr int BFS_BLOCKS = 6;
+static __global__ void __launch_bounds__(PULL_THREADS, BFS_BLOCKS)
+    bfs_pull_walk(Dir d, uint32_t V, const uint32_t *active_in, uint32_t *parent, ActOut act, Counters *ctr) {
   Tally t;
-  size_t nwarps = (size_t)gridDim.x * (PULL_THREADS / 32);
-  unsigned lane = lane_id();
-  for (size_t i = (size_t)blockIdx.x * (PULL_THREADS / 32) + (threadIdx.x >> 5); i < d.nmed; i += nwarps) {
-    uint32_t v = d.med[i];
-    uint32_t found = NONE32;
-    if (!bm_test(act.visited, v)) {
-      unsigned long long b = d.off[v] + d.light, e = d.off[v + 1];
-      for (unsigned long long base = b; base < e; base += 32) {
-        unsigned long long k = base + lane;
-        uint32_t s = 0;
-        bool hit = false;
-        if (k < e) {
-          s = nbr_at(d, k, GG_SITE);
-          hit = bm_test_ldg(active_in, s);
-        }
-        unsigned m = __ballot_sync(GG_FULL, hit);
-        if (m) {
-          found = __shfl_sync(GG_FULL, s, __ffs(m) - 1);
-          break;
-        }
-      }
-    }
-    bool a = lane == 0 && found != NONE32;
-    if (a) parent[v] = found;
-    push_activate(a, v, act, t);
-  }
+  bfs_walk(d, V, active_in, parent, act, t, (size_t)blockIdx.x * (PULL_THREADS / 32) + (threadIdx.x >> 5),
+           (size_t)gridDim.x * (PULL_THREADS / 32));
   t.flush(ctr);
 }
 
 // partials[c] = edge index of the chunk's first active in-neighbour, or ~0.
-static __global__ void __launch_bounds__(PULL_THREADS)
-    bfs_heavy_first(Dir d, const uint32_t *__restrict__ active_in, const uint32_t *__restrict__ visited,
-                    unsigned long long *first) {
+__device__ __forceinline__ void bfs_heavy_walk(const Dir &d, const uint32_t *active_in, const uint32_t *visited,
+                                               unsigned long long *first) {
   // one warp per HEAVY_CHUNK-entry chunk of a list longer than HEAVY_DEG;
   // first[h] = the lowest hit index of heavy vertex h, so a chunk starting
   // past it (or a vertex already visited) is skipped and a scan stops at it
@@ -822,7 +836,7 @@ static __global__ void __launch_bounds__(PULL_THREADS)
       if (lane == 0) best = *(volatile unsigned long long *)(first + h);
       if (__shfl_sync(GG_FULL, best, 0) < base) break;
       const unsigned long long k = base + lane;
-      const bool hit = k < e && bm_test_ldg(active_in, nbr_at(d, k, GG_SITE));
+      const bool hit = k < e && bm_test(active_in, nbr_at(d, k, GG_SITE));
       const unsigned bal = __ballot_sync(GG_FULL, hit);
       if (bal) {
         if (lane == 0) atomicMin(first + h, base + (unsigned long long)(__ffs(bal) - 1));
@@ -833,9 +847,13 @@ static __global__ void __launch_bounds__(PULL_THREADS)
 }
 
 static __global__ void __launch_bounds__(PULL_THREADS)
-    bfs_heavy_finish(Dir d, const unsigned long long *__restrict__ first, uint32_t *parent, ActOut act,
-                     Counters *ctr) {
-  Tally t;
+    bfs_heavy_first(Dir d, const uint32_t *active_in, const uint32_t *visited, unsigned long long *first) {
+  bfs_heavy_walk(d, active_in, visited, first);
+}
+
+// The heavy vertices' parents; first[] is left as it is needed by the next call.
+__device__ __forceinline__ void bfs_heavy_take(const Dir &d, unsigned long long *first, uint32_t *parent,
+                                               const ActOut &act, Tally &t) {
   const size_t n = ((size_t)d.nheavy + 31) / 32 * 32;
   for (size_t h = (size_t)blockIdx.x * blockDim.x + threadIdx.x; h < n; h += (size_t)gridDim.x * blockDim.x) {
     bool a = false;
@@ -843,294 +861,22 @@ static __global__ void __launch_bounds__(PULL_THREADS)
     if (h < d.nheavy) {
       v = d.heavy[h];
       const unsigned long long f = first[h];
-      if (f != ~0ull && !bm_test(act.visited, v)) {
-        parent[v] = nbr_at(d, f, GG_SITE);
-        a = true;
+      if (f != ~0ull) {
+        first[h] = ~0ull;
+        if (!bm_test(act.visited, v)) {
+          parent[v] = nbr_at(d, f, GG_SITE);
+          a = true;
+        }
       }
     }
     push_activate(a, v, act, t);
   }
+}
+static __global__ void __launch_bounds__(PULL_THREADS)
+    bfs_heavy_finish(Dir d, unsigned long long *first, uint32_t *parent, ActOut act, Counters *ctr) {
+  Tally t;
+  bfs_heavy_take(d, first, parent, act, t);
   t.flush(ctr);
-}
-
-// ---------------------------------------------------------------- small sparse runs
-// A run of consecutive sparse calls whose frontiers are small (high-diameter
-// graphs such as grids, and the tails of power-law BFS) is driven from the
-// device: each call is one push_small launch (plus a snapshot gather for CC
-// and SSSP) that reads its queue length and active_edges from SmallRun; the
-// last block to finish (a ticket counter, no waiting) writes the call's trace
-// row, moves the accumulated counters to the next call, and decides whether
-// the next call may also run here -- the same switch (sparse iff active_edges
-// < edges/20) plus size limits.  The host enqueues a batch of launches without
-// synchronising; launches after the run stops return at once.
-constexpr int SMALL_THREADS = 256;
-constexpr uint32_t SMALL_BATCH = 512;        // calls enqueued per host round trip
-constexpr uint32_t SMALL_MAX_QUEUE = 65536;  // largest queue a small call takes
-constexpr unsigned long long SMALL_MAX_AE = 1ull << 20;
-constexpr uint32_t SMALL_MAX_DEG = 1024;     // largest out-degree in a small call's queue
-constexpr int COOP_BLOCKS = 32;              // blocks of a cooperative small run (all resident)
-
-struct SmallRun {
-  unsigned long long ae;         // active_edges of the call about to run
-  unsigned long long edges_lim;  // edges / 20
-  unsigned long long total_ae;   // sum of active_edges over the run's calls
-  unsigned int n;                // its queue length
-  unsigned int go;               // the next launch runs a call
-  unsigned int calls;            // trace rows written in this batch
-  unsigned int level;            // activation stamp of the current call (> 0)
-  unsigned int ticket;           // blocks finished in the current call
-  unsigned int last_activated;   // activated count of the last call
-  unsigned int maxdeg;           // largest out-degree in the queue of the call about to run
-  Counters next;                 // accumulators of the current call
-};
-
-// Queue append from divergent lanes: one atomic per group of lanes that
-// reach this point together.
-__device__ __forceinline__ void queue_append_any(uint32_t v, uint32_t *q, unsigned *qlen) {
-  const unsigned am = __activemask();
-  const int leader = __ffs(am) - 1;
-  const unsigned lane = lane_id();
-  unsigned base = 0;
-  if ((int)lane == leader) base = atomicAdd(qlen, (unsigned)__popc(am));
-  base = __shfl_sync(am, base, leader);
-  q[base + __popc(am & ((1u << lane) - 1u))] = v;
-}
-
-// Activation inside a small push call: stamp-deduplicated unless the op's
-// slot already lets one thread win (BFS's CAS).  Lanes may be divergent.
-template <bool kUnique>
-__device__ __forceinline__ void small_activate(uint32_t v, SmallRun *st, uint32_t *stamp, unsigned level,
-                                               uint32_t *visited, uint32_t *q_out, const uint32_t *out_deg,
-                                               const uint32_t *in_deg, Tally &t) {
-  if (!kUnique) {
-    if (stamp[v] == level || atomicExch(stamp + v, level) == level) return;
-  }
-  if (visited) atomicOr(visited + (v >> 5), 1u << (v & 31));
-  uint32_t od = out_deg[v];
-  t.activated += 1;
-  t.edges += od;
-  t.maxdeg = od > t.maxdeg ? od : t.maxdeg;
-  if (in_deg) t.in_edges += in_deg[v];
-  if (od > 0) queue_append_any(v, q_out, &st->next.qlen);
-}
-
-// One small push call over q_in (n entries): slots, activation, and the
-// call's tally flushed into st->next.  Every thread of the block calls it.
-template <class Op, bool kUnique>
-__device__ __forceinline__ void small_call(SmallRun *st, const uint32_t *__restrict__ q_in, uint32_t *__restrict__ q_out,
-                                           const Dir &d, const Op &op, uint32_t *stamp, uint32_t *visited,
-                                           const uint32_t *__restrict__ out_deg, const uint32_t *__restrict__ in_deg,
-                                           uint32_t n, unsigned level) {
-  const unsigned lane = lane_id();
-  Tally t;
-  const size_t nround = ((size_t)n + 31) / 32 * 32;
-  for (size_t i = (size_t)blockIdx.x * SMALL_THREADS + threadIdx.x; i < nround; i += (size_t)gridDim.x * SMALL_THREADS) {
-    const bool valid = i < n;
-    uint32_t src = 0;
-    unsigned long long b = 0, e = 0;
-    if (valid) {
-      src = q_in[i];
-      b = d.off[src];
-      e = d.off[src + 1];
-    }
-    if (valid && e - b <= LIGHT_DEG) {
-      for (unsigned long long k = b; k < e; k++) {
-        uint32_t dst = nbr_at(d, k, GG_SITE);
-        if (op.push(src, (uint32_t)i, dst, d.w ? d.w[k] : 0.0f))
-          small_activate<kUnique>(dst, st, stamp, level, visited, q_out, out_deg, in_deg, t);
-      }
-    }
-    unsigned coop = __ballot_sync(GG_FULL, valid && e - b > LIGHT_DEG);
-    while (coop) {
-      const unsigned leader = __ffs(coop) - 1;
-      coop &= coop - 1;
-      const unsigned long long lb = __shfl_sync(GG_FULL, b, leader), le = __shfl_sync(GG_FULL, e, leader);
-      const uint32_t lsrc = __shfl_sync(GG_FULL, src, leader);
-      const uint32_t li = (uint32_t)__shfl_sync(GG_FULL, (unsigned long long)i, leader);
-      for (unsigned long long k = lb + lane; k < le; k += 32) {
-        uint32_t dst = nbr_at(d, k, GG_SITE);
-        if (op.push(lsrc, li, dst, d.w ? d.w[k] : 0.0f))
-          small_activate<kUnique>(dst, st, stamp, level, visited, q_out, out_deg, in_deg, t);
-      }
-    }
-  }
-  t.flush(&st->next);
-}
-
-// small_call with the tally and the queue counter in `tally` (the
-// cooperative path keeps three of them).
-template <bool kUnique>
-__device__ __forceinline__ void small_activate_t(uint32_t v, Counters *tally, uint32_t *stamp, unsigned level,
-                                                 uint32_t *visited, uint32_t *q_out, const uint32_t *out_deg,
-                                                 const uint32_t *in_deg, Tally &t) {
-  if (!kUnique) {
-    if (stamp[v] == level || atomicExch(stamp + v, level) == level) return;
-  }
-  if (visited) atomicOr(visited + (v >> 5), 1u << (v & 31));
-  uint32_t od = out_deg[v];
-  t.activated += 1;
-  t.edges += od;
-  t.maxdeg = od > t.maxdeg ? od : t.maxdeg;
-  if (in_deg) t.in_edges += in_deg[v];
-  if (od > 0) queue_append_any(v, q_out, &tally->qlen);
-}
-template <class Op, bool kUnique>
-__device__ __forceinline__ void small_call_t(Counters *tally, const uint32_t *__restrict__ q_in,
-                                             uint32_t *__restrict__ q_out, const Dir &d, const Op &op,
-                                             uint32_t *stamp, uint32_t *visited,
-                                             const uint32_t *__restrict__ out_deg,
-                                             const uint32_t *__restrict__ in_deg, uint32_t n, unsigned level) {
-  const unsigned lane = lane_id();
-  Tally t;
-  const size_t nround = ((size_t)n + 31) / 32 * 32;
-  for (size_t i = (size_t)blockIdx.x * SMALL_THREADS + threadIdx.x; i < nround; i += (size_t)gridDim.x * SMALL_THREADS) {
-    const bool valid = i < n;
-    uint32_t src = 0;
-    unsigned long long b = 0, e = 0;
-    if (valid) {
-      src = q_in[i];
-      b = d.off[src];
-      e = d.off[src + 1];
-    }
-    if (valid && e - b <= LIGHT_DEG) {
-      for (unsigned long long k = b; k < e; k++) {
-        uint32_t dst = nbr_at(d, k, GG_SITE);
-        if (op.push(src, (uint32_t)i, dst, d.w ? d.w[k] : 0.0f))
-          small_activate_t<kUnique>(dst, tally, stamp, level, visited, q_out, out_deg, in_deg, t);
-      }
-    }
-    unsigned coop = __ballot_sync(GG_FULL, valid && e - b > LIGHT_DEG);
-    while (coop) {
-      const unsigned leader = __ffs(coop) - 1;
-      coop &= coop - 1;
-      const unsigned long long lb = __shfl_sync(GG_FULL, b, leader), le = __shfl_sync(GG_FULL, e, leader);
-      const uint32_t lsrc = __shfl_sync(GG_FULL, src, leader);
-      const uint32_t li = (uint32_t)__shfl_sync(GG_FULL, (unsigned long long)i, leader);
-      for (unsigned long long k = lb + lane; k < le; k += 32) {
-        uint32_t dst = nbr_at(d, k, GG_SITE);
-        if (op.push(lsrc, li, dst, d.w ? d.w[k] : 0.0f))
-          small_activate_t<kUnique>(dst, tally, stamp, level, visited, q_out, out_deg, in_deg, t);
-      }
-    }
-  }
-  t.flush(tally);
-}
-
-// Closes a small call (one thread, after every block's tally is in): the
-// trace row, the next call's queue and switch value, and whether it runs.
-__device__ __forceinline__ void small_close(SmallRun *st, unsigned long long *tr_ae, unsigned int *tr_act,
-                                            unsigned level) {
-  const unsigned long long ne = atomicAdd(&st->next.edges, 0ull);
-  const unsigned int na = atomicAdd(&st->next.activated, 0u);
-  const unsigned int nq = atomicAdd(&st->next.qlen, 0u);
-  const unsigned int nm = atomicAdd(&st->next.maxdeg, 0u);
-  const unsigned int r = st->calls;
-  tr_ae[r] = st->ae;
-  tr_act[r] = na;
-  st->calls = r + 1;
-  st->total_ae += st->ae;
-  st->level = level + 1;
-  st->ae = ne;
-  st->n = nq;
-  st->last_activated = na;
-  st->next.edges = 0;
-  st->next.in_edges = 0;
-  st->next.activated = 0;
-  st->next.qlen = 0;
-  st->next.maxdeg = 0;
-  st->ticket = 0;
-  st->maxdeg = nm;
-  st->go = (na > 0 && ne < st->edges_lim && nq <= SMALL_MAX_QUEUE && ne <= SMALL_MAX_AE && nm <= SMALL_MAX_DEG)
-               ? 1u
-               : 0u;
-  __threadfence();
-}
-
-template <class Op, bool kUnique>
-__global__ void __launch_bounds__(SMALL_THREADS)
-    push_small(SmallRun *st, const uint32_t *__restrict__ q_in, uint32_t *__restrict__ q_out, Dir d, Op op,
-               uint32_t *stamp, uint32_t *visited, const uint32_t *__restrict__ out_deg,
-               const uint32_t *__restrict__ in_deg, unsigned long long *tr_ae, unsigned int *tr_act) {
-  __shared__ unsigned s_go, s_n, s_level, s_last;
-  if (threadIdx.x == 0) {
-    s_go = st->go;
-    s_n = st->n;
-    s_level = st->level;
-  }
-  __syncthreads();
-  if (!s_go) return;
-  small_call<Op, kUnique>(st, q_in, q_out, d, op, stamp, visited, out_deg, in_deg, s_n, s_level);
-  __syncthreads();
-  if (threadIdx.x == 0) {
-    __threadfence();
-    s_last = atomicAdd(&st->ticket, 1u) == gridDim.x - 1;
-  }
-  __syncthreads();
-  if (s_last && threadIdx.x == 0) {
-    __threadfence();
-    small_close(st, tr_ae, tr_act, s_level);
-  }
-}
-
-// The same calls in one cooperative launch: up to max_calls of them, the
-// queues alternating (qa -> qb, then qb -> qa, ...), one grid-wide barrier
-// per call.  Call c's tally goes to tally[c % 3]; after the barrier every
-// block reads it and derives the next call's queue length, switch value and
-// whether it runs (identical in all blocks, so all leave the loop together);
-// block 0 writes the trace row and clears tally[(c + 1) % 3], which no block
-// reads any more (the last reads were before the previous barrier).
-template <class Op, bool kUnique>
-__global__ void __launch_bounds__(SMALL_THREADS)
-    push_small_coop(SmallRun *st, Counters *tally, uint32_t *qa, uint32_t *qb, Dir d, Op op, uint32_t *stamp,
-                    uint32_t *visited, const uint32_t *__restrict__ out_deg, const uint32_t *__restrict__ in_deg,
-                    unsigned long long *tr_ae, unsigned int *tr_act, unsigned max_calls) {
-  cooperative_groups::grid_group grid = cooperative_groups::this_grid();
-  unsigned n = st->n, level = st->level, go = st->go, maxdeg = st->maxdeg, na = 0;
-  unsigned long long ae = st->ae, total = st->total_ae;
-  const unsigned long long lim = st->edges_lim;
-  unsigned c = 0;
-  for (; c < max_calls && go; c++) {
-    Counters *cur = tally + (c % 3);
-    if (blockIdx.x == 0 && threadIdx.x == 0) memset(tally + ((c + 1) % 3), 0, sizeof(Counters));
-    small_call_t<Op, kUnique>(cur, (c & 1) ? qb : qa, (c & 1) ? qa : qb, d, op, stamp, visited, out_deg, in_deg, n,
-                              level);
-    grid.sync();
-    const unsigned long long ne = *(volatile unsigned long long *)&cur->edges;
-    na = *(volatile unsigned *)&cur->activated;
-    const unsigned nq = *(volatile unsigned *)&cur->qlen;
-    const unsigned nm = *(volatile unsigned *)&cur->maxdeg;
-    if (blockIdx.x == 0 && threadIdx.x == 0) {
-      tr_ae[c] = ae;
-      tr_act[c] = na;
-    }
-    total += ae;
-    level += 1;
-    ae = ne;
-    n = nq;
-    maxdeg = nm;
-    go = (na > 0 && ne < lim && nq <= SMALL_MAX_QUEUE && ne <= SMALL_MAX_AE && nm <= SMALL_MAX_DEG) ? 1u : 0u;
-  }
-  if (blockIdx.x == 0 && threadIdx.x == 0) {
-    st->calls = c;
-    st->total_ae = total;
-    st->level = level;
-    st->ae = ae;
-    st->n = n;
-    st->last_activated = na;
-    st->maxdeg = maxdeg;
-    st->go = go;
-    __threadfence();
-  }
-}
-
-// Snapshot gather of a small call (CC, SSSP): msg[i] = src[q[i]].
-template <typename T>
-__global__ void small_gather(const SmallRun *st, const uint32_t *__restrict__ q, const T *__restrict__ src,
-                             T *__restrict__ msg) {
-  if (!st->go) return;
-  const uint32_t n = st->n;
-  for (size_t i = (size_t)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += (size_t)gridDim.x * blockDim.x)
-    msg[i] = src[q[i]];
 }
 
 // ---------------------------------------------------------------- queue from bitmap
@@ -1220,9 +966,6 @@ struct Launch {
     unsigned long long cap = (unsigned long long)g->num_sms * 8;
     return (unsigned)(tiles < 1 ? 1 : (tiles > cap ? cap : tiles));
   }
-  unsigned med_grid(const Dir &d) const {
-    return grid_for((size_t)d.nmed * 32, PULL_THREADS, g->num_sms, 8);
-  }
   unsigned heavy_grid(const Dir &d) const {
     return grid_for((size_t)d.nchunks * 32, PULL_THREADS, g->num_sms, 8);
   }
@@ -1308,12 +1051,9 @@ struct Launch {
   }
   int bfs_pull(const Dir &d, const uint32_t *active_in, uint32_t *parent, const ActOut &act, Counters *ctr) {
     cudaStream_t s = g->stream;
-    bfs_pull_light<<<pull_grid(), PULL_THREADS, 0, s>>>(d, g->V, active_in, parent, act, ctr);
+    bfs_pull_walk<<<grid_for(((size_t)g->V + 31) / 32 * 32, PULL_THREADS, g->num_sms, BFS_BLOCKS), PULL_THREADS, 0, s>>>(
+        d, g->V, active_in, parent, act, ctr);
     launches += 1;
-    if (d.nmed) {
-      bfs_pull_medium<<<med_grid(d), PULL_THREADS, 0, s>>>(d, active_in, parent, act, ctr);
-      launches += 1;
-    }
     if (d.nheavy) {
       unsigned long long *first = nullptr;
       GG_TRY(ws(g, WS_PARTIAL, d.nheavy, &first));
@@ -1340,133 +1080,11 @@ struct Launch {
     GG_CUDA(cudaGetLastError());
     return read_small(g, n, pos + words, sizeof(uint32_t));
   }
-  // Runs consecutive small sparse calls on the device (see SmallRun).  On
-  // entry q[*cur] holds the active vertices with out-degree > 0 (nq of them)
-  // and ae is the call's active_edges.  On return *cur, *nq, *ae describe the
-  // first call that did not run here and *n_act is the previous call's
-  // activated count; the trace has one row per call that ran.
-  template <class Op, bool kUnique, typename T>
-  int small_run(const Dir &d, const Op &op, uint32_t *q[2], int *cur, uint32_t *nq, unsigned long long *ae,
-                uint32_t *maxdeg, uint32_t *n_act, uint32_t *visited, const uint32_t *in_deg, const T *snap_src, T *snap_msg,
-                Trace &tr, uint32_t *stamp) {
-    SmallRun *st;
-    unsigned long long *tr_ae;
-    unsigned *tr_act;
-    char *blob;
-    const size_t st_bytes = 256, ae_bytes = sizeof(unsigned long long) * SMALL_BATCH;
-    const size_t act_bytes = sizeof(unsigned) * SMALL_BATCH;
-    GG_TRY(ws(g, WS_SMALL, st_bytes + ae_bytes + act_bytes + 3 * sizeof(Counters) + 64, &blob));
-    Counters *coop_tally = (Counters *)(blob + ((st_bytes + ae_bytes + act_bytes + 63) / 64 * 64));
-    st = (SmallRun *)blob;
-    tr_ae = (unsigned long long *)(blob + st_bytes);
-    tr_act = (unsigned *)(blob + st_bytes + ae_bytes);
-    static thread_local std::vector<unsigned long long> h_ae;
-    static thread_local std::vector<unsigned> h_act;
-    h_ae.resize(SMALL_BATCH);
-    h_act.resize(SMALL_BATCH);
-    SmallRun h;
-    memset(&h, 0, sizeof(h));
-    h.ae = *ae;
-    h.edges_lim = g->E / 20;
-    h.n = *nq;
-    h.go = 1;
-    h.maxdeg = *maxdeg;
-    h.level = next_level();
-    cudaStream_t s = g->stream;
-    const unsigned grid = grid_for(SMALL_MAX_QUEUE, SMALL_THREADS, g->num_sms, 1);
-    // batches of 2, 4, 8, ... launches: a short run wastes few no-op launches;
-    // full batches of a long run replay one captured CUDA graph
-    auto enqueue = [&](uint32_t n) {
-      for (uint32_t i = 0; i < n; i++) {
-        const int c = *cur ^ (int)(i & 1);
-        if (snap_msg) small_gather<T><<<grid, SMALL_THREADS, 0, s>>>(st, q[c], snap_src, snap_msg);
-        push_small<Op, kUnique><<<grid, SMALL_THREADS, 0, s>>>(st, q[c], q[c ^ 1], d, op, stamp, visited,
-                                                                d.deg, in_deg, tr_ae, tr_act);
-      }
-    };
-    cudaGraphExec_t exec = nullptr;
-    int exec_parity = -1;
-    int status = GG_OK;
-    // Without message snapshots the calls need no host step between them: one
-    // cooperative launch runs a whole batch (grid = one block per SM, all
-    // resident by the cooperative launch's guarantee) and stops early.
-    const bool coop = !snap_msg && coop_ok();
-    uint32_t batch = coop ? SMALL_BATCH : 2;
-    for (;;) {
-      cudaError_t e = cudaMemcpyAsync(st, &h, sizeof(h), cudaMemcpyHostToDevice, s);
-      if (e == cudaSuccess && coop) {
-        uint32_t *qa = q[*cur], *qb = q[*cur ^ 1];
-        Dir dd = d;
-        Op oo = op;
-        const uint32_t *deg = d.deg;
-        unsigned mc = batch;
-        Counters *tally = coop_tally;
-        e = cudaMemsetAsync(tally, 0, sizeof(Counters), s);
-        void *args[] = {&st, &tally, &qa, &qb, &dd, &oo, &stamp, &visited, (void *)&deg, (void *)&in_deg,
-                        &tr_ae, &tr_act, &mc};
-        if (e == cudaSuccess)
-          e = cudaLaunchCooperativeKernel((const void *)push_small_coop<Op, kUnique>, dim3(COOP_BLOCKS),
-                                          dim3(SMALL_THREADS), args, 0, s);
-        launches += 1;
-      } else if (e == cudaSuccess && batch == SMALL_BATCH) {
-        if (!exec || exec_parity != *cur) {
-          if (exec) cudaGraphExecDestroy(exec);
-          exec = nullptr;
-          cudaGraph_t graph = nullptr;
-          e = cudaStreamBeginCapture(s, cudaStreamCaptureModeThreadLocal);
-          if (e == cudaSuccess) {
-            enqueue(batch);
-            e = cudaStreamEndCapture(s, &graph);
-          }
-          if (e == cudaSuccess) e = cudaGraphInstantiate(&exec, graph, 0);
-          if (graph) cudaGraphDestroy(graph);
-          exec_parity = *cur;
-        }
-        if (e == cudaSuccess) e = cudaGraphLaunch(exec, s);
-      } else if (e == cudaSuccess) {
-        enqueue(batch);
-      }
-      if (e == cudaSuccess) e = cudaGetLastError();
-      if (e != cudaSuccess) {
-        status = cuda_status(e, "small run");
-        break;
-      }
-      if (!coop) launches += batch * (snap_msg ? 2 : 1);
-      status = read_small(g, &h, st, sizeof(h));
-      if (status == GG_OK) status = read_small(g, h_ae.data(), tr_ae, sizeof(unsigned long long) * batch);
-      if (status == GG_OK) status = read_small(g, h_act.data(), tr_act, sizeof(unsigned) * batch);
-      if (status != GG_OK) break;
-      for (uint32_t r = 0; r < h.calls; r++) {
-        tr.add(0, h_ae[r], h_act[r]);
-        *n_act = h_act[r];
-      }
-      *cur ^= (int)(h.calls & 1);
-      level_ = h.level;
-      if (h.go) {  // the batch ended with the run still going
-        h.calls = 0;
-        batch = batch * 2 < SMALL_BATCH ? batch * 2 : SMALL_BATCH;
-        continue;
-      }
-      break;
-    }
-    if (exec) cudaGraphExecDestroy(exec);
-    if (status != GG_OK) return status;
-    *nq = h.n;
-    *ae = h.ae;
-    *maxdeg = h.maxdeg;
-    return GG_OK;
-  }
   // Cooperative launches available (queried once per device).
   bool coop_ok() const {
     int v = 0;
     return cudaDeviceGetAttribute(&v, cudaDevAttrCooperativeLaunch, g->device) == cudaSuccess && v;
   }
-  static bool small_ok(uint32_t nq, unsigned long long ae, uint32_t maxdeg) {
-    return ae > 0 && nq <= SMALL_MAX_QUEUE && ae <= SMALL_MAX_AE && maxdeg <= SMALL_MAX_DEG;
-  }
-  // Activation stamps grow across small runs of one graph; 0 marks "never".
-  unsigned level_ = 0;
-  unsigned next_level() { return level_ + 1; }
   int scan_queue_degrees(const uint32_t *q, uint32_t n, const uint32_t *deg, unsigned long long **P) {
     unsigned long long *p = nullptr, *scratch = nullptr;
     GG_TRY(ws(g, WS_PREFIX, (size_t)g->V + 2, &p));

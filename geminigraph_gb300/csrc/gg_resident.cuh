@@ -70,7 +70,7 @@ __device__ __forceinline__ uint32_t res_place(uint32_t od, unsigned long long *c
   return (uint32_t)__shfl_sync(am, (uint32_t)base, leader) + __popc(am & ((1u << lane) - 1u));
 }
 // Hubs from the back, q[cap - 1 - i].  Lanes may be divergent.
-__device__ __forceinline__ void res_append(uint32_t v, uint32_t od, uint32_t *q, uint32_t cap, ResTally *slot) {
+__device__ __forceinline__ void res_append(uint32_t v, uint32_t od, uint32_t *q, size_t cap, ResTally *slot) {
   if (od > RES_HUB)
     q[cap - 1 - res_place(od, &slot->happ)] = v;
   else
@@ -86,7 +86,7 @@ struct ResStage {
   uint32_t n, sum, full, base;  // full: entries in place when a group did not fit any more
 };
 // Lanes may be divergent.
-__device__ __forceinline__ void res_stage(uint32_t v, uint32_t od, ResStage &s, uint32_t *q, uint32_t cap,
+__device__ __forceinline__ void res_stage(uint32_t v, uint32_t od, ResStage &s, uint32_t *q, size_t cap,
                                           ResTally *slot) {
   if (od > RES_HUB) {
     q[cap - 1 - res_place(od, &slot->happ)] = v;
@@ -135,23 +135,23 @@ __device__ __forceinline__ void res_stage_flush(ResStage &s, uint32_t *q, ResTal
 // threads; hubs: a warp per chunk of RES_HUB entries.
 template <class Head, class Edge>
 __device__ __forceinline__ void res_expand(const Dir &d, const uint32_t *q, uint32_t n, uint32_t hubs,
-                                           unsigned long long ae, uint32_t cap, Head head, Edge f) {
-  const uint32_t nthreads = gridDim.x * RES_THREADS, tid = blockIdx.x * RES_THREADS + threadIdx.x;
+                                           unsigned long long ae, size_t cap, Head head, Edge f) {
+  const size_t nthreads = (size_t)gridDim.x * RES_THREADS, tid = (size_t)blockIdx.x * RES_THREADS + threadIdx.x;
   const unsigned lane = lane_id();
   const unsigned long long total_n = (unsigned long long)n + hubs;
   const uint32_t group = ae > 16 * total_n && (size_t)n * 32 <= nthreads  ? 32u
                          : ae > 4 * total_n && (size_t)n * 8 <= nthreads ? 8u
                                                                          : 4u;
-  const uint32_t sub = tid % group;
-  for (uint32_t i = tid / group; i < n; i += nthreads / group) {
+  const uint32_t sub = (uint32_t)(tid % group);
+  for (size_t i = tid / group; i < n; i += nthreads / group) {
     const uint32_t src = q[i];
     const unsigned long long b = d.off[src], e = d.off[src + 1];
     const auto m = head(src, sub == 0);
     for (unsigned long long k = b + sub; k < e; k += group) f(m, src, k);
   }
   __syncwarp();
-  const uint32_t nwarps = nthreads / 32, warp = tid / 32;
-  for (uint32_t base = 0; base < hubs; base += 32) {
+  const uint32_t nwarps = (uint32_t)(nthreads / 32), warp = (uint32_t)(tid / 32);
+  for (size_t base = 0; base < hubs; base += 32) {
     uint32_t src = 0, chunks = 0;
     unsigned long long b = 0, e = 0;
     if (base + lane < hubs) {
@@ -184,7 +184,7 @@ __device__ __forceinline__ void res_expand(const Dir &d, const uint32_t *q, uint
 
 // The queue of the bits of bm (hubs apart); a warp per 32 words.
 __device__ __forceinline__ void res_queue_from_bitmap(const uint32_t *bm, size_t words, const uint32_t *out_deg,
-                                                      uint32_t *q, uint32_t cap, ResTally *slot) {
+                                                      uint32_t *q, size_t cap, ResTally *slot) {
   const uint32_t nwarps = gridDim.x * (RES_THREADS / 32), warp = (blockIdx.x * RES_THREADS + threadIdx.x) / 32;
   const unsigned lane = lane_id();
   for (size_t g = warp; g * 32 < words; g += nwarps) {
@@ -203,10 +203,10 @@ __device__ __forceinline__ void res_queue_from_bitmap(const uint32_t *bm, size_t
 
 // The queue without its degree-0 vertices and with its hubs, as the
 // host-driven kernels take it.
-__device__ __forceinline__ void res_plain_queue(const uint32_t *q, uint32_t n, uint32_t hubs, uint32_t cap,
+__device__ __forceinline__ void res_plain_queue(const uint32_t *q, uint32_t n, uint32_t hubs, size_t cap,
                                                 const uint32_t *out_deg, uint32_t *to, ResTally *slot) {
-  const uint32_t nthreads = gridDim.x * RES_THREADS, total = n + hubs;
-  for (uint32_t i = blockIdx.x * RES_THREADS + threadIdx.x; i < (total + 31) / 32 * 32; i += nthreads) {
+  const size_t nthreads = (size_t)gridDim.x * RES_THREADS, total = (size_t)n + hubs;
+  for (size_t i = (size_t)blockIdx.x * RES_THREADS + threadIdx.x; i < (total + 31) / 32 * 32; i += nthreads) {
     const uint32_t v = i < n ? q[i] : i < total ? q[cap - 1 - (i - n)] : 0u;
     const bool keep = i < total && out_deg[v] > 0;
     const unsigned b = __ballot_sync(GG_FULL, keep);

@@ -327,19 +327,16 @@ struct AlignedChunkCount {
   }
 };
 
-// The long-list vertices split into medium and heavy ones; pos, first: the
-// scans of HeavyCount over the list (vertices, chunks).
-__global__ void split_heavy(const uint32_t *__restrict__ big, uint32_t nbig, const uint32_t *__restrict__ deg,
-                            const uint32_t *__restrict__ pos, const uint32_t *__restrict__ first,
-                            uint32_t *__restrict__ med, uint32_t *__restrict__ heavy,
-                            uint32_t *__restrict__ heavy_chunk) {
+// The heavy ones among the long-list vertices; pos, first: the scans of
+// HeavyCount over the list (vertices, chunks).
+__global__ void pick_heavy(const uint32_t *__restrict__ big, uint32_t nbig, const uint32_t *__restrict__ deg,
+                           const uint32_t *__restrict__ pos, const uint32_t *__restrict__ first,
+                           uint32_t *__restrict__ heavy, uint32_t *__restrict__ heavy_chunk) {
   for (size_t i = (size_t)blockIdx.x * blockDim.x + threadIdx.x; i < nbig; i += (size_t)gridDim.x * blockDim.x) {
     const uint32_t v = big[i], h = pos[i];
     if (deg[v] > HEAVY_DEG) {
       heavy[h] = v;
       heavy_chunk[h] = first[i];
-    } else {
-      med[i - h] = v;
     }
     if (i == nbig - 1) heavy_chunk[pos[nbig]] = first[nbig];
   }
@@ -385,7 +382,7 @@ static void hot_bins(const gg_graph *g, Dir *d);
 static int ranks_build(gg_graph *g);
 
 // Degree bins of one direction (see Dir): the long lists (deg > light) with
-// their aligned chunks, split into medium and heavy ones for the BFS pulls.
+// their aligned chunks, and the heavy ones among them for the BFS pulls.
 // Two allocations hold all of them (bins_mem once the number of long lists
 // is known, owner_mem once the chunk counts are).
 static int build_bins(gg_graph *g, Dir *d) {
@@ -420,22 +417,20 @@ static int build_bins(gg_graph *g, Dir *d) {
   GG_CUDA(cudaMemcpyAsync(&tot[1], hpos + n, sizeof(uint32_t), cudaMemcpyDeviceToHost, s));
   GG_CUDA(cudaMemcpyAsync(&tot[2], hfirst + n, sizeof(uint32_t), cudaMemcpyDeviceToHost, s));
   GG_CUDA(cudaStreamSynchronize(s));
-  const size_t nmed = n - tot[1], words = (size_t)tot[0] + tot[2] + nmed + 2 * (size_t)tot[1] + 1;
+  const size_t words = (size_t)tot[0] + tot[2] + 2 * (size_t)tot[1] + 1;
   GG_CUDA(cudaMalloc(&d->owner_mem, sizeof(uint32_t) * words));
   g->graph_bytes += sizeof(uint32_t) * words;
   d->owner_words = words;
   d->nbigchunks = tot[0];
   d->nheavy = tot[1];
   d->nchunks = tot[2];
-  d->nmed = (uint32_t)nmed;
   d->big_owner = d->owner_mem;
   d->chunk_owner = d->big_owner + tot[0];
-  d->med = d->chunk_owner + tot[2];
-  d->heavy = d->med + nmed;
+  d->heavy = d->chunk_owner + tot[2];
   d->heavy_chunk = d->heavy + tot[1];
   fill_chunk_owner<<<grid_for(n, 128, g->num_sms, 8), 128, 0, s>>>(d->big_chunk, n, d->big_owner);
-  split_heavy<<<grid_for(n, 256, g->num_sms, 8), 256, 0, s>>>(d->big, n, d->deg, hpos, hfirst, d->med, d->heavy,
-                                                             d->heavy_chunk);
+  pick_heavy<<<grid_for(n, 256, g->num_sms, 8), 256, 0, s>>>(d->big, n, d->deg, hpos, hfirst, d->heavy,
+                                                            d->heavy_chunk);
   if (tot[1]) fill_chunk_owner<<<grid_for(tot[1], 128, g->num_sms, 8), 128, 0, s>>>(d->heavy_chunk, tot[1],
                                                                                   d->chunk_owner);
   GG_CUDA(cudaGetLastError());
@@ -450,8 +445,8 @@ static void free_bins(gg_graph *g, Dir *d) {
   if (d->owner_mem) cudaFree(d->owner_mem);
   d->bins_mem = d->owner_mem = nullptr;
   d->owner_words = 0;
-  d->med = d->heavy = d->heavy_chunk = d->chunk_owner = d->big = d->big_chunk = d->big_owner = nullptr;
-  d->nmed = d->nheavy = d->nchunks = d->nbig = d->nbigchunks = 0;
+  d->heavy = d->heavy_chunk = d->chunk_owner = d->big = d->big_chunk = d->big_owner = nullptr;
+  d->nheavy = d->nchunks = d->nbig = d->nbigchunks = 0;
 }
 
 // Rebuilds both directions' degree bins for a light-list bound and a pull

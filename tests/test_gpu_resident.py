@@ -48,13 +48,18 @@ GRAPHS = {
 }
 
 
+@pytest.mark.parametrize("layout", [True, False])
 @pytest.mark.parametrize("name", GRAPHS)
-def test_traversals(name):
+def test_traversals(name, layout):
+    """layout False: no rows to pull, so CC and SSSP enter the device for
+    their runs of small sparse calls only, from the host loop and back."""
     V, s, d = GRAPHS[name]
     rng = np.random.default_rng(len(s))
     w = rng.random(len(s), dtype=np.float32)
     g = gg.Graph.from_edges(V, s, d, w)
     gs = gg.Graph.from_edges(V, s, d, w, symmetric=True)
+    g.set_pr_layout(layout)
+    gs.set_pr_layout(layout)
     o, os_ = OracleGraph(V, s, d, w), OracleGraph(V, s, d, w, symmetric=True)
     olabel, octr = os_.cc()
     for root in sorted({0, V - 1, V // 3}):
