@@ -934,37 +934,78 @@ struct BcBwdPull {
   }
 };
 
-__global__ void bc_root(double *np, uint32_t root, uint32_t *visited, uint32_t *active, uint32_t *qlev,
-                        const uint32_t *out_deg, const uint32_t *in_deg, Counters *ctr) {
-  np[root] = 1.0;
-  visited[root >> 5] |= 1u << (root & 31);
-  active[root >> 5] |= 1u << (root & 31);
-  qlev[0] = root;
-  ctr->edges = out_deg[root];
-  ctr->in_edges = in_deg[root];
-}
-
-// inv_num_paths = 1 / num_paths, dependencies = 0 (bc.cpp:103-111).
-__global__ void bc_invert(double *np, double *dep, uint32_t V) {
-  for (size_t v = (size_t)blockIdx.x * blockDim.x + threadIdx.x; v < V; v += (size_t)gridDim.x * blockDim.x) {
-    np[v] = 1.0 / np[v];
+// Path counts and dependencies 0, the root's count 1; the root is level 0.
+// One launch, and the root's number in the layout is read here: as two fills,
+// two clears, a copy of that number to the host and a one-thread kernel it
+// was 45 us of a 480 us call on 4096 vertices.
+__global__ void bc_begin(double *np, double *dep, uint32_t V, uint32_t root, const uint32_t *__restrict__ rank_of,
+                         uint32_t *visited, uint32_t *active, size_t words, uint32_t *qlev,
+                         const uint32_t *__restrict__ out_deg, const uint32_t *__restrict__ in_deg, Counters *ctr) {
+  const uint32_t r = rank_of ? rank_of[root] : root;
+  const size_t t0 = (size_t)blockIdx.x * blockDim.x + threadIdx.x, step = (size_t)gridDim.x * blockDim.x;
+  for (size_t v = t0; v < V; v += step) {
+    np[v] = v == r ? 1.0 : 0.0;
     dep[v] = 0.0;
   }
-}
-
-// process_vertices over one level: visited |= level, dep += inv (bc.cpp:113-120,157-164).
-__global__ void bc_level_apply(const uint32_t *q, uint32_t n, uint32_t *visited, double *dep, const double *inv) {
-  for (size_t i = (size_t)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += (size_t)gridDim.x * blockDim.x) {
-    uint32_t v = q[i];
-    atomicOr(visited + (v >> 5), 1u << (v & 31));
-    dep[v] += inv[v];
+  for (size_t w = t0; w < words; w += step) visited[w] = active[w] = w == r >> 5 ? 1u << (r & 31) : 0u;
+  if (t0 == 0) {
+    qlev[0] = r;
+    ctr->edges = out_deg[r];
+    ctr->in_edges = in_deg[r];
   }
 }
 
-// dependencies = (dep - inv) / inv (bc.cpp:170-176).
-__global__ void bc_final(double *dep, const double *inv, uint32_t V) {
-  for (size_t v = (size_t)blockIdx.x * blockDim.x + threadIdx.x; v < V; v += (size_t)gridDim.x * blockDim.x)
-    dep[v] = (dep[v] - inv[v]) / inv[v];
+// Between two forward calls: the last call's vertices join visited
+// (bc.cpp:91-98), the next call's bitmap and the counters start at 0.  One
+// launch instead of a kernel and two clears (9 us of a small graph's call).
+__global__ void bc_step(uint32_t *visited, const uint32_t *__restrict__ active, uint32_t *next, size_t words,
+                        Counters *ctr) {
+  const size_t t0 = (size_t)blockIdx.x * blockDim.x + threadIdx.x;
+  for (size_t w = t0; w < words; w += (size_t)gridDim.x * blockDim.x) {
+    visited[w] |= active[w];
+    next[w] = 0u;
+  }
+  if (t0 == 0) *ctr = Counters{};
+}
+
+// process_vertices over one level: visited |= level, inv_num_paths = 1 /
+// num_paths, dep += inv (bc.cpp:103-120,157-164); level: also the level's
+// bitmap, for a dense call.  The levels hold the vertices that were reached,
+// side by side: the FP64 unit takes 16 cycles per warp instruction whether 1
+// or 32 lanes divide, and far more for the infinity that 1 / 0 paths gives: a
+// division over all vertices cost 45 us at R-MAT 22 (with bc_final's: the
+// whole call 1681 us before, 1331 us now).
+__global__ void bc_level_apply(const uint32_t *__restrict__ q, uint32_t n, uint32_t *visited, double *dep,
+                               const double *__restrict__ np, double *inv, uint32_t *level) {
+  for (size_t i = (size_t)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += (size_t)gridDim.x * blockDim.x) {
+    const uint32_t v = q[i];
+    const double x = 1.0 / np[v];
+    atomicOr(visited + (v >> 5), 1u << (v & 31));
+    if (level) atomicOr(level + (v >> 5), 1u << (v & 31));
+    inv[v] = x;
+    dep[v] += x;
+  }
+}
+
+// The results in the graph's own numbering: dependencies = (dep - inv) / inv
+// (bc.cpp:170-176) as (dep - inv) * num_paths, which rounds once less, and the
+// inverse path counts.  A vertex that was not reached has 1 / 0 paths and
+// (dep - inf) / inf, written as such: divisions of infinities over all
+// vertices, with the two renumberings after them, took 193 us at R-MAT 22.
+// dep_out and inv_out may be dep and np (no renumbering).
+__global__ void bc_final(const double *dep, const double *np, const double *__restrict__ inv,
+                         const uint32_t *__restrict__ rank_of, uint32_t V, double *dep_out, double *inv_out) {
+  for (size_t v = (size_t)blockIdx.x * blockDim.x + threadIdx.x; v < V; v += (size_t)gridDim.x * blockDim.x) {
+    const uint32_t r = rank_of ? rank_of[v] : (uint32_t)v;
+    const double n = np[r];
+    double x = __longlong_as_double(0x7ff0000000000000ll), y = __longlong_as_double(0x7ff8000000000000ll);
+    if (n != 0.0) {
+      x = inv[r];
+      y = (dep[r] - x) * n;
+    }
+    dep_out[v] = y;
+    inv_out[v] = x;
+  }
 }
 
 static int bc_run(gg_graph *g, uint32_t root, double *dep_host, double *inv_host, gg_run_stats *st) {
@@ -975,14 +1016,14 @@ static int bc_run(gg_graph *g, uint32_t root, double *dep_host, double *inv_host
   GG_CUDA(cudaSetDevice(g->device));
   const uint32_t V = g->V;
   const size_t words = bitmap_words32(V);
-  double *np, *dep;
-  uint32_t *visited, *bm[2], *lvbm, *qlev;
+  double *np, *dep, *inv;
+  uint32_t *visited, *bm[2], *qlev;
   GG_TRY(ws(g, WS_S2, V, &np));
   GG_TRY(ws(g, WS_S3, V, &dep));
+  GG_TRY(ws(g, WS_MSG, V, &inv));
   GG_TRY(ws(g, WS_BM0, words, &visited));
   GG_TRY(ws(g, WS_BM1, words, &bm[0]));
   GG_TRY(ws(g, WS_BM2, words, &bm[1]));
-  GG_TRY(ws(g, WS_BM3, words, &lvbm));
   GG_TRY(ws(g, WS_QLEV, (size_t)V + 2, &qlev));
   // Hot-source layout (as SSSP's): both directions renumbered; path counts
   // are exact and dependencies change only in summation order.
@@ -993,10 +1034,9 @@ static int bc_run(gg_graph *g, uint32_t root, double *dep_host, double *inv_host
   const bool ranked = g->pr_layout && g->pr_ready && (g->symmetric || g->pr_out_ready);
   const Dir &dout = ranked ? (g->symmetric ? g->pr : g->pr_out) : g->out;
   const Dir &din = ranked ? g->pr : g->in;
-  uint32_t start = root;
+  const uint32_t *rank_of = ranked ? g->pr_rank_of : nullptr;
   double *dep_out = dep, *np_out = np;
   if (ranked) {
-    GG_CUDA(cudaMemcpy(&start, g->pr_rank_of + root, sizeof(uint32_t), cudaMemcpyDeviceToHost));
     GG_TRY(ws(g, WS_S0, V, &dep_out));
     GG_TRY(ws(g, WS_S1, V, &np_out));
   }
@@ -1005,12 +1045,10 @@ static int bc_run(gg_graph *g, uint32_t root, double *dep_host, double *inv_host
   cudaStream_t s = g->stream;
   Counters *ctr = g->ws.ctr;
   GG_TRY(timed_begin(g));
-  GG_CUDA(cudaMemsetAsync(visited, 0, words * 4, s));
-  GG_CUDA(cudaMemsetAsync(bm[0], 0, words * 4, s));
   GG_TRY(counters_reset(g));
-  fill_kernel<double><<<grid_for(V, 256, g->num_sms), 256, 0, s>>>(np, V, 0.0);
-  bc_root<<<1, 1, 0, s>>>(np, start, visited, bm[0], qlev, dout.deg, din.deg, ctr);
-  L.launches += 2;
+  bc_begin<<<grid_for(V, 256, g->num_sms), 256, 0, s>>>(np, dep, V, root, rank_of, visited, bm[0], words, qlev,
+                                                        dout.deg, din.deg, ctr);
+  L.launches += 1;
   GG_CUDA(cudaGetLastError());
   Counters c;
   GG_TRY(counters_read(g, &c));
@@ -1024,11 +1062,10 @@ static int bc_run(gg_graph *g, uint32_t root, double *dep_host, double *inv_host
     bool sparse = ae < g->E / 20;
     tr.add(sparse ? 0 : 1, ae, 0);
     int nx = cur ^ 1;
-    GG_CUDA(cudaMemsetAsync(bm[nx], 0, words * 4, s));
-    GG_TRY(counters_reset(g));
+    bc_step<<<grid_for(words, 256, g->num_sms), 256, 0, s>>>(visited, bm[cur], bm[nx], words, ctr);
+    L.launches += 1;
     ActOut a;
     a.active_out = bm[nx];
-    a.q_out = qlev + lev_off.back();
     a.qlen = &ctr->qlen;
     a.out_deg = dout.deg;
     a.in_deg = din.deg;
@@ -1057,9 +1094,6 @@ static int bc_run(gg_graph *g, uint32_t root, double *dep_host, double *inv_host
       uint32_t nl = 0;
       GG_TRY(L.queue_from_bitmap(bm[nx], nullptr, qlev + lev_off.back(), &nl));
     }
-    // visited |= active_out (bc.cpp:91-98)
-    bitmap_or<<<grid_for(words, 256, g->num_sms), 256, 0, s>>>(visited, bm[nx], words);
-    L.launches += 1;
     lev_off.push_back(lev_off.back() + n);
     lev_out.push_back(c.edges);
     lev_in.push_back(c.in_edges);
@@ -1067,16 +1101,18 @@ static int bc_run(gg_graph *g, uint32_t root, double *dep_host, double *inv_host
   }
   // levels 0..top; level `top` is the empty set the last forward call produced
   const int top = (int)lev_off.size() - 2;
-  bc_invert<<<grid_for(V, 256, g->num_sms), 256, 0, s>>>(np, dep, V);
   GG_CUDA(cudaMemsetAsync(visited, 0, words * 4, s));
-  L.launches += 1;
+  // the levels' bitmaps, for dense calls (the forward calls are done with them)
+  uint32_t *lvbm = bm[0], *lvbm_next = bm[1];
+  auto dense_level = [&](int lev) { return lev_in[lev] >= g->E / 20; };
+  if (dense_level(top)) GG_CUDA(cudaMemsetAsync(lvbm, 0, words * 4, s));  // the last level is empty
   // backward on the transposed graph: push over the CSC, pull over the CSR
   const Dir &tout = din, &tin = dout;
   for (int lev = top; lev >= 1; lev--) {
     uint32_t ln = (uint32_t)(lev_off[lev + 1] - lev_off[lev]);
     const uint32_t *ql = qlev + lev_off[lev];
     unsigned long long ae = lev_in[lev];
-    bool sparse = ae < g->E / 20;
+    bool sparse = !dense_level(lev);
     tr.add(sparse ? 0 : 1, ae, 0);
     if (sparse) {
       if (ae > 0) {
@@ -1089,26 +1125,22 @@ static int bc_run(gg_graph *g, uint32_t root, double *dep_host, double *inv_host
         L.launches += 1;
       }
     } else {
-      GG_CUDA(cudaMemsetAsync(lvbm, 0, words * 4, s));
-      if (ln) bitmap_from_queue<<<grid_for(ln, 256, g->num_sms), 256, 0, s>>>(ql, ln, lvbm);
       GG_TRY(tr.kbegin());
       GG_TRY(L.pull(tin, BcBwdPull{dep, lvbm, visited}, ActOut(), ctr));
       GG_TRY(tr.kend());
-      L.launches += 1;
     }
     uint32_t pn = (uint32_t)(lev_off[lev] - lev_off[lev - 1]);
+    uint32_t *mark = lev > 1 && dense_level(lev - 1) ? lvbm_next : nullptr;
+    if (mark) GG_CUDA(cudaMemsetAsync(mark, 0, words * 4, s));
     if (pn)
-      bc_level_apply<<<grid_for(pn, 256, g->num_sms), 256, 0, s>>>(qlev + lev_off[lev - 1], pn, visited, dep, np);
+      bc_level_apply<<<grid_for(pn, 256, g->num_sms), 256, 0, s>>>(qlev + lev_off[lev - 1], pn, visited, dep, np, inv,
+                                                                   mark);
     L.launches += 1;
     GG_CUDA(cudaGetLastError());
+    std::swap(lvbm, lvbm_next);
   }
-  bc_final<<<grid_for(V, 256, g->num_sms), 256, 0, s>>>(dep, np, V);
+  bc_final<<<grid_for(V, 256, g->num_sms), 256, 0, s>>>(dep, np, inv, rank_of, V, dep_out, np_out);
   L.launches += 1;
-  if (ranked) {
-    unrank<double><<<grid_for(V, 256, g->num_sms), 256, 0, s>>>(dep, g->pr_rank_of, V, dep_out);
-    unrank<double><<<grid_for(V, 256, g->num_sms), 256, 0, s>>>(np, g->pr_rank_of, V, np_out);
-    L.launches += 2;
-  }
   GG_CUDA(cudaGetLastError());
   GG_TRY(timed_end(g, st, L.launches));
   GG_TRY(tr.collect());

@@ -109,7 +109,7 @@ enum WsSlot {
   WS_BM0, WS_BM1, WS_BM2, WS_BM3,       // bitmaps
   WS_Q0, WS_Q1, WS_QLEV,                // queues / level order
   WS_PREFIX,                            // uint64 prefix of queue degrees
-  WS_MSG,                               // per-queue-entry message snapshot (4 or 8 B)
+  WS_MSG,                               // a second state array: CC, SSSP (4 B), BC's inverse path counts (8 B)
   WS_S0, WS_S1, WS_S2, WS_S3,           // vertex state arrays
   WS_SCAN,                              // scan scratch
   WS_HUBSUM,                            // per-iteration counters (PageRank)

@@ -926,12 +926,6 @@ static __global__ void iota_u32(uint32_t *__restrict__ a, uint32_t n) {
     a[i] = (uint32_t)i;
 }
 
-// dst |= src, word by word.
-static __global__ void bitmap_or(uint32_t *__restrict__ dst, const uint32_t *__restrict__ src, size_t words) {
-  for (size_t i = (size_t)blockIdx.x * blockDim.x + threadIdx.x; i < words; i += (size_t)gridDim.x * blockDim.x)
-    dst[i] |= src[i];
-}
-
 // Sets the bits of the n queued vertices.
 static __global__ void bitmap_from_queue(const uint32_t *__restrict__ q, uint32_t n, uint32_t *__restrict__ bm) {
   for (size_t i = (size_t)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += (size_t)gridDim.x * blockDim.x) {
