@@ -32,15 +32,14 @@ constexpr int LANES = 64;
 
 typedef LaneCounters MsCounters;
 
-// write_min on a float (core/atomic.hpp:35-42): true if this call lowered *p.
-__device__ __forceinline__ bool atomic_min_float_b(float *p, float v) {
-  if (!(v < 0.0f)) {
-    int old = atomicMin((int *)p, __float_as_int(v));
-    return __int_as_float(old) > v;
-  }
-  unsigned old = atomicMax((unsigned *)p, __float_as_uint(v));
-  return __uint_as_float(old) > v;
+// write_min on a float (core/atomic.hpp:35-42): the value before.
+__device__ __forceinline__ float atomic_min_float_old(float *p, float v) {
+  if (!(v < 0.0f)) return __int_as_float(atomicMin((int *)p, __float_as_int(v)));
+  return __uint_as_float(atomicMax((unsigned *)p, __float_as_uint(v)));
 }
+
+// True if this call lowered *p.
+__device__ __forceinline__ bool atomic_min_float_b(float *p, float v) { return atomic_min_float_old(p, v) > v; }
 
 __device__ __forceinline__ u64 warp_or64(u64 x) {
 #pragma unroll
@@ -782,13 +781,52 @@ __global__ void __launch_bounds__(256)
 
 // ---------------------------------------------------------------- batched SSSP
 
-// Relaxation of every out-edge (u, v, w) of the union frontier, one warp per
-// edge: lane j handles SSSP lanes j and j + 32 of the edge (a coalesced 256 B
-// row of dist[v]).  A lane whose distance at v was lowered gets v's next bit;
-// the first setter of next[v] queues v.  Reads dist[u] as it is now (the
-// fixpoint, hence every lane's result, does not depend on that order).
+constexpr int MSP_TILE_MIN = 64;  // edges per tile of msp_push at least: 8 warps of 8
+// Edges per tile of msp_push, a quarter of the edges a block has to do, so
+// that the blocks end together (batch of 64 on 131072 vertices, 1 / 2 / 4 / 8
+// tiles per block: 5.58 / 5.62 / 5.49 / 5.49 ms) and a step of few edges is
+// spread over as many warps as there are: tiles of 1024 for all left the first
+// two steps of 64 roots, about 2000 edges, to two blocks, 215 us each.
+__device__ __forceinline__ unsigned msp_tile(unsigned long long total) {
+  const unsigned long long per = total / gridDim.x / 4;
+  unsigned t = MSP_TILE_MIN;
+  while (t < (unsigned)PUSH_TILE && t < per) t <<= 1;
+  return t;
+}
+
+// Appends the vertices a tile queued (s_q[0, s_n)) with one atomic: one per
+// vertex, all on one counter, are served one after the other (64000 in a step;
+// 64 roots on 100003 vertices: 3.18 ms so, 3.01 with one per tile).  All threads
+// of the block must call; s_n is 0 afterwards.
+__device__ __forceinline__ void msp_append(const uint32_t *s_q, unsigned *s_n, unsigned *s_at, uint32_t *q_out,
+                                           unsigned *qlen) {
+  __syncthreads();
+  const unsigned c = *s_n;
+  if (c == 0) return;
+  if (threadIdx.x == 0) *s_at = atomicAdd(qlen, c);
+  __syncthreads();
+  const unsigned at = *s_at;
+  for (unsigned i = threadIdx.x; i < c; i += PUSH_THREADS) q_out[at + i] = s_q[i];
+  if (threadIdx.x == 0) *s_n = 0;
+}
+
+// Relaxation of every out-edge (u, v, w) of the union frontier, half a warp per
+// edge: lane j holds SSSP lanes 4j .. 4j + 3 of its edge (a coalesced 256 B row
+// of dist[v]).  A lane whose distance at v was lowered gets v's next bit; the
+// first setter of next[v] queues v.  Reads dist[u] as it is now (the fixpoint,
+// hence every lane's result, does not depend on that order).
+//
+// What bounds it is latency: the chain source -> neighbour -> row of each edge,
+// and the atomics behind it.  So a warp takes a run of up to 32 edges, its lanes
+// find source, neighbour, weight and mask of one edge each, and the rows follow
+// two edges at a time (the source's row from L1 where the run shares it), at 8
+// blocks per SM: rows of 4 or 8 edges at a time with 6 or 4 blocks were slower
+// (64 roots on 100003 vertices: 2.9 - 3.0 / 3.1 ms of the whole call; 2.7 as
+// here with the four atomics of a lane one after the other, 2.4 with all four
+// in flight; a warp per edge, one edge after the other, with an atomic on the
+// queue's length per vertex: 5.6 ms).
 template <bool G>
-__global__ void __launch_bounds__(PUSH_THREADS)
+__global__ void __launch_bounds__(PUSH_THREADS, 8)
     msp_push(const uint32_t *__restrict__ q, const unsigned long long *__restrict__ P, uint32_t n,
              unsigned long long total, Dir d, const u64 *__restrict__ front, u64 *next, float *dist, uint32_t *q_out,
              MsCounters *mc, const MsState *st) {
@@ -802,14 +840,18 @@ __global__ void __launch_bounds__(PUSH_THREADS)
   }
   __shared__ unsigned long long s_P[PUSH_STAGE + 1];
   __shared__ unsigned long long s_base[PUSH_STAGE];
-  __shared__ uint32_t s_src[PUSH_STAGE];
+  __shared__ uint32_t s_src[PUSH_STAGE], s_q[PUSH_TILE];
   __shared__ uint32_t s_lo, s_hi;
+  __shared__ unsigned s_nq, s_at;
+  if (threadIdx.x == 0) s_nq = 0;  // seen after tile_bounds' barrier
   const unsigned lane = lane_id(), w = threadIdx.x >> 5;
-  const unsigned long long ntiles = (total + PUSH_TILE - 1) / PUSH_TILE;
+  const unsigned tile_edges = msp_tile(total);
+  const unsigned run = tile_edges / (PUSH_THREADS / 32) < 32u ? tile_edges / (PUSH_THREADS / 32) : 32u;
+  const unsigned long long ntiles = (total + tile_edges - 1) / tile_edges;
   u64 t_alive = 0, t_edges = 0;
   for (unsigned long long tile = blockIdx.x; tile < ntiles; tile += gridDim.x) {
-    const unsigned long long e0 = tile * PUSH_TILE;
-    const unsigned long long e1 = e0 + PUSH_TILE < total ? e0 + PUSH_TILE : total;
+    const unsigned long long e0 = tile * tile_edges;
+    const unsigned long long e1 = e0 + tile_edges < total ? e0 + tile_edges : total;
     tile_bounds(P, n, e0, e1, &s_lo, &s_hi);
     __syncthreads();
     const uint32_t lo = s_lo, hi = s_hi, cnt = hi - lo;
@@ -824,43 +866,72 @@ __global__ void __launch_bounds__(PUSH_THREADS)
       }
     }
     __syncthreads();
-    // each warp takes every eighth edge of the tile; its lanes cover the 64 SSSP lanes
-    for (unsigned long long e = e0 + w; e < e1; e += PUSH_THREADS / 32) {
-      uint32_t u;
-      unsigned long long k;
-      if (staged) {
-        const uint32_t i = upper_bound_idx<unsigned long long>(s_P, 0, cnt, e) - 1;
-        u = s_src[i];
-        k = s_base[i] + e;
-      } else {
-        const uint32_t i = upper_bound_idx<unsigned long long>(P, lo, hi, e) - 1;
-        u = q[i];
-        k = d.off[u] + (e - P[i]);
-      }
-      const uint32_t v = nbr_at(d, k, GG_SITE);
-      const float wt = d.w[k];
-      const u64 fm = front[u];
-      bool low0 = false, low1 = false;
-      if ((fm >> lane) & 1ull) {
-        const float nd = __fadd_rn(dist[(size_t)u * LANES + lane], wt);
-        float *p = dist + (size_t)v * LANES + lane;
-        if (nd < *(volatile float *)p) low0 = atomic_min_float_b(p, nd);
-      }
-      if ((fm >> (lane + 32)) & 1ull) {
-        const float nd = __fadd_rn(dist[(size_t)u * LANES + lane + 32], wt);
-        float *p = dist + (size_t)v * LANES + lane + 32;
-        if (nd < *(volatile float *)p) low1 = atomic_min_float_b(p, nd);
-      }
-      const u64 low = (u64)__ballot_sync(GG_FULL, low0) | ((u64)__ballot_sync(GG_FULL, low1) << 32);
-      if (low && lane == 0) {
-        const u64 old = atomicOr(next + v, low);
-        if (!old) {
-          q_out[atomicAdd(&mc->qlen, 1u)] = v;
-          t_edges += d.deg[v];
+    // the warps take runs of the tile's edges in turn
+    for (unsigned long long r0 = e0 + (unsigned long long)w * run; r0 < e1;
+         r0 += (unsigned long long)run * (PUSH_THREADS / 32)) {
+      const unsigned m = e1 - r0 < run ? (unsigned)(e1 - r0) : run;
+      uint32_t u = 0, v = 0;
+      float wt = 0.0f;
+      unsigned f0 = 0, f1 = 0;  // the source's lanes 0-31 and 32-63
+      if (lane < m) {
+        const unsigned long long e = r0 + lane;
+        unsigned long long k;
+        if (staged) {
+          const uint32_t i = upper_bound_idx<unsigned long long>(s_P, 0, cnt, e) - 1;
+          u = s_src[i];
+          k = s_base[i] + e;
+        } else {
+          const uint32_t i = upper_bound_idx<unsigned long long>(P, lo, hi, e) - 1;
+          u = q[i];
+          k = d.off[u] + (e - P[i]);
         }
-        t_alive |= low;
+        v = nbr_at(d, k, GG_SITE);
+        wt = d.w[k];
+        const u64 fm = front[u];
+        f0 = (unsigned)fm;
+        f1 = (unsigned)(fm >> 32);
+      }
+      const unsigned h = lane >> 4, j4 = (lane & 15u) * 4u;
+      for (unsigned i0 = 0; i0 < m; i0 += 2) {
+        const unsigned i = i0 + h;  // < 32: the runs are even
+        const uint32_t ui = __shfl_sync(GG_FULL, u, i), vi = __shfl_sync(GG_FULL, v, i);
+        const float wi = __shfl_sync(GG_FULL, wt, i);
+        const unsigned g0 = __shfl_sync(GG_FULL, f0, i), g1 = __shfl_sync(GG_FULL, f1, i);
+        const unsigned f = ((j4 < 32u ? g0 : g1) >> (j4 & 31u)) & 15u;  // none in the lanes past m
+        unsigned low = 0;
+        if (f) {
+          float *p = dist + (size_t)vi * LANES + j4;
+          const float4 a = *(const float4 *)(dist + (size_t)ui * LANES + j4);
+          const float4 o = __ldcg((const float4 *)p);
+          const float x0 = __fadd_rn(a.x, wi), x1 = __fadd_rn(a.y, wi);
+          const float x2 = __fadd_rn(a.z, wi), x3 = __fadd_rn(a.w, wi);
+          // all four in flight before the first result is used; a distance not tried stays
+          float r0 = x0, r1 = x1, r2 = x2, r3 = x3;
+          if ((f & 1u) && x0 < o.x) r0 = atomic_min_float_old(p, x0);
+          if ((f & 2u) && x1 < o.y) r1 = atomic_min_float_old(p + 1, x1);
+          if ((f & 4u) && x2 < o.z) r2 = atomic_min_float_old(p + 2, x2);
+          if ((f & 8u) && x3 < o.w) r3 = atomic_min_float_old(p + 3, x3);
+          low = (r0 > x0 ? 1u : 0u) | (r1 > x1 ? 2u : 0u) | (r2 > x2 ? 4u : 0u) | (r3 > x3 ? 8u : 0u);
+        }
+        if (!__any_sync(GG_FULL, low != 0)) continue;
+        unsigned l0 = j4 < 32u ? low << j4 : 0u, l1 = j4 < 32u ? 0u : low << (j4 - 32u);
+#pragma unroll
+        for (int s = 1; s < 16; s <<= 1) {
+          l0 |= __shfl_xor_sync(GG_FULL, l0, s);
+          l1 |= __shfl_xor_sync(GG_FULL, l1, s);
+        }
+        if ((l0 | l1) && (lane & 15u) == 0) {
+          const u64 bits = (u64)l0 | ((u64)l1 << 32);
+          const u64 old = atomicOr(next + vi, bits);
+          if (!old) {
+            s_q[atomicAdd(&s_nq, 1u)] = vi;  // at most one per edge of the tile
+            t_edges += d.deg[vi];
+          }
+          t_alive |= bits;
+        }
       }
     }
+    msp_append(s_q, &s_nq, &s_at, q_out, &mc->qlen);
     __syncthreads();
   }
   ms_flush(mc, t_alive, t_edges, 0);
@@ -884,8 +955,10 @@ __global__ void __launch_bounds__(PUSH_THREADS, 8)
   }
   __shared__ unsigned long long s_P[PUSH_STAGE + 1];
   __shared__ unsigned long long s_base[PUSH_STAGE];
-  __shared__ uint32_t s_src[PUSH_STAGE];
+  __shared__ uint32_t s_src[PUSH_STAGE], s_q[PUSH_TILE];
   __shared__ uint32_t s_lo, s_hi;
+  __shared__ unsigned s_nq, s_at;
+  if (threadIdx.x == 0) s_nq = 0;  // seen after tile_bounds' barrier
   const unsigned long long ntiles = (total + PUSH_TILE - 1) / PUSH_TILE;
   u64 t_alive = 0, t_edges = 0;
   for (unsigned long long tile = blockIdx.x; tile < ntiles; tile += gridDim.x) {
@@ -930,12 +1003,13 @@ __global__ void __launch_bounds__(PUSH_THREADS, 8)
       if (low) {
         const u64 old = atomicOr(next + v, low);
         if (!old) {
-          q_out[atomicAdd(&mc->qlen, 1u)] = v;
+          s_q[atomicAdd(&s_nq, 1u)] = v;  // at most one per edge of the tile
           t_edges += d.deg[v];
         }
         t_alive |= low;
       }
     }
+    msp_append(s_q, &s_nq, &s_at, q_out, &mc->qlen);
     __syncthreads();
   }
   ms_flush(mc, t_alive, t_edges, 0);
@@ -1139,8 +1213,8 @@ int LanePool::build_queue() {
   return GG_OK;
 }
 
-static unsigned push_grid_for(const gg_graph *g, unsigned long long total) {
-  unsigned long long tiles = (total + PUSH_TILE - 1) / PUSH_TILE;
+static unsigned push_grid_for(const gg_graph *g, unsigned long long total, unsigned tile_edges) {
+  unsigned long long tiles = (total + tile_edges - 1) / tile_edges;
   unsigned long long cap = (unsigned long long)g->num_sms * 8;
   return (unsigned)(tiles < 1 ? 1 : (tiles > cap ? cap : tiles));
 }
@@ -1186,7 +1260,8 @@ int LanePool::push_kernels(bool per_thread, int *n) {
   else
     GG_CUDA((exclusive_scan<unsigned long long, QueueDegreeIn>(QueueDegreeIn{q_[cur_], g_->out.deg}, nq_, prefix_,
                                                                scan64_, s_, n)));
-  const unsigned grid = G ? (unsigned)g_->num_sms * 8 : push_grid_for(g_, ae_);
+  const unsigned grid =
+      G ? (unsigned)g_->num_sms * 8 : push_grid_for(g_, ae_, kind_ == SSSP && !per_thread ? MSP_TILE_MIN : PUSH_TILE);
   if (!G && tr_) GG_TRY(tr_->kbegin());
   if (kind_ == BFS)
     ms_push<G><<<grid, PUSH_THREADS, 0, s_>>>(q_[cur_], prefix_, nq_, ae_, g_->out, front_, visit_, next_, lvl_,
@@ -1369,9 +1444,10 @@ int LanePool::sssp_bucket_step() {
     GG_CUDA((exclusive_scan<unsigned long long, QueueDegreeIn>(QueueDegreeIn{q_[cur_], g_->out.deg}, nq_, prefix_,
                                                                scan64_, s_, &launches)));
     if (tr_) GG_TRY(tr_->kbegin());
-    (__builtin_popcountll(active_) <= (int)g_->batched_thread_lanes ? msp_push_thread<false> : msp_push<false>)<<<
-        push_grid_for(g_, ae_), PUSH_THREADS, 0, s_>>>(q_[cur_], prefix_, nq_, ae_, g_->out, front_, next_,
-                                                              dist_, q_[cur_ ^ 1], mc_, nullptr);
+    const bool per_thread = __builtin_popcountll(active_) <= (int)g_->batched_thread_lanes;
+    (per_thread ? msp_push_thread<false> : msp_push<false>)<<<
+        push_grid_for(g_, ae_, per_thread ? PUSH_TILE : MSP_TILE_MIN), PUSH_THREADS, 0, s_>>>(
+        q_[cur_], prefix_, nq_, ae_, g_->out, front_, next_, dist_, q_[cur_ ^ 1], mc_, nullptr);
     if (tr_) GG_TRY(tr_->kend());
     launches += 1;
   }
