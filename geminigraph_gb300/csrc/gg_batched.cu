@@ -508,33 +508,32 @@ __global__ void lanes_reset_dist(float *dist, uint32_t V, u64 mask) {
     if ((mask >> (i % LANES)) & 1ull) dist[i] = 1e9f;
 }
 
-// Roots into lanes: frontier bit, visited bit / distance 0, discovery iteration.
+// Roots into lanes, a thread each (their loads in one go: one thread for all
+// took 30 - 63 us for 64 roots, this one 4): frontier bit, visited bit /
+// distance 0, discovery iteration.
 // list: the roots' level-list entries (instead of their level rows).
 __global__ void lanes_admit(const uint32_t *roots, const int *lanes, int n, u64 *front, u64 *visit, uint32_t *lvl,
                             uint32_t *par, float *dist, uint32_t iter, const uint32_t *out_deg, MsCounters *mc,
                             u64 *lane_sum, LevelEntry *list) {
-  if (threadIdx.x != 0 || blockIdx.x != 0) return;
-  u64 edges = 0;
-  for (int i = 0; i < n; i++) {
-    const uint32_t r = roots[i];
-    const int l = lanes[i];
-    if (!front[r]) edges += out_deg[r];
-    front[r] |= 1ull << l;
-    if (visit) visit[r] |= 1ull << l;
-    if (list) {
-      const u64 m = 1ull << l;
-      list[i] = make_uint4(r, iter, (unsigned)m, (unsigned)(m >> 32));
-    } else if (lvl) {
-      lvl[(size_t)r * LANES + l] = iter;
-    }
-    if (par) par[(size_t)r * LANES + l] = r;
-    if (dist) dist[(size_t)r * LANES + l] = 0.0f;
-    if (lane_sum) {
-      lane_sum[l] = 1;
-      lane_sum[LANES + l] = out_deg[r];
-    }
+  const int i = blockIdx.x * blockDim.x + threadIdx.x;
+  if (i >= n) return;
+  const uint32_t r = roots[i];
+  const int l = lanes[i];
+  const u64 m = 1ull << l;
+  const uint32_t deg = out_deg[r];
+  // several roots may be one vertex: its edges count once
+  if (atomicOr(front + r, m) == 0) atomicAdd(&mc->edges, (u64)deg);
+  if (visit) atomicOr(visit + r, m);
+  if (list)
+    list[i] = make_uint4(r, iter, (unsigned)m, (unsigned)(m >> 32));
+  else if (lvl)
+    lvl[(size_t)r * LANES + l] = iter;
+  if (par) par[(size_t)r * LANES + l] = r;
+  if (dist) dist[(size_t)r * LANES + l] = 0.0f;
+  if (lane_sum) {
+    lane_sum[l] = 1;
+    lane_sum[LANES + l] = deg;
   }
-  mc->edges = edges;
 }
 
 // Levels of the lanes slot[l] >= 0 from the level lists, lane-major:
@@ -1176,7 +1175,7 @@ int LanePool::admit(const uint32_t *roots, const int *lanes, int n) {
   else
     lanes_reset_dist<<<grid_for((size_t)V * LANES, 256, g_->num_sms, 16), 256, 0, s_>>>(dist_, V, mask);
   GG_CUDA(cudaMemsetAsync(mc_, 0, sizeof(LaneCounters), s_));
-  lanes_admit<<<1, 32, 0, s_>>>(roots_dev_, lanes_dev_, n, front_, visit_, lvl_, par_, dist_, iter_, g_->out.deg, mc_,
+  lanes_admit<<<1, LANES, 0, s_>>>(roots_dev_, lanes_dev_, n, front_, visit_, lvl_, par_, dist_, iter_, g_->out.deg, mc_,
                                 lane_sum_, list_mode_ ? list_ + list_n_ : nullptr);
   launches += 2;
   GG_CUDA(cudaGetLastError());
