@@ -1855,6 +1855,8 @@ static int run_batch(gg_graph *g, LanePool::Kind kind, const uint32_t *roots, in
   const uint32_t V = g->V;
   int lanes[LANES];
   for (int i = 0; i < nroots; i++) lanes[i] = i;
+  const size_t out_bytes = sizeof(uint32_t) * (size_t)V * nroots;  // levels, parents and distances alike
+  Prefault pages(levels ? (void *)levels : (void *)dist_out, out_bytes, par_out, out_bytes);
   cudaStream_t gs = g->stream;
   g->stream = p->stream();  // events and traces on the pool's stream
   status = timed_begin(g);
@@ -1876,6 +1878,7 @@ static int run_batch(gg_graph *g, LanePool::Kind kind, const uint32_t *roots, in
   p->retire(mask);
   p->set_trace(nullptr);
   if (status != GG_OK) return status;
+  pages.wait();
   if (levels) GG_CUDA(cudaMemcpy(levels, d_lv, sizeof(int32_t) * V * nroots, cudaMemcpyDeviceToHost));
   if (par_out) GG_CUDA(cudaMemcpy(par_out, d_pa, sizeof(uint32_t) * V * nroots, cudaMemcpyDeviceToHost));
   if (dist_out) GG_CUDA(cudaMemcpy(dist_out, d_di, sizeof(float) * V * nroots, cudaMemcpyDeviceToHost));

@@ -426,6 +426,7 @@ static int bc_batched_run(gg_graph *g, const uint32_t *roots, int n, double *dep
   GG_CUDA(cudaMemcpyAsync(levels[0].v.p, r0.data(), sizeof(uint32_t) * r0.size(), cudaMemcpyHostToDevice, s));
   GG_CUDA(cudaMemcpyAsync(levels[0].m.p, m0.data(), sizeof(u64) * m0.size(), cudaMemcpyHostToDevice, s));
   GG_CUDA(cudaMemcpyAsync(roots_b.p, roots, sizeof(uint32_t) * n, cudaMemcpyHostToDevice, s));
+  Prefault pages(dep_host, sizeof(double) * (size_t)n * V, inv_host, sizeof(double) * (size_t)n * V);
   GG_TRY(timed_begin(g));
   GG_CUDA(cudaMemsetAsync(np, 0, lanes_bytes, s));
   GG_CUDA(cudaMemsetAsync(dep, 0, lanes_bytes, s));
@@ -544,6 +545,7 @@ static int bc_batched_run(gg_graph *g, const uint32_t *roots, int n, double *dep
   launches += 1;
   GG_CUDA(cudaGetLastError());
   GG_TRY(timed_end(g, st, launches));
+  pages.wait();
   if (dep_host) GG_CUDA(cudaMemcpy(dep_host, out_dep, sizeof(double) * (size_t)n * V, cudaMemcpyDeviceToHost));
   if (inv_host) GG_CUDA(cudaMemcpy(inv_host, out_inv, sizeof(double) * (size_t)n * V, cudaMemcpyDeviceToHost));
   if (reached_host) {

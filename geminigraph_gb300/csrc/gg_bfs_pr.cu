@@ -430,6 +430,7 @@ static int bfs_run(gg_graph *g, uint32_t root, uint32_t *parent_host, gg_run_sta
       L.launches += 1;
     }
   };
+  Prefault pages(parent_host, sizeof(uint32_t) * V);
   GG_TRY(timed_begin(g));
   bfs_begin<<<grid_for(V, 256, g->num_sms), 256, 0, s>>>(parent, V, visited, words, root, q[0], g->out.deg, blob,
                                                         coop ? small_lim : 0ull, lim);
@@ -540,6 +541,7 @@ static int bfs_run(gg_graph *g, uint32_t root, uint32_t *parent_host, gg_run_sta
   }
   GG_TRY(timed_end(g, st, L.launches));
   GG_TRY(tr.collect());
+  pages.wait();
   if (parent_host) GG_CUDA(cudaMemcpy(parent_host, parent, sizeof(uint32_t) * V, cudaMemcpyDeviceToHost));
   g->result[0] = parent;
   g->result[1] = nullptr;
@@ -737,6 +739,7 @@ static int pr_run(gg_graph *g, int iterations, T *ranks_host, double *deltas_hos
   }
   GG_TRY(timed_begin(g));
   GG_CUDA(cudaGraphLaunch(exec, s));
+  Prefault pages(ranks_host, sizeof(T) * V);
   const T *result = ranked ? out : buf[cur];
   GG_TRY(timed_end(g, st, L.launches));
   GG_TRY(tr.collect());
@@ -750,6 +753,7 @@ static int pr_run(gg_graph *g, int iterations, T *ranks_host, double *deltas_hos
     delete[] hc;
     GG_CUDA(e);
   }
+  pages.wait();
   if (ranks_host) GG_CUDA(cudaMemcpy(ranks_host, result, sizeof(T) * V, cudaMemcpyDeviceToHost));
   g->result[0] = result;
   g->result[1] = nullptr;

@@ -679,9 +679,10 @@ __global__ void unrank(const T *__restrict__ by_rank, const uint32_t *__restrict
 }
 
 // The end of a whole run: its time and its result.
-static int relax_done(gg_graph *g, gg_run_stats *st, const Launch &L, void *user, const void *dev, const void *host,
-                      size_t bytes) {
+static int relax_done(gg_graph *g, gg_run_stats *st, const Launch &L, Prefault &pages, void *user, const void *dev,
+                      const void *host, size_t bytes) {
   GG_TRY(timed_read(g, st, L.launches));
+  pages.wait();
   if (user && host)
     memcpy(user, host, bytes);
   else if (user)
@@ -716,6 +717,7 @@ static int cc_run(gg_graph *g, uint32_t *label_host, gg_run_stats *st) {
   Trace tr(st, g, "gg_cc");
   cudaStream_t s = g->stream;
   Counters *ctr = g->ws.ctr;
+  Prefault pages(label_host, sizeof(uint32_t) * V);
   GG_TRY(timed_begin(g));
   CcPull pull{};
   pull.hot = ranked ? g->l1_hot_bytes / 4 : 0xffffffffu;
@@ -725,7 +727,7 @@ static int cc_run(gg_graph *g, uint32_t *label_host, gg_run_stats *st) {
   void *const states[2] = {lab[0], lab[1]};
   GG_TRY((relax_whole<CcRun>(g, dout, din, pull, ranked, 0, states, q, bm, out, sizeof(uint32_t) * V, L, tr, st, &whole,
                              &dev, &host)));
-  if (whole) return relax_done(g, st, L, label_host, dev, host, sizeof(uint32_t) * V);
+  if (whole) return relax_done(g, st, L, pages, label_host, dev, host, sizeof(uint32_t) * V);
   // label[v] = v over active_in = all (cc.cpp:31-37)
   if (ranked)
     copy_twice<uint32_t><<<grid_for(V, 256, g->num_sms), 256, 0, s>>>(g->pr_id_of_rank, V, lab[0], lab[1]);
@@ -765,6 +767,7 @@ static int cc_run(gg_graph *g, uint32_t *label_host, gg_run_stats *st) {
   }
   GG_TRY(timed_end(g, st, L.launches));
   GG_TRY(tr.collect());
+  pages.wait();
   if (label_host) GG_CUDA(cudaMemcpy(label_host, res, sizeof(uint32_t) * V, cudaMemcpyDeviceToHost));
   g->result[0] = res;
   g->result[1] = nullptr;
@@ -820,6 +823,7 @@ static int sssp_run(gg_graph *g, uint32_t root, float *dist_host, gg_run_stats *
   pull.hot = ranked ? g->l1_hot_bytes / 4 : 0xffffffffu;
   pull.wmin = g->ps_wmin;
   pull.width = g->ps_width;
+  Prefault pages(dist_host, sizeof(float) * V);
   GG_TRY(timed_begin(g));
   bool whole = false;
   void *dev = nullptr;
@@ -827,7 +831,7 @@ static int sssp_run(gg_graph *g, uint32_t root, float *dist_host, gg_run_stats *
   void *const states[2] = {dist[0], dist[1]};
   GG_TRY((relax_whole<SsspRun>(g, dout, din, pull, ranked, root, states, q, bm, out, sizeof(float) * V, L, tr, st, &whole,
                                &dev, &host)));
-  if (whole) return relax_done(g, st, L, dist_host, dev, host, sizeof(float) * V);
+  if (whole) return relax_done(g, st, L, pages, dist_host, dev, host, sizeof(float) * V);
   if (ranked) GG_CUDA(cudaMemcpy(&start, g->pr_rank_of + root, sizeof(uint32_t), cudaMemcpyDeviceToHost));
   GG_CUDA(cudaMemsetAsync(bm[0], 0, words * 4, s));
   GG_TRY(counters_reset(g));
@@ -849,6 +853,7 @@ static int sssp_run(gg_graph *g, uint32_t root, float *dist_host, gg_run_stats *
   }
   GG_TRY(timed_end(g, st, L.launches));
   GG_TRY(tr.collect());
+  pages.wait();
   if (dist_host) GG_CUDA(cudaMemcpy(dist_host, res, sizeof(float) * V, cudaMemcpyDeviceToHost));
   g->result[0] = res;
   g->result[1] = nullptr;
@@ -1044,6 +1049,7 @@ static int bc_run(gg_graph *g, uint32_t root, double *dep_host, double *inv_host
   Trace tr(st, g, "gg_bc");
   cudaStream_t s = g->stream;
   Counters *ctr = g->ws.ctr;
+  Prefault pages(dep_host, sizeof(double) * V, inv_host, sizeof(double) * V);
   GG_TRY(timed_begin(g));
   GG_TRY(counters_reset(g));
   bc_begin<<<grid_for(V, 256, g->num_sms), 256, 0, s>>>(np, dep, V, root, rank_of, visited, bm[0], words, qlev,
@@ -1144,6 +1150,7 @@ static int bc_run(gg_graph *g, uint32_t root, double *dep_host, double *inv_host
   GG_CUDA(cudaGetLastError());
   GG_TRY(timed_end(g, st, L.launches));
   GG_TRY(tr.collect());
+  pages.wait();
   if (dep_host) GG_CUDA(cudaMemcpy(dep_host, dep_out, sizeof(double) * V, cudaMemcpyDeviceToHost));
   if (inv_host) GG_CUDA(cudaMemcpy(inv_host, np_out, sizeof(double) * V, cudaMemcpyDeviceToHost));
   g->result[0] = dep_out;

@@ -21,6 +21,7 @@
 #include <stdio.h>
 
 #include <string>
+#include <thread>
 #include <type_traits>
 #include <vector>
 
@@ -259,6 +260,28 @@ inline int ws(gg_graph *g, WsSlot slot, size_t count, T **out) {
   return ws_get(g, slot, count * sizeof(T), (void **)out);
 }
 int ws_free_all(gg_graph *g);
+// The pages of up to two result arrays in host memory, made present and
+// writable (their contents stay) from the constructor on, by threads of its
+// own where the arrays are large, while the device computes: a copy into pages
+// that are not there yet waits for the kernel to clear each one (154 MB: 5.7
+// ms; 0.9 ms into pages that are).  wait() before the copy; the destructor
+// waits as well.
+class Prefault {
+ public:
+  struct Range {
+    void *p;
+    size_t n;
+  };
+  Prefault(void *a, size_t na, void *b = nullptr, size_t nb = 0);
+  ~Prefault() { wait(); }
+  Prefault(const Prefault &) = delete;
+  Prefault &operator=(const Prefault &) = delete;
+  void wait();
+
+ private:
+  std::thread main_;
+};
+
 int counters_reset(gg_graph *g);
 int counters_read(gg_graph *g, Counters *out);
 // Small device-to-host reads on the graph's stream, copied by the SMs into
