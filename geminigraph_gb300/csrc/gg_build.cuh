@@ -19,13 +19,79 @@ struct SortValues {
   uint32_t *in = nullptr, *b0 = nullptr, *b1 = nullptr, *last = nullptr;
 };
 
+// The digits of a sort on key bits [lo_bit, hi_bit): of about equal width, at
+// most 8 bits, so no pass sorts on a narrow remainder.  Where the two halves
+// of the bits take as many passes apart as together, no digit spans them.
+constexpr int RS_THREADS = 512;
+constexpr int RS_BINS = 256;
+constexpr int RS_MAX_PASSES = 8;
+struct RsPlan {
+  int passes;
+  int shift[RS_MAX_PASSES];
+  int bits[RS_MAX_PASSES];
+  uint32_t mask[RS_MAX_PASSES];
+};
+inline int rs_passes(int bits) { return (bits + 7) / 8; }
+inline bool rs_halves(int bits) { return bits % 2 == 0 && 2 * rs_passes(bits / 2) == rs_passes(bits); }
+inline RsPlan rs_plan(int lo_bit, int hi_bit) {
+  RsPlan p;
+  p.passes = 0;
+  const int halves = rs_halves(hi_bit - lo_bit) ? 2 : 1, width = (hi_bit - lo_bit) / halves;
+  for (int h = 0; h < halves; h++)
+    for (int i = 0, n = rs_passes(width), at = h * width; i < n && p.passes < RS_MAX_PASSES; i++) {
+      const int bits = ((h + 1) * width - at + n - i - 1) / (n - i);
+      p.shift[p.passes] = lo_bit + at;
+      p.mask[p.passes] = (1u << bits) - 1u;
+      p.bits[p.passes++] = bits;
+      at += bits;
+    }
+  return p;
+}
+
+// Whether the first digits of b's sort are a's.
+inline bool rs_leads(const RsPlan &a, const RsPlan &b) {
+  bool same = a.passes <= b.passes;
+  for (int p = 0; same && p < a.passes; p++) same = a.shift[p] == b.shift[p] && a.bits[p] == b.bits[p];
+  return same;
+}
+
+// Digit counts of every pass while the keys are at hand, per block in shared
+// memory (all RS_THREADS threads call rs_count_begin and _end).  The passes are
+// unrolled, so that shifts and masks are operands from the constant bank: read
+// by index, one pass's after the other's, they took 0.61 ms for 134 M keys of
+// 46 bits, and 1.25 ms in the kernel that makes the keys (0.51 without
+// counting); unrolled, 0.57 there.  Two copies of the counters by lane are no
+// faster, 4 and 8 slower (0.86).
+typedef uint32_t RsCounters[RS_MAX_PASSES][RS_BINS];
+__device__ __forceinline__ void rs_count_begin(RsCounters &h) {
+  for (int i = threadIdx.x; i < RS_MAX_PASSES * RS_BINS; i += RS_THREADS) (&h[0][0])[i] = 0;
+  __syncthreads();
+}
+__device__ __forceinline__ void rs_count(RsCounters &h, const RsPlan &plan, uint64_t k) {
+#pragma unroll
+  for (int p = 0; p < RS_MAX_PASSES; p++)
+    if (p < plan.passes) atomicAdd(&h[p][(uint32_t)(k >> plan.shift[p]) & plan.mask[p]], 1u);
+}
+__device__ __forceinline__ void rs_count_end(const RsCounters &h, const RsPlan &plan, uint32_t *hist) {
+  __syncthreads();
+  for (int i = threadIdx.x; i < plan.passes * RS_BINS; i += RS_THREADS)
+    if ((&h[0][0])[i]) atomicAdd(hist + i, (&h[0][0])[i]);
+}
+
+// What the head of a sort's scratch holds: nothing yet; the digit counts of
+// rs_plan(lo_bit, hi_bit) (added to scratch after radix_clear); or the places
+// that an earlier sort of the same keys made for its first passes, which are
+// this one's (rs_leads).
+enum RsCounts { RS_NONE, RS_COUNTED, RS_PLACED };
+int radix_clear(gg_graph *g, void *scratch, size_t n);
+
 // Stable LSD radix sort of n < 2^32 keys (and values) on the key bits
 // [lo_bit, hi_bit), ping-ponging the keys between k0 (the input) and k1;
 // *kres / *vres name the buffers holding the result.  scratch: device memory
 // of radix_scratch_bytes(n), 16-byte aligned.  Waits for the stream.
 size_t radix_scratch_bytes(size_t n);
 int radix_sort(gg_graph *g, void *scratch, uint64_t *k0, uint64_t *k1, const SortValues &v, size_t n, int lo_bit,
-               int hi_bit, uint64_t **kres, uint32_t **vres);
+               int hi_bit, uint64_t **kres, uint32_t **vres, RsCounts have = RS_NONE);
 
 // Neighbour / weight storage in device memory, or in mapped pinned host memory.
 int adj_alloc(gg_graph *g, bool host, void **p, size_t bytes);

@@ -14,6 +14,8 @@
 // directions: 54.8 ms with a count kernel, a scan and a register scatter per
 // pass (3.35 ms a scatter, 960 GB/s), 18.5 ms with these passes (1.13 ms
 // each, 2.9 TB/s; the ranking's ballots and block barriers are what is left).
+// With the counts taken where the keys are made, and the CSC's from the CSR's
+// sort, 18.6 ms for 19.7 on the same box.
 // 256 to 1024 threads with 8 to 20 keys each: 18.5 to 22 ms; ranking by
 // __match_any_sync: 21.4 ms.
 #include "gg_build.cuh"
@@ -22,41 +24,23 @@
 
 namespace gg {
 
-constexpr int RS_THREADS = 512;
 constexpr int RS_WARPS = RS_THREADS / 32;
 constexpr int RS_ITEMS = 12;
 constexpr int RS_TILE = RS_THREADS * RS_ITEMS;
-constexpr int RS_BINS = 256;
-constexpr int RS_MAX_PASSES = 8;
 // Polls of one predecessor's word before a tile gives up (about a second):
 // tiles are numbered in the order they start and publish their counts before
 // they wait, so a wait ends unless a device fault stopped an earlier tile.
 constexpr unsigned RS_SPIN = 1u << 20;
 
-struct RsPlan {
-  int passes;
-  int shift[RS_MAX_PASSES];
-  int bits[RS_MAX_PASSES];
-};
-
-// Digit counts of every pass, one read of the keys.  Two copies of the
-// counters (even and odd warps) halve the same-address atomics of skewed digits.
+// Digit counts of every pass, one read of the keys (a graph build's are taken
+// where the keys are made).
 __global__ void __launch_bounds__(RS_THREADS)
     rs_histogram(const uint64_t *__restrict__ keys, size_t n, RsPlan plan, uint32_t *__restrict__ hist) {
-  __shared__ uint32_t h[2][RS_MAX_PASSES][RS_BINS];
-  for (int i = threadIdx.x; i < 2 * RS_MAX_PASSES * RS_BINS; i += RS_THREADS) (&h[0][0][0])[i] = 0;
-  __syncthreads();
-  const int copy = (threadIdx.x >> 5) & 1;
-  for (size_t i = (size_t)blockIdx.x * RS_THREADS + threadIdx.x; i < n; i += (size_t)gridDim.x * RS_THREADS) {
-    const uint64_t k = keys[i];
-    for (int p = 0; p < plan.passes; p++)
-      atomicAdd(&h[copy][p][(uint32_t)(k >> plan.shift[p]) & ((1u << plan.bits[p]) - 1u)], 1u);
-  }
-  __syncthreads();
-  for (int i = threadIdx.x; i < plan.passes * RS_BINS; i += RS_THREADS) {
-    const uint32_t c = (&h[0][0][0])[i] + (&h[1][0][0])[i];
-    if (c) atomicAdd(hist + i, c);
-  }
+  __shared__ RsCounters h;
+  rs_count_begin(h);
+  for (size_t i = (size_t)blockIdx.x * RS_THREADS + threadIdx.x; i < n; i += (size_t)gridDim.x * RS_THREADS)
+    rs_count(h, plan, keys[i]);
+  rs_count_end(h, plan, hist);
 }
 
 // hist[p][d] -> the position where digit d of pass p starts.
@@ -217,18 +201,21 @@ constexpr size_t RS_HEAD = sizeof(uint32_t) * (RS_MAX_PASSES * RS_BINS + RS_MAX_
 static_assert(RS_HEAD % 16 == 0, "the look-back words follow the head");
 size_t radix_scratch_bytes(size_t n) { return RS_HEAD + sizeof(unsigned long long) * RS_BINS * rs_tiles(n); }
 
-// Digits are of equal width (at most 8 bits), so no pass sorts on a narrow
-// remainder.
+int radix_clear(gg_graph *g, void *scratch, size_t n) {
+  GG_CUDA(cudaMemsetAsync(scratch, 0, radix_scratch_bytes(n), g->stream));
+  return GG_OK;
+}
+
 int radix_sort(gg_graph *g, void *scratch, uint64_t *k0, uint64_t *k1, const SortValues &v, size_t n, int lo_bit,
-               int hi_bit, uint64_t **kres, uint32_t **vres) {
+               int hi_bit, uint64_t **kres, uint32_t **vres, RsCounts have) {
   *kres = k0;
   *vres = v.in;
-  RsPlan plan;
-  plan.passes = n > 1 ? (hi_bit - lo_bit + 7) / 8 : 0;
-  if (plan.passes > RS_MAX_PASSES) {
+  if (n > 1 && rs_passes(hi_bit - lo_bit) > RS_MAX_PASSES) {
     set_error("radix sort of %d key bits", hi_bit - lo_bit);
     return GG_ERR_INVALID;
   }
+  RsPlan plan = rs_plan(lo_bit, hi_bit);
+  if (n <= 1) plan.passes = 0;
   if (plan.passes == 0) {
     if (v.in && v.last && n) {
       GG_CUDA(cudaMemcpyAsync(v.last, v.in, sizeof(uint32_t) * n, cudaMemcpyDefault, g->stream));
@@ -236,19 +223,20 @@ int radix_sort(gg_graph *g, void *scratch, uint64_t *k0, uint64_t *k1, const Sor
     }
     return GG_OK;
   }
-  for (int p = 0, at = lo_bit; p < plan.passes; p++) {
-    plan.shift[p] = at;
-    plan.bits[p] = (hi_bit - at + plan.passes - p - 1) / (plan.passes - p);
-    at += plan.bits[p];
-  }
   uint32_t *hist = (uint32_t *)scratch;
   unsigned *ticket = hist + RS_MAX_PASSES * RS_BINS;
   unsigned *err = ticket + RS_MAX_PASSES;
   unsigned long long *look = (unsigned long long *)((char *)scratch + RS_HEAD);
   const size_t tiles = rs_tiles(n);
-  GG_CUDA(cudaMemsetAsync(scratch, 0, radix_scratch_bytes(n), g->stream));
-  rs_histogram<<<grid_for(n, RS_THREADS, g->num_sms, 4), RS_THREADS, 0, g->stream>>>(k0, n, plan, hist);
-  rs_bases<<<1, SCAN_THREADS, 0, g->stream>>>(hist, plan.passes);
+  if (have == RS_PLACED) {
+    GG_CUDA(cudaMemsetAsync(ticket, 0, radix_scratch_bytes(n) - ((char *)ticket - (char *)scratch), g->stream));
+  } else {
+    if (have == RS_NONE) {
+      GG_TRY(radix_clear(g, scratch, n));
+      rs_histogram<<<grid_for(n, RS_THREADS, g->num_sms, 4), RS_THREADS, 0, g->stream>>>(k0, n, plan, hist);
+    }
+    rs_bases<<<1, SCAN_THREADS, 0, g->stream>>>(hist, plan.passes);
+  }
   GG_CUDA(cudaGetLastError());
   if (v.in)
     GG_CUDA(cudaFuncSetAttribute(rs_pass<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)rs_smem<true>()));
