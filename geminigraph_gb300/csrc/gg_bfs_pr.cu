@@ -284,6 +284,12 @@ __device__ __forceinline__ void bfs_walk_wide(const Dir &d, uint32_t V, const ui
   }
 }
 
+// Up to this many vertices: larger graphs' dense calls are long enough to be
+// launched one by one, with the walk's registers to themselves (whole call, one
+// launch / one by one: R-MAT 26 2.54 / 2.37 ms, R-MAT 24 0.83 / 0.84, R-MAT 20
+// 0.27 / 0.33, 8 M vertices uniform 1.05 / 1.08).
+constexpr uint32_t DENSE_RUN_MAX = 1u << 24;
+
 // On return st.n is the queue's length, st.hubs the largest out-degree in it.
 __global__ void __launch_bounds__(RES_THREADS, DENSE_BLOCKS) bfs_dense_run(DenseArgs p, ResState st) {
   cooperative_groups::grid_group grid = cooperative_groups::this_grid();
@@ -315,7 +321,7 @@ __global__ void __launch_bounds__(RES_THREADS, DENSE_BLOCKS) bfs_dense_run(Dense
     if (wide)
       bfs_walk_wide(p.in, V, p.bm[f], p.parent, act, t, tid / 32, nthreads / 32);
     else
-      bfs_walk(p.in, V, p.bm[f], p.parent, act, t, tid / 32, nthreads / 32);
+      bfs_walk<2>(p.in, V, p.bm[f], p.parent, act, t, tid / 32, nthreads / 32);
     if (!wide && p.in.nheavy) {
       bfs_heavy_walk(p.in, p.bm[f], p.visited, p.first);
       grid.sync();
@@ -389,7 +395,7 @@ static int bfs_run(gg_graph *g, uint32_t root, uint32_t *parent_host, gg_run_sta
   cudaStream_t s = g->stream;
   Counters *ctr = g->ws.ctr;
   const bool coop = L.coop_ok() && g->ws.stage;
-  const bool dense_runs = coop && !(st && st->call_ms);
+  const bool dense_runs = coop && !(st && st->call_ms) && g->V <= DENSE_RUN_MAX;
   // the reference's mode (core/graph.hpp:1503-1509), recorded in the trace;
   // the kernel that runs follows g->bfs_pull_div (any in-neighbour on the
   // frontier is a valid parent, so the levels do not depend on it)

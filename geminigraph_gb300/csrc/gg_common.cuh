@@ -51,8 +51,9 @@ int cuda_status(cudaError_t e, const char *what);
 // ---------------------------------------------------------------- graph
 // Degree bins of one direction, built once at load time (the GB300 form of
 // Graph::tune_chunks, core/graph.hpp:1341-1404): pull kernels give a light
-// list (deg <= LIGHT_DEG) one lane, a medium list one warp, and split every
-// heavy list (deg > HEAVY_DEG) into HEAVY_CHUNK-edge chunks, one block each.
+// list (deg <= Dir.light) one lane and cut longer ones into Dir.chunk-edge
+// pieces, a warp each; BFS, which stops at the first hit, gives a warp to lists
+// up to HEAVY_DEG and cuts heavy ones into HEAVY_CHUNK-edge chunks.
 constexpr uint32_t LIGHT_DEG = 32;     // default light-list bound (Dir.light; autotuned)
 constexpr uint32_t HEAVY_DEG = 2048;
 constexpr uint32_t HEAVY_CHUNK = 2048;
@@ -110,7 +111,7 @@ enum WsSlot {
   WS_BM0, WS_BM1, WS_BM2, WS_BM3,       // bitmaps
   WS_Q0, WS_Q1, WS_QLEV,                // queues / level order
   WS_PREFIX,                            // uint64 prefix of queue degrees
-  WS_MSG,                               // a second state array: CC, SSSP (4 B), BC's inverse path counts (8 B)
+  WS_MSG,                               // messages of queued vertices: CC, SSSP (4 B); BC's inverse path counts (8 B)
   WS_S0, WS_S1, WS_S2, WS_S3,           // vertex state arrays
   WS_SCAN,                              // scan scratch
   WS_HUBSUM,                            // per-iteration counters (PageRank)

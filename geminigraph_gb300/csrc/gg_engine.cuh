@@ -718,44 +718,49 @@ __global__ void __launch_bounds__(ROWS_THREADS, ROWS_BLOCKS)
 // entries at a time, up to HEAVY_DEG entries (a kernel of a warp per such list
 // took 237 us a call at R-MAT 26, nearly all of it finding visited vertices).
 // HEAVY lists are bfs_heavy_first's from the start.
+// CHUNKS: of 32 entries a warp reads at a time of the longer lists.  Two keep
+// more loads in flight, one leaves the kernel 38 registers for 42: bfs_pull_walk
+// at R-MAT 26 2.53 / 2.37 ms a BFS with two / one, bfs_dense_run at R-MAT 24 0.83
+// / 0.86.
+template <int CHUNKS>
 __device__ __forceinline__ void bfs_walk(const Dir &d, uint32_t V, const uint32_t *active_in, uint32_t *parent,
-                                         const ActOut &act, Tally &t, size_t warp, size_t nwarps) {
-  const size_t groups = ((size_t)V + 31) / 32;
+                                         const ActOut &act, Tally &t, uint32_t warp, uint32_t nwarps) {
+  const uint32_t groups = V / 32 + (V % 32 != 0);  // at most 2^27: g + 2 * nwarps fits
   const unsigned lane = lane_id();
-  auto words = [&](size_t g, uint32_t &vis, uint32_t &todo) {
+  auto words = [&](uint32_t g, uint32_t &vis, uint32_t &todo) {
     vis = todo = 0;
     if (g < groups) {
       vis = act.visited[g];
       todo = d.nz[g] & ~vis;
     }
   };
-  auto bounds = [&](size_t g, uint32_t todo, unsigned long long &b, unsigned long long &e) {
-    b = e = 0;
+  auto bounds = [&](uint32_t g, uint32_t todo, unsigned long long &b, uint32_t &n) {
+    b = 0;
+    n = 0;
     if ((todo >> lane) & 1u) {
-      b = d.off[g * 32 + lane];
-      e = d.off[g * 32 + lane + 1];
+      const size_t v = (size_t)g * 32 + lane;
+      b = d.off[v];
+      n = (uint32_t)(d.off[v + 1] - b);
     }
   };
-  uint32_t vis, todo, vis1, todo1;
-  unsigned long long b, e;
+  uint32_t vis, todo, vis1, todo1, n;
+  unsigned long long b;
   words(warp, vis, todo);
   words(warp + nwarps, vis1, todo1);
-  bounds(warp, todo, b, e);
-  for (size_t g = warp; g < groups; g += nwarps) {
-    uint32_t vis2, todo2;
-    unsigned long long b1, e1;
+  bounds(warp, todo, b, n);
+  for (uint32_t g = warp; g < groups; g += nwarps) {
+    uint32_t vis2, todo2, n1;
+    unsigned long long b1;
     words(g + 2 * nwarps, vis2, todo2);
-    bounds(g + nwarps, todo1, b1, e1);
+    bounds(g + nwarps, todo1, b1, n1);
     if (todo) {  // uniform
       uint32_t found = NONE32;
-      const unsigned long long n = e - b;
-      const bool heavy = n > HEAVY_DEG;
-      const unsigned long long lim = heavy ? b : n <= d.light ? e : b + d.light;
+      const uint32_t lim = n > HEAVY_DEG ? 0u : n < d.light ? n : d.light;
       constexpr int STEP = 4;
-      for (unsigned long long k = b; k < lim && found == NONE32; k += STEP) {
+      for (uint32_t k = 0; k < lim && found == NONE32; k += STEP) {
         uint32_t u[STEP];
 #pragma unroll
-        for (int j = 0; j < STEP; j++) u[j] = k + j < lim ? nbr_at(d, k + j, GG_SITE) : NONE32;
+        for (int j = 0; j < STEP; j++) u[j] = k + j < lim ? nbr_at(d, b + k + j, GG_SITE) : NONE32;
         unsigned hits = 0;
 #pragma unroll
         for (int j = 0; j < STEP; j++) hits |= (u[j] != NONE32 && bm_test(active_in, u[j])) ? 1u << j : 0u;
@@ -763,23 +768,24 @@ __device__ __forceinline__ void bfs_walk(const Dir &d, uint32_t V, const uint32_
         for (int j = STEP - 1; j >= 0; j--)
           if ((hits >> j) & 1u) found = u[j];
       }
-      for (unsigned rest = __ballot_sync(GG_FULL, found == NONE32 && n > d.light && !heavy); rest; rest &= rest - 1) {
+      for (unsigned rest = __ballot_sync(GG_FULL, found == NONE32 && n > d.light && n <= HEAVY_DEG); rest;
+           rest &= rest - 1) {
         const int j = __ffs(rest) - 1;
-        const unsigned long long ej = __shfl_sync(GG_FULL, e, j);
+        const unsigned long long bj = __shfl_sync(GG_FULL, b, j);
+        const uint32_t nj = __shfl_sync(GG_FULL, n, j);
         uint32_t hit = NONE32;
-        for (unsigned long long base = __shfl_sync(GG_FULL, lim, j); base < ej && hit == NONE32; base += 64) {
-          const unsigned long long k = base + lane;
-          uint32_t s0 = 0, s1 = 0;
-          bool h0 = false, h1 = false;
-          if (k < ej) s0 = nbr_at(d, k, GG_SITE);
-          if (k + 32 < ej) s1 = nbr_at(d, k + 32, GG_SITE);
-          if (k < ej) h0 = bm_test(active_in, s0);
-          if (k + 32 < ej) h1 = bm_test(active_in, s1);
-          const unsigned m0 = __ballot_sync(GG_FULL, h0), m1 = __ballot_sync(GG_FULL, h1);
-          if (m0)
-            hit = __shfl_sync(GG_FULL, s0, __ffs(m0) - 1);
-          else if (m1)
-            hit = __shfl_sync(GG_FULL, s1, __ffs(m1) - 1);
+        for (uint32_t k = d.light + lane; k - lane < nj && hit == NONE32; k += 32 * CHUNKS) {
+          uint32_t u[CHUNKS];
+          bool h[CHUNKS];
+#pragma unroll
+          for (int c = 0; c < CHUNKS; c++) u[c] = k + 32 * c < nj ? nbr_at(d, bj + k + 32 * c, GG_SITE) : NONE32;
+#pragma unroll
+          for (int c = 0; c < CHUNKS; c++) h[c] = u[c] != NONE32 && bm_test(active_in, u[c]);
+#pragma unroll
+          for (int c = 0; c < CHUNKS; c++) {
+            const unsigned m = __ballot_sync(GG_FULL, h[c]);
+            if (m && hit == NONE32) hit = __shfl_sync(GG_FULL, u[c], __ffs(m) - 1);
+          }
         }
         if ((int)lane == j) found = hit;
       }
@@ -790,7 +796,8 @@ __device__ __forceinline__ void bfs_walk(const Dir &d, uint32_t V, const uint32_
         act.visited[g] = vis | bits;
       }
       if (a) {
-        const uint32_t v = (uint32_t)(g * 32 + lane), od = act.out_deg[v];
+        const size_t v = (size_t)g * 32 + lane;
+        const uint32_t od = act.out_deg[v];
         parent[v] = found;
         t.activated += 1;
         t.edges += od;
@@ -802,7 +809,7 @@ __device__ __forceinline__ void bfs_walk(const Dir &d, uint32_t V, const uint32_
     vis1 = vis2;
     todo1 = todo2;
     b = b1;
-    e = e1;
+    n = n1;
   }
 }
 // Six blocks of 256 threads per SM (R-MAT 26: 2.35 ms a BFS; eight, with
@@ -811,7 +818,7 @@ constexpr int BFS_BLOCKS = 6;
 static __global__ void __launch_bounds__(PULL_THREADS, BFS_BLOCKS)
     bfs_pull_walk(Dir d, uint32_t V, const uint32_t *active_in, uint32_t *parent, ActOut act, Counters *ctr) {
   Tally t;
-  bfs_walk(d, V, active_in, parent, act, t, (size_t)blockIdx.x * (PULL_THREADS / 32) + (threadIdx.x >> 5),
+  bfs_walk<1>(d, V, active_in, parent, act, t, (size_t)blockIdx.x * (PULL_THREADS / 32) + (threadIdx.x >> 5),
            (size_t)gridDim.x * (PULL_THREADS / 32));
   t.flush(ctr);
 }
@@ -987,7 +994,7 @@ struct Launch {
     GG_CUDA(cudaGetLastError());
     return GG_OK;
   }
-  // All bins of one dense call, in order: light, medium, heavy chunks, heavy finish.
+  // All bins of one dense call: rows, or the light kernel beside the chunks, then the finish.
   template <class Op>
   int pull(const Dir &d, const Op &op, const ActOut &act, Counters *ctr) {
     if (d.sell_desc) return pull_hot(d, op, act, ctr);
