@@ -372,7 +372,10 @@ const void *gg_result_device_ptr(const gg_graph *g, int which);
  * 32nd entry (clear); pull_vector bit 1 makes the reduction pulls' light
  * lanes read their lists by aligned 32-byte windows (two 16-byte loads per
  * eight entries) instead of one entry per load.  gg_graph_set_bins sets all
- * three (light_deg 1..2048; pull_chunk 128, 256 or 512; pull_vector 0..3).  gg_autotune times the
+ * three (light_deg 1..2048; pull_chunk 128, 256 or 512; pull_vector 0..3);
+ * until it is called the hot-source layout takes bounds of its own (light_deg
+ * from the mean degree, 32 to 1024, chunks of 512), and pull_vector applies to
+ * the plain adjacency.  gg_autotune times the
  * 36 candidates (light_deg 16 to 512) on the graph itself with CUDA events, on the workloads the
  * objective mask names (GG_TUNE_PAGERANK: four float PageRank iterations;
  * GG_TUNE_BFS: one BFS; GG_TUNE_BATCHED: one 64-root gg_bfs_batched, and
@@ -418,8 +421,11 @@ int gg_autotune(gg_graph *g, uint32_t objective, const char *cache_dir, gg_tune_
 /* PageRank's adjacency layout (no reference counterpart; the reference pulls
  * its CSC as loaded).  hot_sources = 1 (the default): on its first call
  * gg_pagerank / gg_pagerank_f32 build, and keep with the graph, a copy of the
- * incoming adjacency with vertices renumbered by descending out-degree and
- * each in-list sorted by the new numbers; the iterations run there and the
+ * incoming adjacency with vertices renumbered by descending class of
+ * out-degree, then by descending in-degree, and each in-list sorted by the new
+ * numbers (gg_sssp's in-lists by weight class, a copy of its own); lists up to
+ * the light bound are stored 32 vertices at a time, column-major, where there
+ * is memory for it.  The iterations run there and the
  * ranks are mapped back to vertex order.  Sums then run in that order, so
  * ranks differ from the plain layout's in the last bits only.  hot_sources =
  * 0 frees the copy and pulls the plain incoming adjacency.  The copy is
@@ -460,8 +466,9 @@ int gg_graph_set_dense_push(gg_graph *g, uint32_t divisor);
  * per-call trace (which records the reference's mode) do not depend on it. */
 int gg_graph_set_bfs_pull(gg_graph *g, uint32_t divisor);
 
-/* Reduction pulls (PageRank, CC, SSSP, BC backward) whose light-list and
- * chunk kernels run side by side on two streams (no reference counterpart):
+/* Reduction pulls (PageRank, CC, SSSP, BC backward) on the plain adjacency,
+ * whose light-list and chunk kernels run side by side on two streams (no
+ * reference counterpart; the hot-source layout's lists are one kernel's):
  * light_blocks in 1..7 launches the light kernel over light_blocks blocks per
  * SM and the chunk kernel over the other 8 - light_blocks, so both are
  * resident on every SM from the start; 0 (default) launches each over the
